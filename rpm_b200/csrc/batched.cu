@@ -492,44 +492,112 @@ __global__ void __launch_bounds__(128) k_b_control(BatchDev B) {
 // of the Hessenberg matrix.  A second pass runs only when the first lost more
 // than 1 - 1/sqrt(2) of the norm (the Kahan-Parlett / DGKS criterion, "twice
 // is enough"); the last pass's norm gives H(j+1, j) and the next scale.
-__global__ void __launch_bounds__(kEwThreads) k_b_arn_dots(BatchDev B, int j, int pass) {
-  __shared__ double2 red[kEwThreads / 32][kBMaxK];
+//
+// Bound by the basis traffic (8 (j + 1) N bytes).  The projections are summed
+// in one fixed order (a thread's elements, the butterfly over its warp, the
+// warps, the blocks), because a projection's last bit reaches FP32 elements;
+// the order is the one of a per-vector loop with two warp sums per vector,
+// which took 240 us per call on the uneven mix (6 vectors of 221,184, 10 of
+// 13,824 and 16 of 864 elements, 20 basis vectors on average).  Here a thread
+// loads kArnVec basis vectors' elements before it uses them, the warp sums of
+// kArnVec vectors share one transposed butterfly (9 exchanges instead of 40),
+// the last block stages the partials through shared memory, and blocks past a
+// trajectory's end leave at once.
+constexpr int kArnVec = 4;      // basis vectors per round
+constexpr int kArnFinish = 32;  // block partials staged per round of the final sum
+
+// Blocks that hold elements of a trajectory of n components.
+__device__ __forceinline__ int ew_blocks(long long n) { return (int)((n + kEwChunk - 1) / kEwChunk); }
+
+// As traj_last_block for the first `blocks` blocks of a trajectory.
+__device__ __forceinline__ bool traj_last_of(unsigned* counter, int blocks) {
+  __shared__ bool is_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) is_last = atomicAdd(counter, 1u) == (unsigned)blocks - 1u;
+  __syncthreads();
+  if (is_last) __threadfence();
+  return is_last;
+}
+
+// Warp sums of eight values per lane by halving the set at each of the first
+// three butterfly levels: lane l ends with the sum of v[(l >> 2) & 7] (bit 4
+// selects v[4..7], bit 3 the upper pair, bit 2 the upper one).  The pairs that
+// are added are those of warp_sum, so the bits are too.
+__device__ __forceinline__ double warp_sum8(double (&v)[8]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int half = 4, o = 16; half >= 1; half >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (c < half) {
+        const double keep = up ? v[c + half] : v[c];
+        const double give = up ? v[c] : v[c + half];
+        v[c] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+    }
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  return v[0];
+}
+
+__global__ void __launch_bounds__(kEwThreads, 2) k_b_arn_dots(BatchDev B, int j, int pass) {
+  // warp sums [warp][vector]; then the staged block partials [block][vector]
+  __shared__ double2 red[kArnFinish][kBMaxK];
   __shared__ double rn[kEwThreads / 32];
+  static_assert(kArnFinish >= kEwThreads / 32, "staging buffer holds the warp sums");
   const int b = blockIdx.y;
   TrajState& s = B.st[b];
-  if (s.skip || (pass == 2 && s.cgs_done)) return;
+  const long long n = s.n;
+  const int blocks = ew_blocks(n);
+  if ((int)blockIdx.x >= blocks || s.skip || (pass == 2 && s.cgs_done)) return;
   const float2* base = B.V + (size_t)b * (B.m + 1) * B.ld;
   const float2* w = base + (size_t)(j + 1) * B.ld;
   const long long i0 = (long long)blockIdx.x * kEwChunk + threadIdx.x;
-  float2 wv[kEwPer];
+  double2 wv[kEwPer];
 #pragma unroll
   for (int k = 0; k < kEwPer; ++k) {
     const long long e = i0 + (long long)k * kEwThreads;
-    wv[k] = e < s.n ? w[e] : make_float2(0.f, 0.f);
+    wv[k] = e < n ? to_d2(w[e]) : make_double2(0.0, 0.0);
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (pass == 1) {  // |w|^2 before the projection (second-pass criterion)
     double nn = 0.0;
 #pragma unroll
-    for (int k = 0; k < kEwPer; ++k) nn = fma((double)wv[k].x, (double)wv[k].x, fma((double)wv[k].y, (double)wv[k].y, nn));
+    for (int k = 0; k < kEwPer; ++k) nn = fma(wv[k].x, wv[k].x, fma(wv[k].y, wv[k].y, nn));
     nn = warp_sum(nn);
     if (lane == 0) rn[warp] = nn;
   }
-  for (int i = 0; i <= j; ++i) {
-    const float2* v = base + (size_t)i * B.ld;
-    double2 acc = make_double2(0.0, 0.0);
+  for (int i = 0; i <= j; i += kArnVec) {
+    float2 q[kArnVec][kEwPer];
 #pragma unroll
-    for (int k = 0; k < kEwPer; ++k) {
-      const long long e = i0 + (long long)k * kEwThreads;
-      if (e < s.n) {
-        const float2 q = v[e];  // conj(q) * w
-        acc.x += (double)q.x * wv[k].x + (double)q.y * wv[k].y;
-        acc.y += (double)q.x * wv[k].y - (double)q.y * wv[k].x;
+    for (int c = 0; c < kArnVec; ++c) {
+      const float2* v = base + (size_t)min(i + c, j) * B.ld;
+#pragma unroll
+      for (int k = 0; k < kEwPer; ++k) {
+        const long long e = i0 + (long long)k * kEwThreads;
+        q[c][k] = e < n ? v[e] : make_float2(0.f, 0.f);
       }
     }
-    acc.x = warp_sum(acc.x);
-    acc.y = warp_sum(acc.y);
-    if (lane == 0) red[warp][i] = acc;
+    double acc[2 * kArnVec];
+#pragma unroll
+    for (int c = 0; c < kArnVec; ++c) {
+      double ax = 0.0, ay = 0.0;  // conj(q) * w: both products of a component are exact in FP64
+#pragma unroll
+      for (int k = 0; k < kEwPer; ++k) {
+        const double qx = q[c][k].x, qy = q[c][k].y;
+        ax = __dadd_rn(ax, __fma_rn(qx, wv[k].x, __dmul_rn(qy, wv[k].y)));
+        ay = __dadd_rn(ay, __fma_rn(qx, wv[k].y, -__dmul_rn(qy, wv[k].x)));
+      }
+      acc[2 * c] = ax;
+      acc[2 * c + 1] = ay;
+    }
+    const double t = warp_sum8(acc);
+    const int at = (lane >> 2) & 7;  // value of this lane: component at & 1 of vector i + at / 2
+    if ((lane & 3) == 0 && i + (at >> 1) <= j)
+      reinterpret_cast<double*>(&red[warp][i + (at >> 1)])[at & 1] = t;
   }
   __syncthreads();
   double2* part = B.adots + ((size_t)b * B.nblk + blockIdx.x) * kBMaxK;
@@ -543,15 +611,30 @@ __global__ void __launch_bounds__(kEwThreads) k_b_arn_dots(BatchDev B, int j, in
     for (int w2 = 0; w2 < kEwThreads / 32; ++w2) t += rn[w2];
     B.part[((size_t)b * B.nblk + blockIdx.x) * 2 + 1] = t;
   }
-  if (traj_last_block(B.count + b)) {
-    if (pass == 1 && threadIdx.x == 0) {
-      double t = 0.0;
-      for (int k = 0; k < (int)gridDim.x; ++k) t += __ldcg(B.part + ((size_t)b * B.nblk + k) * 2 + 1);
-      s.wnorm2 = t;
+  if (traj_last_of(B.count + b, blocks)) {
+    // partials of all blocks, added in block order
+    const double2* parts = B.adots + (size_t)b * B.nblk * kBMaxK;
+    const double* norms = B.part + (size_t)b * B.nblk * 2 + 1;
+    double2 t = make_double2(0.0, 0.0);
+    double tn = 0.0;
+    for (int k0 = 0; k0 < blocks; k0 += kArnFinish) {
+      const int rows = min(kArnFinish, blocks - k0);
+      __syncthreads();
+      for (int idx = threadIdx.x; idx < rows * kBMaxK; idx += blockDim.x) {
+        const int r = idx / kBMaxK, i = idx % kBMaxK;
+        if (i <= j) red[r][i] = __ldcg(parts + (size_t)(k0 + r) * kBMaxK + i);
+      }
+      double mine = 0.0;  // warp 2: the norms, one block per lane
+      if (pass == 1 && warp == 2 && lane < rows) mine = __ldcg(norms + 2 * (k0 + lane));
+      __syncthreads();
+      if ((int)threadIdx.x <= j)
+        for (int r = 0; r < rows; ++r) t = cadd(t, red[r][threadIdx.x]);
+      if (pass == 1 && warp == 2)
+        for (int r = 0; r < rows; ++r) tn += __shfl_sync(0xffffffffu, mine, r);
     }
-    for (int i = threadIdx.x; i <= j; i += blockDim.x) {
-      double2 t = make_double2(0.0, 0.0);
-      for (int k = 0; k < (int)gridDim.x; ++k) t = cadd(t, __ldcg(B.adots + ((size_t)b * B.nblk + k) * kBMaxK + i));
+    if (pass == 1 && warp == 2 && lane == 0) s.wnorm2 = tn;
+    const int i = threadIdx.x;
+    if (i <= j) {
       B.hcur[(size_t)b * kBMaxK + i] = t;
       double2& h = B.hess[((size_t)b * (kBMaxK + 1) + i) * kBMaxK + j];
       h = pass == 1 ? t : cadd(h, t);
@@ -577,12 +660,19 @@ __global__ void __launch_bounds__(kEwThreads) k_b_arn_scale(BatchDev B, int j, i
   }
 }
 
+// w -= V h, |w|^2 and, when no second pass follows, H(j + 1, j) and the next
+// scale.  The trajectories are walked backwards, so that the basis vectors
+// that k_b_arn_dots read last are found in L2; a thread sums its elements side
+// by side (each element's sum runs over i in ascending order): 135 us per call
+// on the uneven mix before, with one element's chain of loads at a time.
 __global__ void __launch_bounds__(kEwThreads) k_b_arn_axpy(BatchDev B, int j, int pass) {
   __shared__ float2 hc[kBMaxK];
   __shared__ double red[32];
-  const int b = blockIdx.y;
+  const int b = gridDim.y - 1 - blockIdx.y;
   TrajState& s = B.st[b];
-  if (s.skip || (pass == 2 && s.cgs_done)) return;
+  const long long n = s.n;
+  const int blocks = ew_blocks(n);
+  if ((int)blockIdx.x >= blocks || s.skip || (pass == 2 && s.cgs_done)) return;
   for (int i = threadIdx.x; i <= j; i += blockDim.x) {
     const double2 t = B.hcur[(size_t)b * kBMaxK + i];
     hc[i] = make_float2((float)t.x, (float)t.y);
@@ -591,18 +681,45 @@ __global__ void __launch_bounds__(kEwThreads) k_b_arn_axpy(BatchDev B, int j, in
   float2* base = B.V + (size_t)b * (B.m + 1) * B.ld;
   float2* w = base + (size_t)(j + 1) * B.ld;
   double nn = 0.0;
-  const long long end = min(s.n, (long long)(blockIdx.x + 1) * kEwChunk);
-  for (long long e = (long long)blockIdx.x * kEwChunk + threadIdx.x; e < end; e += kEwThreads) {
-    float2 x = w[e];
-    for (int i = 0; i <= j; ++i) x = cfma(make_float2(-hc[i].x, -hc[i].y), base[(size_t)i * B.ld + e], x);
-    w[e] = x;
-    nn = fma((double)x.x, (double)x.x, fma((double)x.y, (double)x.y, nn));
+  const long long i0 = (long long)blockIdx.x * kEwChunk + threadIdx.x;
+  float2 x[kEwPer];
+#pragma unroll
+  for (int k = 0; k < kEwPer; ++k) {
+    const long long e = i0 + (long long)k * kEwThreads;
+    x[k] = e < n ? w[e] : make_float2(0.f, 0.f);
+  }
+#pragma unroll 2
+  for (int i = 0; i <= j; ++i) {
+    const float2 c = make_float2(-hc[i].x, -hc[i].y);
+    const float2* v = base + (size_t)i * B.ld;
+    float2 q[kEwPer];
+#pragma unroll
+    for (int k = 0; k < kEwPer; ++k) {
+      const long long e = i0 + (long long)k * kEwThreads;
+      q[k] = e < n ? v[e] : make_float2(0.f, 0.f);
+    }
+#pragma unroll
+    for (int k = 0; k < kEwPer; ++k) x[k] = cfma(c, q[k], x[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < kEwPer; ++k) {
+    const long long e = i0 + (long long)k * kEwThreads;
+    if (e < n) {
+      w[e] = x[k];
+      nn = fma((double)x[k].x, (double)x[k].x, fma((double)x[k].y, (double)x[k].y, nn));
+    }
   }
   nn = block_sum(nn, red);
   if (threadIdx.x == 0) B.part[((size_t)b * B.nblk + blockIdx.x) * 2] = nn;
-  if (traj_last_block(B.count + b) && threadIdx.x == 0) {
+  if (traj_last_of(B.count + b, blocks) && threadIdx.x < 32) {
+    // one block's partial per lane, added in block order
+    const double* parts = B.part + (size_t)b * B.nblk * 2;
     double tot = 0.0;
-    for (int k = 0; k < (int)gridDim.x; ++k) tot += __ldcg(B.part + ((size_t)b * B.nblk + k) * 2);
+    for (int k0 = 0; k0 < blocks; k0 += 32) {
+      const double mine = k0 + (int)threadIdx.x < blocks ? __ldcg(parts + 2 * (k0 + threadIdx.x)) : 0.0;
+      for (int r = 0; r < min(32, blocks - k0); ++r) tot += __shfl_sync(0xffffffffu, mine, r);
+    }
+    if (threadIdx.x != 0) return;
     if (pass == 1) {
       // "twice is enough" (Kahan-Parlett / DGKS): a projection that keeps more
       // than 1/sqrt(2) of the norm needs no second Gram-Schmidt pass
