@@ -280,7 +280,8 @@ typedef struct rpm_batch_config {
                                   launches per Lanczos iteration             */
   int wavefront;               /* persistent kernel: vectors that advance
                                   together through the iterations (<=0:
-                                  equal groups of at most 16) */
+                                  equal groups by tiles, at most 20 vectors
+                                  of 221,184 or 80 of 13,824 elements) */
   int reorth_policy;           /* RPM_REORTH_NONE (0): three-term recurrence
                                   only; RPM_REORTH_PERIODIC (1): after every
                                   `reorth_period` iterations the next Lanczos

@@ -61,7 +61,7 @@ class BatchedPropagator:
     kernel (else the per-iteration passes); "passes" launches the two
     shape-specialised passes per iteration.  ``wavefront``: vectors that move
     through the iterations together in the persistent kernel (0: equal groups
-    of at most 16).
+    by tiles, at most 20 vectors of 221,184 or 80 of 13,824 elements).
     ``reorth_period`` > 0 reorthogonalises the next Lanczos vector against the
     whole basis after every that many iterations (two classical Gram-Schmidt
     passes in FP64 over the complex64 basis); 0 keeps the plain three-term

@@ -1521,13 +1521,20 @@ static void record_step(rpm_batch* Bh, const BatchDev& B, const Layout& L, cudaS
       P.slot0 = (long long)G.b0 * (m + 1);
       P.m = m;
       P.nb = G.nb;
-      // wavefront groups: the requested size, or equal groups of at most 16
-      // vectors (48 vectors: three of 16, 0.1675 ms per iteration against
-      // 0.1755 ms for four of 12; a partial last group costs more)
+      // Wavefront groups: the requested size, or equal groups of at most
+      // kGroupTiles pass-R tiles.  Every phase of a group is one round of its
+      // tiles over the SMs, so a group needs several tiles per SM (30 vectors
+      // of 13,824 elements, 9 tiles each: 21 us per iteration as one group of
+      // 270 tiles, 39 us as two of 135; 320 vectors: 149 us at 64 per group,
+      // 393 us at 16), and no more, so that its vectors stay in L2 (48 vectors
+      // of 221,184 elements, 36 tiles each: 167 us at 16 per group, 170 us at
+      // 24; 20 vectors: 17.0 ms per run as one group, 18.2 ms as two).
       if (Bh->cfg.wavefront > 0) {
         P.gv = Bh->cfg.wavefront;
       } else {
-        const int ngroups = (G.nb + 15) / 16;
+        constexpr int kGroupTiles = 720;
+        const int per_group = std::max(1, kGroupTiles / persistent_r_tiles(G.plan));
+        const int ngroups = (G.nb + per_group - 1) / per_group;
         P.gv = (G.nb + ngroups - 1) / ngroups;
       }
       P.j0 = j0;

@@ -623,15 +623,17 @@ Launcher by_warps(int warps) {
   }
 }
 
-Launcher pick(const CubePlan& plan, int* ltiles) {
+Launcher pick(const CubePlan& plan, int* rtiles, int* ltiles) {
   if (!plan.fast) return nullptr;
   const int l1 = plan.fl_n1, lh = plan.fl_nh, r1 = plan.fr_n1, rh = plan.fr_nh;
   const int warps = g_consumer_warps.load(std::memory_order_relaxed);
   if (l1 == 2 && lh == 5 && r1 == 1 && rh == 6) {
+    if (rtiles) *rtiles = PShape<2, 5, 1, 6>::RT;
     if (ltiles) *ltiles = PShape<2, 5, 1, 6>::LT;
     return by_warps<2, 5, 1, 6>(warps);
   }
   if (l1 == 2 && lh == 3 && r1 == 1 && rh == 4) {
+    if (rtiles) *rtiles = PShape<2, 3, 1, 4>::RT;
     if (ltiles) *ltiles = PShape<2, 3, 1, 4>::LT;
     return by_warps<2, 3, 1, 4>(warps);
   }
@@ -662,12 +664,17 @@ CUtensorMap basis_rows_map(const float2* V, long long nslots, long long ld, int 
 
 int persistent_l_tiles(const CubePlan& plan) {
   int lt = 0;
-  return pick(plan, &lt) ? lt : 0;
+  return pick(plan, nullptr, &lt) ? lt : 0;
+}
+
+int persistent_r_tiles(const CubePlan& plan) {
+  int rt = 0;
+  return pick(plan, &rt, nullptr) ? rt : 0;
 }
 
 bool launch_lanczos_persistent(const PersistentLanczos& p, const CubePlan& plan, const float2* V_base, long long nslots,
                                cudaStream_t stream) {
-  const Launcher fn = pick(plan, nullptr);
+  const Launcher fn = pick(plan, nullptr, nullptr);
   if (!fn) return false;
   if (p.nb < 1 || p.m < 1 || p.gv < 1 || p.j0 < 0 || p.j1 <= p.j0 || p.j1 > p.m)
     fail(RPM_E_INVALID, "persistent Lanczos: empty launch or bad iteration range");
