@@ -141,8 +141,8 @@ int rpm_bin_transition_lines(const double* lam_dev, const void* sp_dev, const vo
  * (run loops of frameworks that own all device memory through a pool or
  * arena, where a cudaMalloc would synchronise the device and escape their
  * accounting; fixed-budget embedded runtimes).  It picks the same kernels as
- * rpm_hpsi for the same arguments.  Its only scratch, batch x ld elements of
- * the partial result between the two radical passes, lives in a 4 MiB array
+ * rpm_hpsi for the same arguments.  The only scratch of any of them, batch x ld
+ * elements of the partial result between the two radical passes, lives in a 4 MiB array
  * compiled into the library, which every GPU that loads the library keeps
  * until process exit; larger batch x ld x element-size requests fail with
  * RPM_E_UNSUPPORTED (systems without a radical split need no scratch).

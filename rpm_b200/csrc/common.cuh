@@ -186,6 +186,10 @@ struct CubeView {
   const void* orecR;
   const void* orecL;
   int orec_bytes_r, orec_bytes_l;
+  // complex128 views of standard-layout systems: per group index of each
+  // radical the records of the direct H psi (hpsi_direct.cuh); else null
+  const void* lrec;
+  const void* rrec;
 };
 
 }  // namespace rpm

@@ -3,7 +3,7 @@
 // Three exact forms of the reference's matrix-free action
 // (rpm_statevector_engine.py:95-108 generic, :221-245 radical split):
 //
-// * Cube form (default for radical-split systems).  The state is viewed as
+// * Cube form (complex64, and complex128 outside the direct kernel's layout).  The state is viewed as
 //   Psi[l, r], l over (electron A, FAD nuclei), r over (electron B, TrpH
 //   nuclei).  Two shared-memory-tiled passes:
 //     pass L: a tile of all l x 2*TR columns (both electron-B halves) ->
@@ -31,6 +31,7 @@
 
 #include "common.cuh"
 #include "hpsi.cuh"
+#include "hpsi_direct.cuh"
 
 namespace rpm {
 
@@ -767,7 +768,9 @@ template <class T>
 void launch_cube(const HpsiArgs<T>& a, const CubePlan& p, T* ya, int batch, cudaStream_t st) {
   const CubeTuning tu = cube_tuning();
   const bool tuned = tu.ni_l || tu.ni_r || tu.tr || tu.tl;
-  if (!tuned && launch_cube_fast<T>(a, p, ya, batch, st)) return;
+  if constexpr (std::is_same<T, float2>::value) {
+    if (!tuned && launch_cube_fast<T>(a, p, ya, batch, st)) return;
+  }
   const int ni_l = tu.ni_l > 0 ? std::min(tu.ni_l, p.ni_l) : p.ni_l;
   const int ni_r = tu.ni_r > 0 ? std::min(tu.ni_r, p.ni_r) : p.ni_r;
   if (ni_l >= 2) {
@@ -883,10 +886,29 @@ CubePlan cube_plan(rpm_system* const* systems, int nsys) {
   return p;
 }
 
+// The direct H psi takes every complex128 call of a standard-layout system: one
+// launch without scratch, at any batch (the full system: 13 us for one vector
+// and 334 us for 64 against 35 and 428 us of two shape-specialised tiled
+// passes, whose few large tiles left most SMs idle for small batches; 864
+// dimensions, 32 vectors: 10 against 23 us of two general cube passes).  An
+// explicit cube-kernel variant (rpm_set_cube_tuning) keeps the cube kernels.
+template <class T>
+static bool try_direct(rpm_system* sys, const T* in, T* out, int batch, long long ld, const double* scale_dev,
+                       cudaStream_t stream) {
+  if constexpr (std::is_same<T, double2>::value) {
+    const CubeTuning tu = cube_tuning();
+    if (tu.ni_l || tu.ni_r || tu.tr || tu.tl || !direct_usable(sys) || batch > 65535) return false;
+    launch_direct(sys, in, out, batch, ld, scale_dev, stream);
+    return true;
+  }
+  return false;
+}
+
 template <class T>
 void launch_hpsi(rpm_system* sys, const T* in, T* out, int batch, long long ld, cudaStream_t stream) {
   if (!sys->on_device) fail(RPM_E_INVALID, "system was created host-only");
   if (batch < 1) return;
+  if (try_direct<T>(sys, in, out, batch, ld, nullptr, stream)) return;
   if (sys->split) {
     T* ya = static_cast<T*>(system_scratch(sys, SLOT_YA, (size_t)batch * ld * sizeof(T)));
     if (sys->cube && sys->cube64.inner_l >= 1 && sys->cube64.inner_r >= 1) {
@@ -918,6 +940,7 @@ void launch_hpsi_scaled(rpm_system* sys, const T* in, T* out, int batch, long lo
     fail(RPM_E_UNSUPPORTED,
          "scaled H psi needs a Hermitian radical-split system with a trailing spin-1/2 digit per radical");
   if (batch < 1) return;
+  if (try_direct<T>(sys, in, out, batch, ld, scale_dev, stream)) return;
   T* ya = static_cast<T*>(system_scratch(sys, SLOT_YA, (size_t)batch * ld * sizeof(T)));
   HpsiArgs<T> a{};
   a.in = in;
@@ -1028,9 +1051,10 @@ static void launch_hpsi_noalloc(rpm_system* sys, const T* in, T* out, int batch,
     fail(RPM_E_UNSUPPORTED, "rpm_hpsi_noalloc: batch x ld x element size = " + std::to_string(need) +
                                 " bytes exceeds its fixed 4 MiB scratch; use rpm_hpsi or a smaller batch");
   }
+  // the kernel choice of launch_hpsi: the direct form (no scratch), the cube
+  // form, else the CSR passes, else the per-term kernel (no scratch)
+  if (try_direct<T>(sys, in, out, batch, ld, nullptr, stream)) return;
   T* ya = static_cast<T*>(noalloc_scratch());
-  // the kernel choice of launch_hpsi: cube form, else the CSR passes, else
-  // the per-term kernel (which needs no scratch)
   if (sys->cube && sys->cube64.inner_l >= 1 && sys->cube64.inner_r >= 1) {
     HpsiArgs<T> a{};
     a.in = in;

@@ -1,4 +1,4 @@
-// Shape-specialised H psi passes (complex64 and complex128) for the standard
+// Shape-specialised complex64 H psi passes for the standard
 // radical layout.
 //
 // Scope: radical-split systems whose tensor axes are ordered
@@ -34,8 +34,7 @@
 // beta_{j-1} v_{j-1} (staged there for the combine) from the partial, so
 // pass L never reads v_{j-1}.  Pass L walks the batch in reverse order so
 // that the partials and inputs written or read last are still in L2 when it
-// starts.  complex128 runs the same passes with one element per 16-byte copy,
-// an odd row stride in 16-byte units, no fused recurrence and one CTA per SM.
+// starts.  (complex128 runs the direct kernel, hpsi_direct.cu.)
 #include <mutex>
 #include <utility>
 #include <vector>
@@ -159,7 +158,7 @@ __global__ void __launch_bounds__(PassR<T, N1, NH>::WARPS * 32, FastT<T>::MINB)
   T* tab = reinterpret_cast<T*>(smem_raw);
   ORec<T>* orec = reinterpret_cast<ORec<T>*>(smem_raw + P::TAB_BYTES);
   T* tile = reinterpret_cast<T*>(smem_raw + P::TAB_BYTES + P::OREC_BYTES);
-  T* ptile = tile + TR * RS;  // complex64 only
+  T* ptile = tile + TR * RS;
   const int half_l = view->half_l;
   const int row0 = blockIdx.x * TR;
   const int rows = min(TR, 2 * half_l - row0);
@@ -178,10 +177,9 @@ __global__ void __launch_bounds__(PassR<T, N1, NH>::WARPS * 32, FastT<T>::MINB)
   };
   // fused Lanczos (j > 0): the tile receives w'_j and ptile v_{j-1}; below,
   // v_j = (w'_j - alpha_{j-1} v_{j-1}) * scale replaces w'_j in the tile and in `in`
-  const bool combine = EPU == 2 && a.lz.on && !a.lz.first;
+  const bool combine = a.lz.on && !a.lz.first;
   const bool with_prev = combine && a.lz.on == 1;  // Arnoldi (on == 2) only rescales
-  const T* pv = nullptr;
-  if constexpr (EPU == 2) pv = with_prev ? a.lz.prev + (long long)b * a.ld : nullptr;
+  const T* pv = with_prev ? a.lz.prev + (long long)b * a.ld : nullptr;
   for (int idx = threadIdx.x; idx < units; idx += NT) {
     int slot;
     long long g;
@@ -193,7 +191,7 @@ __global__ void __launch_bounds__(PassR<T, N1, NH>::WARPS * 32, FastT<T>::MINB)
   __syncthreads();
   build_orec<T, S, K - 2, 4>(tab, orec, NO, threadIdx.x, NT);
   copy_wait_all();
-  if constexpr (EPU == 2) if (combine) {
+  if (combine) {
     // each thread combines the units it copied (visible to it after its own wait)
     const float al = with_prev ? (float)a.lz.alpha_prev[(long long)b * a.lz.dstride] : 0.0f;
     const float sc = (float)in_scale(a, b);
@@ -257,18 +255,14 @@ __global__ void __launch_bounds__(PassL<T, N1, NH>::WARPS * 32, FastT<T>::MINB)
   build_orec<T, S, K - 3, 8>(tab, orec, NO, threadIdx.x, NT);
   copy_wait_all();
   __syncthreads();
-  const bool fused = EPU == 2 && a.lz.on == 1;
+  const bool fused = a.lz.on == 1;
   const bool store = !fused || !a.lz.last;
   const R sf = a.lz.on ? R(1) : (R)in_scale(a, b);  // fused / Arnoldi: pass R wrote the scaled v_j
   double dot = 0.0, nw = 0.0, nv = 0.0;
   l_tile_math<T, N1, NH>(tab, orec, tile, view->pair, HR, c0, quarter, yb + (long long)b * (a.ya_ld ? a.ya_ld : a.ld),
                          a.out + (long long)b * a.ld, sf, store, threadIdx.x >> 5, P::WARPS, dot, nw, nv);
-  if constexpr (EPU == 2) {
-    if (fused) finish_lanczos(a, b, dot, nw, nv);
-    else if (a.dot_part && !a.lz.on) finish_dot_fast(a, b, dot);
-  } else {
-    if (a.dot_part) finish_dot_fast(a, b, dot);
-  }
+  if (fused) finish_lanczos(a, b, dot, nw, nv);
+  else if (a.dot_part && !a.lz.on) finish_dot_fast(a, b, dot);
 }
 
 // ---------------------------------------------------------------------------
@@ -313,8 +307,7 @@ using LaunchL = void (*)(const HpsiArgs<T>&, const T*, int, int, cudaStream_t);
 template <class T>
 using LaunchR = void (*)(const HpsiArgs<T>&, T*, int, int, cudaStream_t);
 
-// Shared memory a CTA may use (the complex128 tiles are twice as large: a
-// pattern whose pass does not fit has no complex128 variant).
+// Shared memory a CTA may use (a pattern whose pass does not fit has none).
 constexpr int kFastMaxSmem = 227 * 1024;
 
 template <class T, int N1, int NH>
@@ -399,12 +392,8 @@ bool cube_fast_usable(const HpsiArgs<T>& a, const CubePlan& p, const T* ya) {
   const long long yld = a.ya_ld ? a.ya_ld : a.ld;
   auto aligned = [](const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; };
   if (!aligned(a.in) || !aligned(a.out) || !aligned(ya)) return false;
-  if constexpr (FastT<T>::EPU == 2) {
-    if ((a.ld & 1) || (yld & 1)) return false;
-    if (a.lz.on == 1 && !a.lz.first && !aligned(a.lz.prev)) return false;
-  } else {
-    if (a.lz.on) return false;  // the fused recurrence is complex64 only
-  }
+  if ((a.ld & 1) || (yld & 1)) return false;
+  if (a.lz.on == 1 && !a.lz.first && !aligned(a.lz.prev)) return false;
   return pick_l<T>(p.fl_n1, p.fl_nh) && pick_r<T>(p.fr_n1, p.fr_nh);
 }
 
@@ -421,9 +410,7 @@ bool launch_cube_fast(const HpsiArgs<T>& a, const CubePlan& p, T* ya, int batch,
 }
 
 template bool cube_fast_usable<float2>(const HpsiArgs<float2>&, const CubePlan&, const float2*);
-template bool cube_fast_usable<double2>(const HpsiArgs<double2>&, const CubePlan&, const double2*);
 template bool launch_cube_fast<float2>(const HpsiArgs<float2>&, const CubePlan&, float2*, int, cudaStream_t);
-template bool launch_cube_fast<double2>(const HpsiArgs<double2>&, const CubePlan&, double2*, int, cudaStream_t);
 
 }  // namespace rpm
 

@@ -34,19 +34,12 @@ struct Shape {
   static constexpr int NTAB = offD(K);
 };
 
-// Element type: complex64 stages two elements per 16-byte copy and carries
-// the fused Lanczos recurrence; complex128 stages one and runs plain H psi
-// (and holds twice the registers per element, so one CTA per SM is assumed).
+// Element type: complex64 (two elements per 16-byte copy).
 template <class T> struct FastT;
 template <> struct FastT<float2> {
   using R = float;
   static constexpr int EPU = 2;
   static constexpr int MINB = 2;
-};
-template <> struct FastT<double2> {
-  using R = double;
-  static constexpr int EPU = 1;
-  static constexpr int MINB = 1;
 };
 
 // Per outer index: diagonal and electron-flip coefficients merged over the
@@ -153,11 +146,11 @@ struct PassR {
   static constexpr int NO = HR / 4;      // outer indices per row
   static constexpr int NTASK = (NO + 1) / 2;  // warp tasks: two outer indices each
   // padded row stride (elements): an odd number of 16-byte units
-  static constexpr int RS = EPU == 2 ? 2 * HR + 2 : 2 * HR + 1;
+  static constexpr int RS = 2 * HR + 2;
   static constexpr int TAB_BYTES = align16c(S::NTAB * (int)sizeof(T));
   static constexpr int OREC_BYTES = align16c(NO * (int)sizeof(ORec<T>));
-  // tables, records, the tile and (complex64, fused Lanczos) the tile of v_{j-1}
-  static constexpr int SMEM = TAB_BYTES + OREC_BYTES + (EPU == 2 ? 2 : 1) * TR * RS * (int)sizeof(T);
+  // tables, records, the tile and (fused Lanczos) the tile of v_{j-1}
+  static constexpr int SMEM = TAB_BYTES + OREC_BYTES + 2 * TR * RS * (int)sizeof(T);
   // 8 warps: measured faster than 12 or 16, which force register spills
   static constexpr int WARPS =
       NTASK % 8 == 0 ? 8 : NTASK % 6 == 0 ? 6 : NTASK % 4 == 0 ? 4 : NTASK % 3 == 0 ? 3 : NTASK < 8 ? NTASK : 8;
@@ -222,7 +215,7 @@ __device__ __forceinline__ void r_tile_math(const T* tab, const ORec<T>* orec, c
   using S = typename P::S;
   using R = typename FastT<T>::R;
   constexpr int K = S::K;
-  constexpr int HR = P::HR, NO = P::NO, RS = P::RS, EPU = P::EPU;
+  constexpr int HR = P::HR, NO = P::NO, RS = P::RS;
   const int lane = threadIdx.x & 31;
   const int row = lane & 15, hsel = lane >> 4;
   const T* rowp = tile + row * RS;
@@ -241,17 +234,12 @@ __device__ __forceinline__ void r_tile_math(const T* tab, const ORec<T>* orec, c
     auto load = [&](int delta, T (&y)[2][4]) {
 #pragma unroll
       for (int ep = 0; ep < 2; ++ep) {
-        if constexpr (EPU == 2) {
-          const float4 u = *reinterpret_cast<const float4*>(rowp + ep * HR + 4 * o + delta);
-          const float4 v = *reinterpret_cast<const float4*>(rowp + ep * HR + 4 * o + delta + 2);
-          y[ep][0] = make_float2(u.x, u.y);
-          y[ep][1] = make_float2(u.z, u.w);
-          y[ep][2] = make_float2(v.x, v.y);
-          y[ep][3] = make_float2(v.z, v.w);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) y[ep][i] = rowp[ep * HR + 4 * o + delta + i];
-        }
+        const float4 u = *reinterpret_cast<const float4*>(rowp + ep * HR + 4 * o + delta);
+        const float4 v = *reinterpret_cast<const float4*>(rowp + ep * HR + 4 * o + delta + 2);
+        y[ep][0] = make_float2(u.x, u.y);
+        y[ep][1] = make_float2(u.z, u.w);
+        y[ep][2] = make_float2(v.x, v.y);
+        y[ep][3] = make_float2(v.z, v.w);
       }
     };
     T x[2][4], acc[2][4];
@@ -276,18 +264,7 @@ __device__ __forceinline__ void r_tile_math(const T* tab, const ORec<T>* orec, c
         partner_mac(c, y, acc);
       }
     }
-    if (active && EPU == 1) {
-#pragma unroll
-      for (int e = 0; e < 2; ++e)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          T v = acc[e][i];
-          v.x *= sf;
-          v.y *= sf;
-          y_b[e * quarter + 4 * o + i] = v;
-        }
-    }
-    if constexpr (EPU == 2) if (active) {
+    if (active) {
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const long long at = e * quarter + 4 * o;
@@ -380,20 +357,18 @@ __device__ __forceinline__ void l_tile_math(const T* tab, const ORec<T>* orec, c
     const int lo = o * 8 + lg * 4;  // l of cube element i = 0
     T pb[2][4];  // pass-R partial of the cube (with -beta_{j-1} v_{j-1} when fused), loaded early
     bool staged = false;
-    if constexpr (P::EPU == 2) {
-      if (pbuf) {
-        // 32 segments of 8 consecutive columns (64 bytes), four 16-byte copies each
+    if (pbuf) {
+      // 32 segments of 8 consecutive columns (64 bytes), four 16-byte copies each
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int cidx = lane + 32 * k;
-          const int seg = cidx >> 2, piece = cidx & 3;
-          const int se = seg >> 4, si = (seg >> 2) & 3, sh = (seg >> 1) & 1, sg = seg & 1;
-          copy16(pbuf + seg * 8 + 2 * piece,
-                 y_vec + (2 * se + sh) * quarter + (long long)(o * 8 + sg * 4 + si) * HR + c0 + 2 * piece);
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-        staged = true;
+      for (int k = 0; k < 4; ++k) {
+        const int cidx = lane + 32 * k;
+        const int seg = cidx >> 2, piece = cidx & 3;
+        const int se = seg >> 4, si = (seg >> 2) & 3, sh = (seg >> 1) & 1, sg = seg & 1;
+        copy16(pbuf + seg * 8 + 2 * piece,
+               y_vec + (2 * se + sh) * quarter + (long long)(o * 8 + sg * 4 + si) * HR + c0 + 2 * piece);
       }
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+      staged = true;
     }
     if (!staged) {
 #pragma unroll

@@ -13,6 +13,7 @@
 #include <set>
 
 #include "common.cuh"
+#include "hpsi_direct.cuh"
 
 namespace rpm {
 
@@ -235,6 +236,51 @@ static std::vector<float2> to_f2(const std::vector<cd>& v) {
   return out;
 }
 
+// Direct-H psi records of one radical (hpsi_direct.cuh), one per value of its
+// nuclear digits.
+static std::vector<direct::HRec> direct_records(const CubeSide& side, const std::vector<double2>& tab) {
+  std::vector<direct::HRec> out(side.half);
+  for (int g = 0; g < side.half; ++g) {
+    direct::HRec r{};
+    r.d[0] = tab[0].x;
+    r.d[1] = tab[1].x;
+    r.f[0] = tab[2];
+    r.f[1] = tab[3];
+    for (int k = 0; k < side.K; ++k) {
+      const int m = (g / side.gs[k]) % side.dim[k];
+      r.digits |= (unsigned long long)m << (4 * k);
+      for (int e = 0; e < 2; ++e) {
+        r.d[e] += tab[side.offD[k] + e * side.dim[k] + m].x;
+        const double2 f = tab[side.offF[k] + e * side.dim[k] + m];
+        r.f[e].x += f.x;
+        r.f[e].y += f.y;
+      }
+    }
+    out[g] = r;
+  }
+  return out;
+}
+
+// Standard layout psi[eA][eB][l][r] within the direct H psi's limits.
+static bool direct_layout(const rpm_system* sys) {
+  int partners[2] = {0, 0}, side = 0;
+  for (const CubeSide* s : {&sys->cube_l, &sys->cube_r}) {
+    for (int k = 0; k < s->K; ++k) {
+      if (s->dim[k] > direct::kMaxDigit) return false;
+      partners[side] += s->dim[k] - 1;
+    }
+    if (partners[side] > direct::kMaxPartners) return false;
+    ++side;
+  }
+  if (sys->cube_l.ntab + sys->cube_r.ntab > direct::kMaxTables) return false;
+  const long long n = sys->n, hl = sys->half_l, hr = sys->half_r;
+  for (long long l = 0; l < (long long)sys->offl.size(); ++l)
+    if (sys->offl[l] != (l / hl) * (n / 2) + (l % hl) * hr) return false;
+  for (long long r = 0; r < (long long)sys->offr.size(); ++r)
+    if (sys->offr[r] != (r / hr) * (n / 4) + (r % hr)) return false;
+  return true;
+}
+
 static void upload_system(rpm_system* sys) {
   check_cuda(cudaGetDevice(&sys->device), "cudaGetDevice");
   // generic per-term tables (always present)
@@ -317,6 +363,12 @@ static void upload_system(rpm_system* sys) {
         c32.orecL = upload<float>(sys, rl.data(), rl.size() * sizeof(float));
         c32.orec_bytes_r = (int)(rr.size() * sizeof(float));
         c32.orec_bytes_l = (int)(rl.size() * sizeof(float));  // records (padded to 16 bytes) + 128 pair bytes
+      }
+      c64.lrec = c64.rrec = c32.lrec = c32.rrec = nullptr;
+      if (direct_layout(sys)) {
+        const auto lr = direct_records(cl, tl64), rr = direct_records(cr, tr64);
+        c64.lrec = upload<direct::HRec>(sys, lr.data(), lr.size() * sizeof(direct::HRec));
+        c64.rrec = upload<direct::HRec>(sys, rr.data(), rr.size() * sizeof(direct::HRec));
       }
       sys->cube64_dev = upload<CubeView<double2>>(sys, &c64, sizeof(c64));
       sys->cube32_dev = upload<CubeView<float2>>(sys, &c32, sizeof(c32));
