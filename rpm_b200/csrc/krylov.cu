@@ -21,6 +21,7 @@
 
 #include "common.cuh"
 #include "krylov.cuh"
+#include "plain_lanczos.cuh"
 
 namespace rpm {
 
@@ -29,18 +30,10 @@ constexpr int kRowsPerThread = 4;
 constexpr int kRowsPerBlock = kThreads * kRowsPerThread;
 
 // ---------------------------------------------------------------------------
-// Lanczos kernels (single vector, complex128)
-// Device scalars (LanczosScalars) live in SLOT_SMALL.
+// Lanczos kernels (single vector, complex128), for systems outside the
+// one-launch build's layout (plain_lanczos.cu).  Device scalars
+// (LanczosScalars) live in SLOT_SMALL.
 // ---------------------------------------------------------------------------
-struct LanczosScalars {
-  unsigned counter[8];
-  int stop;       // basis size after a breakdown (0 = running)
-  int pad;
-  double norm;    // ||state||
-  double2 h1[RPM_MAX_KRYLOV];
-  double2 h2[RPM_MAX_KRYLOV];
-};
-
 // v0 = state / ||state|| ; first launch computes ||state||^2 partials.
 __global__ void __launch_bounds__(kThreads) k_norm_partial(const double2* __restrict__ x, long long n,
                                                           double2* partials, LanczosScalars* sc, int init) {
@@ -528,6 +521,13 @@ static double2* reduce_partials(rpm_system* sys, size_t count) {
   return static_cast<double2*>(system_scratch(sys, SLOT_REDUCE, count * sizeof(double2)));
 }
 
+// A grid barrier of the one-launch build gave up: clear its counters, report.
+[[noreturn]] static void barrier_timeout(LanczosScalars* sc, cudaStream_t st) {
+  cudaMemsetAsync(sc, 0, sizeof(LanczosScalars), st);
+  cudaStreamSynchronize(st);
+  fail(RPM_E_TIMEOUT, "plain Lanczos kernel: a grid barrier gave up (time limit)");
+}
+
 static int row_blocks(long long n) { return (int)((n + kRowsPerBlock - 1) / kRowsPerBlock); }
 
 // Launches a basis build; the size and ||state|| land in the system's
@@ -538,6 +538,7 @@ static void lanczos_basis_launch(rpm_system* sys, const double2* state, int max_
   const int m = (int)std::min<long long>(max_dim, n);
   if (m < 1 || m > RPM_MAX_KRYLOV) fail(RPM_E_UNSUPPORTED, "Krylov dimension must be in [1, 128]");
   LanczosScalars* sc = scalars(sys);
+  if (launch_plain_basis(sys, state, m, tol, basis, alpha, beta, sc, st)) return;
   const int nb = row_blocks(n);
   double2* partials = reduce_partials(sys, (size_t)nb * (RPM_MAX_KRYLOV + 1));
   double2* w = static_cast<double2*>(system_scratch(sys, SLOT_WORK, (size_t)n * sizeof(double2)));
@@ -565,11 +566,12 @@ void lanczos_basis(rpm_system* sys, const double2* state, int max_dim, double to
   LanczosScalars* sc = scalars(sys);
   struct {
     int stop;
-    int pad;
+    int timeout;
     double norm;
   } info;
   check_cuda(cudaMemcpyAsync(&info, &sc->stop, sizeof(info), cudaMemcpyDeviceToHost, st), "copy lanczos info");
   check_cuda(cudaStreamSynchronize(st), "lanczos sync");
+  if (info.timeout) barrier_timeout(sc, st);
   *norm = info.norm;
   if (info.stop < 0) fail(RPM_E_INVALID, "Cannot propagate the zero vector.");
   *actual = info.stop > 0 ? info.stop : m;
@@ -602,7 +604,8 @@ struct PlainIn {
 };
 
 struct PlainOut {
-  int status;  // 0 accepted, 1 rejected, 2 the maximum basis is needed, 3 eigen-solver failure, 4 zero vector
+  int status;  // 0 accepted, 1 rejected, 2 the maximum basis is needed, 3 eigen-solver failure, 4 zero vector,
+               // 5 a grid barrier of the basis build gave up
   int size, selected, lo, exact, pad;
   double err, norm, new_norm;
 };
@@ -704,7 +707,7 @@ __global__ void __launch_bounds__(kPlainWarps * 32) k_plain_control(const double
       }
       if (last != in.max_dim) add(in.max_dim);
     }
-    s_status = stop < 0 ? 4 : 0;
+    s_status = sc->timeout ? 5 : stop < 0 ? 4 : 0;
     s_size = stop < 0 ? 0 : size;
     s_exact = exact;
     s_ndims = nd;
@@ -955,6 +958,7 @@ static void plain_propagate(rpm_system* sys, const rpm_plain_knobs& k, double2* 
       run(in);
       matvecs += o.size;
     }
+    if (o.status == 5) barrier_timeout(sc, st);
     if (o.status == 4) fail(RPM_E_INVALID, "Cannot propagate the zero vector.");
     if (o.status == 3) fail(RPM_E_NUMERIC, "tridiagonal eigen-solver did not converge");
     if (o.status == 1) {

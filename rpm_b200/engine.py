@@ -461,9 +461,10 @@ class PropagationResult:
 class _Krylov:
     """Device tridiagonal (alpha, beta) + its spectra, for one basis build."""
 
-    def __init__(self, prop, size: int):
+    def __init__(self, prop, size: int, norm: float):
         self.prop = prop
         self.size = size
+        self.norm = norm  # ||state|| as the basis was normalised with
         self._records: dict[int, int] = {}
 
     def spectra(self, dims):
@@ -541,7 +542,7 @@ class AdaptiveLanczosPropagator:
                   float(self.breakdown_tolerance), _lib.ptr(basis), _lib.ptr(self._alpha), _lib.ptr(self._beta),
                   ctypes.byref(actual), ctypes.byref(norm), _lib.stream_handle())
         self.hamiltonian.matvec_count += actual.value
-        return _Krylov(self, actual.value)
+        return _Krylov(self, actual.value, norm.value)
 
     def _evaluate(self, kry: _Krylov, pairs, times, state_norm, gram=None):
         """Coefficients/errors/values for (dimension, embedded dimension or None) at times."""
@@ -658,7 +659,6 @@ class AdaptiveLanczosPropagator:
         _lib.call("rpm_norm", self.hamiltonian._system.handle, _lib.ptr(state), ctypes.byref(norm0),
                   _lib.stream_handle())
         maximum_norm_error = abs(norm0.value - 1.0)
-        state_norm_now = norm0.value
         starting = self.hamiltonian.matvec_count
         if times[0] == 0.0:
             values[0] = observable(state) if gpu_singlet else observable(state.cpu().numpy())
@@ -678,9 +678,9 @@ class AdaptiveLanczosPropagator:
             trial = min(step, remaining)
             if trial < self.minimum_step_us:
                 raise RuntimeError("Lanczos step fell below the configured minimum.")
-            state_norm = state_norm_now
             target = self.maximum_dimension if prefer_max else self.minimum_dimension
             kry = self._basis(state, target)
+            state_norm = kry.norm
             local_budget = self.state_error_budget * trial / max(final_time, trial)
             selected = None
             coef_row = None
@@ -764,7 +764,6 @@ class AdaptiveLanczosPropagator:
                     bounds[at] = state_error_to_population_bound(state_errors[at])
             new_norm = self._combine(selected, coef_row, state_norm, next_state)
             state, next_state = next_state, state
-            state_norm_now = new_norm
             current_time = step_end
             accumulated_error += endpoint_error
             accepted += 1
