@@ -189,6 +189,15 @@ int rpm_krylov_eval(const double* spectra_dev, int nreq, const rpm_krylov_req* r
                     void* coef_dev, int coef_ld, double* err_host, double* value_host,
                     void* stream);
 
+/* As rpm_krylov_eval straight from the tridiagonal (alpha, beta) of a basis of
+ * `size` vectors, without spectra: hi and lo of a request are dimensions (lo <=
+ * 0: none).  The exponentials are Chebyshev series of the tridiagonal, so that
+ * small embedded errors carry no eigen-solver rounding (ENG:569-609, 690-715). */
+int rpm_krylov_coefficients(const double* alpha_dev, const double* beta_dev, int size, int nreq,
+                            const rpm_krylov_req* reqs_host, double safety, double state_norm, const void* gram_dev,
+                            int gram_ld, void* coef_dev, int coef_ld, double* err_host, double* value_host,
+                            void* stream);
+
 /* G = A^H A for the singlet amplitudes A = (V[0,1,:] - V[1,0,:])/sqrt 2 of the
  * first m complex128 basis columns (ENG:521-529); gram_dev is m x m complex128,
  * Hermitian-symmetrised. */

@@ -117,6 +117,7 @@ SIGNATURES: dict[str, list] = {
     "rpm_lanczos_basis": [_P, _P, _I, _D, _P, _P, _P, _PI, _PD, _P],
     "rpm_tridiag_spectra": [_P, _P, _I, _PI, _P, _P],
     "rpm_krylov_eval": [_P, _I, ctypes.POINTER(rpm_krylov_req), _D, _D, _P, _I, _P, _I, _PD, _PD, _P],
+    "rpm_krylov_coefficients": [_P, _P, _I, _I, ctypes.POINTER(rpm_krylov_req), _D, _D, _P, _I, _P, _I, _PD, _PD, _P],
     "rpm_singlet_gram": [_P, _P, _I, _P, _P],
     "rpm_combine": [_P, _P, _I, _P, _D, _P, _PD, _P],
     "rpm_plain_propagate": [_P, _P, _P, _PD, _I, _I, _D, _PD, _PD, _P, _P],

@@ -249,6 +249,7 @@ enum Slot : int {
   SLOT_WORK = 2,      // Lanczos work vector
   SLOT_SMALL = 3,     // small device scalars (alpha, beta, h coefficients, flags)
   SLOT_GRAM = 4,      // Gram partials
+  SLOT_PLAIN = 5,     // basis and step buffers of the device-driven plain propagation
 };
 void* system_scratch(rpm_system* sys, int slot, size_t bytes);
 // H psi launchers (hpsi.cu).  `scale_dev`, when non-null, multiplies the input

@@ -583,18 +583,25 @@ void lanczos_basis(rpm_system* sys, const double2* state, int max_dim, double to
 // ---------------------------------------------------------------------------
 // One Krylov step of the reference controller (rpm_statevector_engine.py:
 // 717-933) is a fixed launch sequence with one host read at its end: the
-// basis, the singlet Gram of the basis, k_plain_control (the spectra of every
-// dimension the step's candidate list needs, one warp each; the embedded
-// error of every candidate at the trial step; the first one within the
+// basis, the singlet Gram of the basis, k_plain_control (the embedded error of
+// every candidate dimension at the trial step; the first one within the
 // budget; the coefficient row of the new state and the populations and
 // error estimates at the step's observation points), and k_plain_combine
 // (the new state and its norm).  The host only keeps the step-size logic.
-// records for dimensions <= 64: [0] size, [1] status, eigenvalues, eigenvectors by columns
+//
+// exp(-i T t) e1 comes from the Chebyshev series of the tridiagonal itself,
+//   sum_k (2 - delta_k0) (-i)^k J_k(r t) T_k((T - c) / r) e1,
+// r and c from Gershgorin's circles, J_k by Miller's backward recurrence: one
+// warp per (candidate, time), two entries of the vector per lane, about
+// r t + 13 (r t)^(1/3) steps of a neighbour exchange and three multiply-adds.
+// T_d and T_(d - offset) run side by side with the same coefficients, and no
+// eigen-decomposition is needed (serial implicit QR of every candidate: 390
+// us per step at 30, 630 us at 40 dimensions).
 constexpr int kPlainLD = 64;
-constexpr int kPlainRec = 2 + kPlainLD + kPlainLD * kPlainLD;  // doubles per spectra record
 constexpr int kPlainWarps = 16;
 constexpr int kPlainMaxCand = 15;                             // candidate dimensions per step
-constexpr int kPlainMaxDims = 2 * kPlainMaxCand + 1;
+constexpr double kChebMaxArg = 256.0;  // longer times go in equal parts
+constexpr int kChebTerms = 384;         // >= 256 + 13 * 256^(1/3) + 14 + the recurrence's head start
 
 struct PlainIn {
   int mode;  // 0: the minimum dimension alone; 1: ladder from the minimum; 2: ladder from minimum + increment
@@ -610,92 +617,240 @@ struct PlainOut {
   double err, norm, new_norm;
 };
 
-// c_i(t) = sum_k z_ik exp(-i lambda_k t) z_0k for i < m of one record, by one
-// warp into warp-private c (the arithmetic of spectral_coefficients).
-static __device__ void warp_coefficients(const double* rec, double t, double2* ph, double2* c) {
+// Series length that leaves a remainder below 1e-17 for argument x.
+static __device__ __forceinline__ int cheb_terms(double x) { return (int)(x + 13.0 * cbrt(x)) + 14; }
+
+// bes[k] = J_k(x), k <= K, by one warp: backwards from a start eight orders
+// above K, normalised by J_0^2 + 2 sum J_k^2 = 1 (every J_k above the
+// argument is positive, which fixes the sign).
+static __device__ void warp_bessel(double x, int K, double* bes) {
+  if ((threadIdx.x & 31) == 0) {
+    if (x == 0.0) {
+      for (int k = 1; k <= K; ++k) bes[k] = 0.0;
+      bes[0] = 1.0;
+    } else {
+      const double two = 2.0 / x;
+      double hi = 0.0, now = 1e-60, sum = 0.0;
+      for (int k = K + 8; k >= 1; --k) {
+        if (k <= K) bes[k] = now;
+        sum = fma(now, now, sum);
+        const double lower = fma(k * two, now, -hi);
+        hi = now;
+        now = lower;
+        if (fabs(now) > 1e90) {  // small arguments: the ratio to J_0 leaves the range of the squares
+          now *= 1e-120;
+          hi *= 1e-120;
+          sum *= 1e-240;
+          for (int q = k; q <= K; ++q) bes[q] *= 1e-120;
+        }
+      }
+      bes[0] = now;
+      const double inv = 1.0 / sqrt(fma(2.0, sum, now * now));
+      for (int k = 0; k <= K; ++k) bes[k] *= inv;
+    }
+  }
+  __syncwarp();
+}
+
+// One tridiagonal's share of the series: lane holds the vector entries
+// NE lane .. NE lane + NE - 1.
+template <int NE>
+struct ChebRow {
+  double diag[NE], off[NE + 1];  // scaled diagonal; couplings to entry NE lane - 1 + i and the next
+  double re[NE], im[NE];         // start vector
+  __device__ void load(const double* d, const double* o, int dim, int lane) {
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+      const int i = NE * lane + e;
+      diag[e] = i < dim ? d[i] : 0.0;
+      off[e] = i > 0 && i < dim ? o[i - 1] : 0.0;
+      re[e] = i == 0 ? 1.0 : 0.0;
+      im[e] = 0.0;
+    }
+    const int next = NE * lane + NE;
+    off[NE] = next < dim ? o[next - 1] : 0.0;
+  }
+  // (now, before) <- (c T now - before, now)
+  __device__ void recur(double c, double (&now)[NE], double (&before)[NE]) const {
+    const double left = __shfl_up_sync(0xffffffffu, now[NE - 1], 1), right = __shfl_down_sync(0xffffffffu, now[0], 1);
+    double y[NE];
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+      const double l = e ? now[e - 1] : left, r = e + 1 < NE ? now[e + 1] : right;
+      y[e] = fma(c, fma(diag[e], now[e], fma(off[e], l, off[e + 1] * r)), -before[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+      before[e] = now[e];
+      now[e] = y[e];
+    }
+  }
+  // start <- phase * sum_k (2 - delta) (-i)^k J_k T_k start
+  __device__ void advance(const double* bes, int K, double2 phase, bool complex_start) {
+    double a[NE], b[NE], e[NE], f[NE], sr[NE], si[NE];
+#pragma unroll
+    for (int i = 0; i < NE; ++i) {
+      a[i] = re[i];
+      e[i] = im[i];
+      b[i] = f[i] = sr[i] = si[i] = 0.0;
+    }
+    for (int k = 0; k <= K; ++k) {
+      const double w = (k & 2 ? -1.0 : 1.0) * (k ? 2.0 : 1.0) * bes[k];
+#pragma unroll
+      for (int i = 0; i < NE; ++i) {
+        if (k & 1) {  // (-i)^k = -i, i
+          si[i] = fma(-w, a[i], si[i]);
+          sr[i] = fma(w, e[i], sr[i]);
+        } else {
+          sr[i] = fma(w, a[i], sr[i]);
+          si[i] = fma(w, e[i], si[i]);
+        }
+      }
+      recur(k ? 2.0 : 1.0, a, b);
+      if (complex_start) recur(k ? 2.0 : 1.0, e, f);
+    }
+#pragma unroll
+    for (int i = 0; i < NE; ++i) {
+      re[i] = fma(sr[i], phase.x, -si[i] * phase.y);
+      im[i] = fma(sr[i], phase.y, si[i] * phase.x);
+    }
+  }
+};
+
+// The scaled tridiagonal of a basis: (T - centre) / radius.
+struct ChebScale {
+  double centre, radius;
+};
+
+// Gershgorin interval of the whole tridiagonal (its leading blocks lie
+// inside), and diag / off scaled with it, by one warp; false: not finite.
+static __device__ bool warp_scale(const double* alpha, const double* beta, int size, double* diag, double* off,
+                                  ChebScale* sc) {
   const int lane = threadIdx.x & 31;
-  const int m = (int)rec[0];
-  const double* lam = rec + 2;
-  const double* z = rec + 2 + kPlainLD;
-  for (int k = lane; k < m; k += 32) {
-    double s, co;
-    sincos(lam[k] * t, &s, &co);
-    const double w = z[k * kPlainLD];  // first component of eigenvector k
-    ph[k] = make_double2(co * w, -s * w);
+  double lo = DBL_MAX, hi = -DBL_MAX;
+  bool bad = false;
+  for (int i = lane; i < size; i += 32) {
+    const double a = alpha[i];
+    const double r = (i > 0 ? fabs(beta[i - 1]) : 0.0) + (i + 1 < size ? fabs(beta[i]) : 0.0);
+    bad = bad || !isfinite(a) || !isfinite(r);
+    lo = fmin(lo, a - r);
+    hi = fmax(hi, a + r);
   }
-  __syncwarp();
-  for (int i = lane; i < m; i += 32) {
-    double2 acc = make_double2(0.0, 0.0);
-    for (int k = 0; k < m; ++k) {
-      const double zz = z[k * kPlainLD + i];
-      acc.x = fma(zz, ph[k].x, acc.x);
-      acc.y = fma(zz, ph[k].y, acc.y);
-    }
-    c[i] = acc;
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
   }
+  const double centre = 0.5 * (lo + hi), radius = 0.5 * (hi - lo), inv = radius > 0.0 ? 1.0 / radius : 0.0;
+  for (int i = lane; i < size; i += 32) {
+    diag[i] = (alpha[i] - centre) * inv;
+    off[i] = i + 1 < size ? beta[i] * inv : 0.0;
+  }
+  if (lane == 0) *sc = ChebScale{centre, radius};
   __syncwarp();
+  return !__any_sync(0xffffffffu, bad);
 }
 
-// |c_hi - [c_lo; 0]|^2 over the warp.
-static __device__ double warp_diff2(const double2* ch, int mh, const double2* cl, int ml) {
+// ch = exp(-i T_mh t) e1 (32 NE entries) by one warp; returns
+// |ch - [exp(-i T_ml t) e1; 0]|^2 (0 for ml = 0).
+template <int NE>
+static __device__ double warp_exp_e1(const double* diag, const double* off, ChebScale sc, int mh, int ml, double t,
+                                     double* bes, double2* ch) {
+  const int lane = threadIdx.x & 31;
+  const int parts = max(1, (int)ceil(sc.radius * t / kChebMaxArg));
+  const double tau = t / parts, x = sc.radius * tau;
+  const int K = min(cheb_terms(x), kChebTerms - 1);
+  warp_bessel(x, K, bes);
+  double s, c;
+  sincos(sc.centre * tau, &s, &c);
+  const double2 phase = make_double2(c, -s);
+  ChebRow<NE> hi, lo;
+  hi.load(diag, off, mh, lane);
+  lo.load(diag, off, ml, lane);
+  for (int p = 0; p < parts; ++p) {
+    hi.advance(bes, K, phase, p > 0);
+    if (ml > 0) lo.advance(bes, K, phase, p > 0);
+  }
   double acc = 0.0;
-  for (int i = threadIdx.x & 31; i < mh; i += 32) {
-    double2 d = ch[i];
-    if (i < ml) {
-      d.x -= cl[i].x;
-      d.y -= cl[i].y;
-    }
-    acc = fma(d.x, d.x, fma(d.y, d.y, acc));
+#pragma unroll
+  for (int e = 0; e < NE; ++e) {
+    ch[NE * lane + e] = make_double2(hi.re[e], hi.im[e]);
+    const double x0 = hi.re[e] - lo.re[e], y0 = hi.im[e] - lo.im[e];
+    acc = fma(x0, x0, fma(y0, y0, acc));
   }
-  return warp_sum(acc);
+  acc = ml > 0 ? warp_sum(acc) : 0.0;
+  __syncwarp();
+  return acc;
 }
 
-constexpr size_t kPlainSmem = sizeof(double) * kPlainWarps * 2 * kPlainLD + sizeof(double2) * kPlainWarps * 4 * kPlainLD;
+// sum_ij conj(c_i) G_ij c_j over the leading m entries, one warp; G Hermitian, read by rows.
+static __device__ double warp_quadratic(const double2* gram, int ld, const double2* c, int m) {
+  double v = 0.0;
+  for (int i = threadIdx.x & 31; i < m; i += 32) {
+    double2 gc = make_double2(0.0, 0.0);
+    for (int k = 0; k < m; ++k) gc = cfma_conj(gram[(size_t)k * ld + i], c[k], gc);
+    v += c[i].x * gc.x + c[i].y * gc.y;
+  }
+  return warp_sum(v);
+}
+
+// rpm_krylov_coefficients: one warp per request (dimensions up to 32 NE).
+template <int NE>
+__global__ void __launch_bounds__(32) k_krylov_coefficients(const double* __restrict__ alpha,
+                                                            const double* __restrict__ beta, int size,
+                                                            const rpm_krylov_req* reqs, double safety,
+                                                            double state_norm, const double2* __restrict__ gram,
+                                                            int gram_ld, double2* coef, int coef_ld, double* err_out,
+                                                            double* value_out) {
+  __shared__ double diag[32 * NE], off[32 * NE], bes[kChebTerms];
+  __shared__ double2 ch[32 * NE];
+  __shared__ ChebScale sc;
+  const rpm_krylov_req rq = reqs[blockIdx.x];
+  warp_scale(alpha, beta, size, diag, off, &sc);
+  const double e2 = warp_exp_e1<NE>(diag, off, sc, rq.hi, max(rq.lo, 0), rq.time, bes, ch);
+  for (int i = threadIdx.x; i < rq.hi; i += 32) coef[(size_t)blockIdx.x * coef_ld + i] = ch[i];
+  const double v = gram ? warp_quadratic(gram, gram_ld, ch, rq.hi) : 0.0;
+  if (threadIdx.x == 0) {
+    err_out[blockIdx.x] = rq.lo > 0 ? safety * state_norm * sqrt(e2) : 0.0;
+    if (gram) value_out[blockIdx.x] = state_norm * state_norm * v;
+  }
+}
+
+constexpr size_t kPlainSmem = kPlainWarps * (sizeof(double2) * kPlainLD + sizeof(double) * kChebTerms);
 
 __global__ void __launch_bounds__(kPlainWarps * 32) k_plain_control(const double* __restrict__ alpha,
                                                                    const double* __restrict__ beta,
-                                                                   const LanczosScalars* sc, PlainIn in, double* recs,
+                                                                   const LanczosScalars* sc, PlainIn in,
                                                                    const double2* __restrict__ gram,
                                                                    const double* __restrict__ times, double* values,
                                                                    double* perr, double2* coef, PlainOut* out) {
-  extern __shared__ double psm[];
-  __shared__ int s_dims[kPlainMaxDims], s_hi[kPlainMaxCand], s_lo[kPlainMaxCand];
-  __shared__ int s_ndims, s_ncand, s_status, s_sel, s_size, s_exact, s_bad;
+  extern __shared__ __align__(16) unsigned char praw[];
+  __shared__ double s_diag[kPlainLD], s_off[kPlainLD];
+  __shared__ int s_hi[kPlainMaxCand], s_lo[kPlainMaxCand];  // candidate dimensions (lo 0: exact)
+  __shared__ int s_ncand, s_status, s_sel, s_size, s_exact;
   __shared__ double s_err[kPlainMaxCand], s_norm;
+  __shared__ ChebScale s_scale;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* dd = psm + warp * 2 * kPlainLD;
-  double* ee = dd + kPlainLD;
-  double2* wb = reinterpret_cast<double2*>(psm + kPlainWarps * 2 * kPlainLD) + warp * 4 * kPlainLD;
-  double2* rot = wb;
-  double2* ph = wb + kPlainLD;
-  double2* ch = wb + 2 * kPlainLD;
-  double2* cl = wb + 3 * kPlainLD;
+  double2* ch = reinterpret_cast<double2*>(praw) + warp * kPlainLD;
+  double* bes = reinterpret_cast<double*>(praw + sizeof(double2) * kPlainWarps * kPlainLD) + warp * kChebTerms;
   if (threadIdx.x == 0) {
     const int stop = sc->stop;
     s_norm = sc->norm;
-    s_bad = 0;
     const int size = stop > 0 ? stop : in.built;
     const int exact = size < in.target;
-    int nd = 0, nc = 0;
-    auto record = [&](int d) {
-      for (int i = 0; i < nd; ++i)
-        if (s_dims[i] == d) return i;
-      s_dims[nd] = d;
-      return nd++;
-    };
+    int nc = 0;
     // (d, d - offset) as the reference's candidate evaluation (ENG:690-715)
     auto add = [&](int d) {
       d = min(d, size);
       const int lo = max(1, d - in.offset);
-      s_hi[nc] = record(d);
-      s_lo[nc] = lo == d ? -1 : record(lo);
+      s_hi[nc] = d;
+      s_lo[nc] = lo == d ? 0 : lo;
       ++nc;
     };
     if (stop < 0) {
       nc = 0;
     } else if (exact) {
-      s_hi[0] = record(size);
-      s_lo[0] = -1;
+      s_hi[0] = size;
+      s_lo[0] = 0;
       nc = 1;
     } else if (in.mode == 0) {
       add(in.min_dim);
@@ -710,40 +865,23 @@ __global__ void __launch_bounds__(kPlainWarps * 32) k_plain_control(const double
     s_status = sc->timeout ? 5 : stop < 0 ? 4 : 0;
     s_size = stop < 0 ? 0 : size;
     s_exact = exact;
-    s_ndims = nd;
     s_ncand = nc;
   }
   __syncthreads();
   if (s_status == 0) {
-    for (int r = warp; r < s_ndims; r += kPlainWarps) {
-      const int dim = s_dims[r];
-      double* rec = recs + (size_t)r * kPlainRec;
-      for (int i = lane; i < dim; i += 32) {
-        dd[i] = alpha[i];
-        ee[i] = (i + 1 < dim) ? beta[i] : 0.0;
-      }
-      __syncwarp();
-      const int bad = tridiag_qr_warp_cols<false>(dim, dd, ee, rec + 2 + kPlainLD, kPlainLD, rot);
-      for (int i = lane; i < dim; i += 32) rec[2 + i] = dd[i];
-      if (lane == 0) {
-        rec[0] = dim;
-        rec[1] = bad;
-        if (bad) s_bad = 1;
-      }
-      __syncwarp();
+    const int size = s_size;
+    if (warp == 0) {
+      const bool fine = warp_scale(alpha, beta, size, s_diag, s_off, &s_scale);
+      if (lane == 0 && !fine) s_status = 3;
     }
     __syncthreads();
+  }
+  if (s_status == 0) {
     for (int c = warp; c < s_ncand; c += kPlainWarps) {
-      const double* rh = recs + (size_t)s_hi[c] * kPlainRec;
-      double e2 = 0.0;
-      if (s_lo[c] >= 0) {
-        const double* rl = recs + (size_t)s_lo[c] * kPlainRec;
-        warp_coefficients(rh, in.trial, ph, ch);
-        warp_coefficients(rl, in.trial, ph, cl);
-        e2 = warp_diff2(ch, (int)rh[0], cl, (int)rl[0]);
-      }
-      if (lane == 0) s_err[c] = s_lo[c] >= 0 ? in.safety * s_norm * sqrt(e2) : 0.0;
-      __syncwarp();
+      double err = 0.0;
+      if (s_lo[c] > 0)
+        err = in.safety * s_norm * sqrt(warp_exp_e1<2>(s_diag, s_off, s_scale, s_hi[c], s_lo[c], in.trial, bes, ch));
+      if (lane == 0) s_err[c] = err;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -754,40 +892,28 @@ __global__ void __launch_bounds__(kPlainWarps * 32) k_plain_control(const double
           break;
         }
       s_sel = sel;
-      s_status = s_bad ? 3 : sel >= 0 ? 0 : (in.mode == 0 && in.max_dim > in.min_dim ? 2 : 1);
+      s_status = sel >= 0 ? 0 : (in.mode == 0 && in.max_dim > in.min_dim ? 2 : 1);
     }
     __syncthreads();
   }
   const int status = s_status;
   if (status == 0) {
-    const int sel = s_sel;
-    const double* rh = recs + (size_t)s_hi[sel] * kPlainRec;
-    const double* rl = s_lo[sel] >= 0 ? recs + (size_t)s_lo[sel] * kPlainRec : nullptr;
-    const int mh = (int)rh[0], ml = rl ? (int)rl[0] : 0;
-    if (warp == 0) {
-      warp_coefficients(rh, in.trial, ph, ch);
-      for (int i = lane; i < mh; i += 32) coef[i] = ch[i];
-    }
+    const int mh = s_hi[s_sel], ml = s_lo[s_sel];
     const double nn = s_norm * s_norm;
-    for (int p = warp; p < in.npts; p += kPlainWarps) {
-      const double dt = times[in.first + p] - in.t_now;
-      warp_coefficients(rh, dt, ph, ch);
-      double e2 = 0.0;
-      if (rl) {
-        warp_coefficients(rl, dt, ph, cl);
-        e2 = warp_diff2(ch, mh, cl, ml);
+    // point npts: the end of the step (its coefficients make the new state)
+    for (int p = warp; p <= in.npts; p += kPlainWarps) {
+      const bool endpoint = p == in.npts;
+      const double dt = endpoint ? in.trial : times[in.first + p] - in.t_now;
+      const double e2 = warp_exp_e1<2>(s_diag, s_off, s_scale, mh, endpoint ? 0 : ml, dt, bes, ch);
+      if (endpoint) {
+        for (int i = lane; i < mh; i += 32) coef[i] = ch[i];
+        __syncwarp();
+        continue;
       }
-      // c^H G c with the singlet Gram of the basis (leading dimension: the basis size)
-      double v = 0.0;
-      for (int i = lane; i < mh; i += 32) {
-        double2 gc = make_double2(0.0, 0.0);
-        for (int k = 0; k < mh; ++k) gc = cfma(gram[(size_t)i * in.built + k], ch[k], gc);
-        v += ch[i].x * gc.x + ch[i].y * gc.y;
-      }
-      v = warp_sum(v);
+      const double v = warp_quadratic(gram, in.built, ch, mh);
       if (lane == 0) {
         values[in.first + p] = nn * v;
-        perr[in.first + p] = rl ? in.safety * s_norm * sqrt(e2) : 0.0;
+        perr[in.first + p] = ml > 0 ? in.safety * s_norm * sqrt(e2) : 0.0;
       }
       __syncwarp();
     }
@@ -799,10 +925,9 @@ __global__ void __launch_bounds__(kPlainWarps * 32) k_plain_control(const double
     o.exact = s_exact;
     o.norm = s_norm;
     if (status == 0) {
-      const int sel = s_sel;
-      o.selected = (int)recs[(size_t)s_hi[sel] * kPlainRec];
-      o.lo = s_lo[sel] >= 0 ? (int)recs[(size_t)s_lo[sel] * kPlainRec] : 0;
-      o.err = s_err[sel];
+      o.selected = s_hi[s_sel];
+      o.lo = s_lo[s_sel];
+      o.err = s_err[s_sel];
     }
     *out = o;
   }
@@ -849,16 +974,11 @@ __global__ void __launch_bounds__(kThreads) k_plain_combine(const double2* __res
   }
 }
 
-// Device buffers of one plain propagation (stream-ordered allocation).
+// Device buffers of a plain propagation, kept with the system (SLOT_PLAIN).
 struct PlainBuffers {
-  cudaStream_t st = nullptr;
-  void* base = nullptr;
   double2 *basis = nullptr, *gram = nullptr, *coef = nullptr;
-  double *alpha = nullptr, *beta = nullptr, *recs = nullptr, *times = nullptr, *values = nullptr, *perr = nullptr;
+  double *alpha = nullptr, *beta = nullptr, *times = nullptr, *values = nullptr, *perr = nullptr;
   PlainOut* out = nullptr;
-  ~PlainBuffers() {
-    if (base) cudaFreeAsync(base, st);
-  }
 };
 
 static void plain_propagate(rpm_system* sys, const rpm_plain_knobs& k, double2* state, const double* times, int ntimes,
@@ -867,7 +987,6 @@ static void plain_propagate(rpm_system* sys, const rpm_plain_knobs& k, double2* 
   const long long n = sys->n;
   const int mmax = (int)std::min<long long>(k.maximum_dimension, n);
   PlainBuffers b;
-  b.st = st;
   size_t off = 0;
   auto take = [&](size_t bytes) {
     const size_t at = off;
@@ -876,23 +995,20 @@ static void plain_propagate(rpm_system* sys, const rpm_plain_knobs& k, double2* 
   };
   const size_t o_basis = take(sizeof(double2) * (size_t)mmax * n), o_gram = take(sizeof(double2) * 64 * 64),
                o_coef = take(sizeof(double2) * kPlainLD), o_alpha = take(sizeof(double) * kPlainLD),
-               o_beta = take(sizeof(double) * kPlainLD), o_recs = take(sizeof(double) * kPlainMaxDims * kPlainRec),
-               o_times = take(sizeof(double) * ntimes), o_values = take(sizeof(double) * ntimes),
+               o_beta = take(sizeof(double) * kPlainLD), o_times = take(sizeof(double) * ntimes), o_values = take(sizeof(double) * ntimes),
                o_perr = take(sizeof(double) * ntimes), o_out = take(sizeof(PlainOut));
-  check_cuda(cudaMallocAsync(&b.base, off, st), "cudaMallocAsync(plain propagation)");
-  char* base = static_cast<char*>(b.base);
+  // (a stream-ordered allocation per call was mapped anew each time: up to
+  // 80 ms for the full system's 145 MB)
+  char* base = static_cast<char*>(system_scratch(sys, SLOT_PLAIN, off));
   b.basis = reinterpret_cast<double2*>(base + o_basis);
   b.gram = reinterpret_cast<double2*>(base + o_gram);
   b.coef = reinterpret_cast<double2*>(base + o_coef);
   b.alpha = reinterpret_cast<double*>(base + o_alpha);
   b.beta = reinterpret_cast<double*>(base + o_beta);
-  b.recs = reinterpret_cast<double*>(base + o_recs);
   b.times = reinterpret_cast<double*>(base + o_times);
   b.values = reinterpret_cast<double*>(base + o_values);
   b.perr = reinterpret_cast<double*>(base + o_perr);
   b.out = reinterpret_cast<PlainOut*>(base + o_out);
-  // basis slots beyond a breakdown stay finite for the Gram
-  check_cuda(cudaMemsetAsync(b.base, 0, off, st), "cudaMemsetAsync(plain propagation)");
   check_cuda(cudaMemcpyAsync(b.times, times, sizeof(double) * ntimes, cudaMemcpyHostToDevice, st), "copy times");
   static bool attr = false;
   if (!attr) {
@@ -907,8 +1023,8 @@ static void plain_propagate(rpm_system* sys, const rpm_plain_knobs& k, double2* 
   auto run = [&](const PlainIn& in) {
     lanczos_basis_launch(sys, state, in.target, k.breakdown_tolerance, b.basis, b.alpha, b.beta, st);
     if (in.npts > 0) singlet_gram_launch(sys, b.basis, in.built, b.gram, st);
-    k_plain_control<<<1, kPlainWarps * 32, kPlainSmem, st>>>(b.alpha, b.beta, sc, in, b.recs, b.gram, b.times,
-                                                            b.values, b.perr, b.coef, b.out);
+    k_plain_control<<<1, kPlainWarps * 32, kPlainSmem, st>>>(b.alpha, b.beta, sc, in, b.gram, b.times, b.values,
+                                                            b.perr, b.coef, b.out);
     k_plain_combine<<<nb, kThreads, 0, st>>>(b.basis, n, b.coef, state, partials, &sc->counter[6], b.out);
     check_launch("plain step");
     check_cuda(cudaMemcpyAsync(&o, b.out, sizeof(PlainOut), cudaMemcpyDeviceToHost, st), "copy step record");
@@ -1058,6 +1174,39 @@ int rpm_krylov_eval(const double* spectra_dev, int nreq, const rpm_krylov_req* r
       check_cuda(cudaMemcpyAsync(value_host, d_val, sizeof(double) * nreq, cudaMemcpyDeviceToHost, st), "copy values");
     check_cuda(cudaFreeAsync(dbuf, st), "cudaFreeAsync(eval)");
     check_cuda(cudaStreamSynchronize(st), "eval sync");
+  });
+}
+
+int rpm_krylov_coefficients(const double* alpha_dev, const double* beta_dev, int size, int nreq,
+                            const rpm_krylov_req* reqs_host, double safety, double state_norm, const void* gram_dev,
+                            int gram_ld, void* coef_dev, int coef_ld, double* err_host, double* value_host,
+                            void* stream) {
+  return guarded([&] {
+    if (!alpha_dev || !beta_dev || nreq < 1 || !reqs_host || !coef_dev || !err_host) fail(RPM_E_INVALID, "bad arguments");
+    if (gram_dev && !value_host) fail(RPM_E_INVALID, "value_host required with a Gram matrix");
+    if (size < 1 || size > RPM_MAX_KRYLOV) fail(RPM_E_UNSUPPORTED, "Krylov dimension must be in [1, 128]");
+    for (int k = 0; k < nreq; ++k)
+      if (reqs_host[k].hi < 1 || reqs_host[k].hi > size || reqs_host[k].lo > reqs_host[k].hi ||
+          !(reqs_host[k].time >= 0.0) || reqs_host[k].hi > coef_ld || (gram_dev && reqs_host[k].hi > gram_ld))
+        fail(RPM_E_INVALID, "bad coefficient request");
+    auto st = static_cast<cudaStream_t>(stream);
+    const size_t req_bytes = sizeof(rpm_krylov_req) * nreq;
+    void* dbuf = nullptr;
+    check_cuda(cudaMallocAsync(&dbuf, req_bytes + sizeof(double) * 2 * nreq, st), "cudaMallocAsync(coefficients)");
+    auto* d_req = static_cast<rpm_krylov_req*>(dbuf);
+    auto* d_err = reinterpret_cast<double*>(static_cast<char*>(dbuf) + req_bytes);
+    double* d_val = d_err + nreq;
+    check_cuda(cudaMemcpyAsync(d_req, reqs_host, req_bytes, cudaMemcpyHostToDevice, st), "copy reqs");
+    auto* kern = size <= 64 ? k_krylov_coefficients<2> : k_krylov_coefficients<4>;
+    kern<<<nreq, 32, 0, st>>>(alpha_dev, beta_dev, size, d_req, safety, state_norm,
+                              static_cast<const double2*>(gram_dev), gram_ld, static_cast<double2*>(coef_dev), coef_ld,
+                              d_err, d_val);
+    check_launch("k_krylov_coefficients");
+    check_cuda(cudaMemcpyAsync(err_host, d_err, sizeof(double) * nreq, cudaMemcpyDeviceToHost, st), "copy err");
+    if (gram_dev)
+      check_cuda(cudaMemcpyAsync(value_host, d_val, sizeof(double) * nreq, cudaMemcpyDeviceToHost, st), "copy values");
+    check_cuda(cudaFreeAsync(dbuf, st), "cudaFreeAsync(coefficients)");
+    check_cuda(cudaStreamSynchronize(st), "coefficients sync");
   });
 }
 

@@ -155,13 +155,9 @@ static __device__ int tridiag_qr(int m, double* d, double* e, double* z, int ldz
 // rotations to its rows of the eigenvector matrix.  d, e: diagonal and
 // off-diagonal (d -> eigenvalues); m <= 64.  z: m x m eigenvector matrix
 // stored by columns, z[k * ldz + i] = component i of eigenvector k, so that
-// the lanes' row updates touch consecutive addresses.  FAST = true normalises
-// the rotations with rsqrt and carries the entries the next rotation reads in
-// registers; FAST = false keeps the block-wide solver's arithmetic exactly
-// (hypot and two divisions, operands re-read from memory), so that the plain
-// path's decisions stay those matched to the reference.  Returns 0 on
-// convergence.
-template <bool FAST>
+// the lanes' row updates touch consecutive addresses.  The rotations are
+// normalised with rsqrt and carry the entries the next rotation reads in
+// registers.  Returns 0 on convergence.
 static __device__ int tridiag_qr_warp_cols(int m, double* d, double* e, double* z, int ldz, double2* rot) {
   const int lane = threadIdx.x & 31;
   for (int idx = lane; idx < m * m; idx += 32) {
@@ -192,33 +188,7 @@ static __device__ int tridiag_qr_warp_cols(int m, double* d, double* e, double* 
     if (++sweeps > 40 * m) return 1;
     const unsigned long long below = q >= 2 ? (~nzm) & ((1ull << (q - 1)) - 1ull) : 0ull;
     const int p = below ? 64 - __clzll(below) : 0;
-    if (lane == 0 && !FAST) {
-      const double delta = 0.5 * (d[q - 1] - d[q]);
-      const double eq = e[q - 1];
-      const double denom = delta + copysign(hypot(delta, eq), delta);
-      const double mu = d[q] - eq * eq / denom;
-      double x = d[p] - mu, y = e[p];
-      for (int k = p; k < q; ++k) {
-        double c = 1.0, sn = 0.0;
-        const double r = hypot(x, y);
-        if (r > 0.0) {
-          c = x / r;
-          sn = y / r;
-        }
-        if (k > p) e[k - 1] = r;
-        const double a = d[k], bb = e[k], cc = d[k + 1];
-        d[k] = c * c * a + 2.0 * c * sn * bb + sn * sn * cc;
-        d[k + 1] = sn * sn * a - 2.0 * c * sn * bb + c * c * cc;
-        e[k] = c * sn * (cc - a) + (c * c - sn * sn) * bb;
-        if (k + 1 < q) {
-          x = e[k];
-          y = sn * e[k + 1];
-          e[k + 1] = c * e[k + 1];
-        }
-        rot[k] = make_double2(c, sn);
-      }
-    }
-    if (lane == 0 && FAST) {
+    if (lane == 0) {
       const double delta = 0.5 * (d[q - 1] - d[q]);
       const double eq = e[q - 1];
       const double denom = delta + copysign(hypot(delta, eq), delta);

@@ -370,7 +370,7 @@ class SingletPopulationObservable:
     """Singlet population with the exact Krylov-basis projection shortcut (ENG:500-538).
 
     With this observable the propagator evaluates ``V^H P_S V`` and every
-    population on the GPU (rpm_singlet_gram / rpm_krylov_eval).
+    population on the GPU (rpm_singlet_gram / rpm_krylov_coefficients).
     """
 
     def __init__(self, dimensions: Iterable[int]) -> None:
@@ -458,27 +458,13 @@ class PropagationResult:
 # Plain FP64 propagator
 # ---------------------------------------------------------------------------
 
+@dataclass(frozen=True)
 class _Krylov:
-    """Device tridiagonal (alpha, beta) + its spectra, for one basis build."""
+    """One basis build: the size of its device tridiagonal (alpha, beta) and
+    ||state|| as the basis was normalised with."""
 
-    def __init__(self, prop, size: int, norm: float):
-        self.prop = prop
-        self.size = size
-        self.norm = norm  # ||state|| as the basis was normalised with
-        self._records: dict[int, int] = {}
-
-    def spectra(self, dims):
-        """Ensure spectra records exist for every d in ``dims``; return their indices."""
-        want = [d for d in dict.fromkeys(dims) if d not in self._records]
-        if want:
-            base = len(self._records)
-            arr = np.asarray(want, dtype=np.int32)
-            target = self.prop._spectra[base:base + len(want)]
-            _lib.call("rpm_tridiag_spectra", _lib.ptr(self.prop._alpha), _lib.ptr(self.prop._beta), len(want),
-                      _lib.iptr(arr), _lib.ptr(target), _lib.stream_handle())
-            for k, d in enumerate(want):
-                self._records[d] = base + k
-        return [self._records[d] for d in dims]
+    size: int
+    norm: float
 
 
 class AdaptiveLanczosPropagator:
@@ -527,7 +513,6 @@ class AdaptiveLanczosPropagator:
             self._basis_buf = torch.empty((m, n), dtype=torch.complex128, device="cuda")
             self._alpha = torch.zeros(m, dtype=torch.float64, device="cuda")
             self._beta = torch.zeros(max(m, 1), dtype=torch.float64, device="cuda")
-            self._spectra = torch.zeros((4 * m + 8, _lib.RPM_SPECTRUM_DOUBLES), dtype=torch.float64, device="cuda")
             self._gram = torch.empty((min(m, 64), min(m, 64)), dtype=torch.complex128, device="cuda")
             self._buffers_for = key
         return self._basis_buf
@@ -542,27 +527,21 @@ class AdaptiveLanczosPropagator:
                   float(self.breakdown_tolerance), _lib.ptr(basis), _lib.ptr(self._alpha), _lib.ptr(self._beta),
                   ctypes.byref(actual), ctypes.byref(norm), _lib.stream_handle())
         self.hamiltonian.matvec_count += actual.value
-        return _Krylov(self, actual.value, norm.value)
+        return _Krylov(actual.value, norm.value)
 
     def _evaluate(self, kry: _Krylov, pairs, times, state_norm, gram=None):
         """Coefficients/errors/values for (dimension, embedded dimension or None) at times."""
         torch = _torch()
-        dims = []
-        for d, lo in pairs:
-            dims.append(d)
-            if lo is not None:
-                dims.append(lo)
-        idx = dict(zip(dims, kry.spectra(dims)))
         reqs = (_lib.rpm_krylov_req * len(pairs))()
         for k, ((d, lo), t) in enumerate(zip(pairs, times)):
-            reqs[k].hi = idx[d]
-            reqs[k].lo = -1 if lo is None else idx[lo]
+            reqs[k].hi = d
+            reqs[k].lo = -1 if lo is None else lo
             reqs[k].time = float(t)
         coef = torch.zeros((len(pairs), _lib.RPM_MAX_KRYLOV), dtype=torch.complex128, device="cuda")
         err = np.zeros(len(pairs))
         val = np.zeros(len(pairs))
-        _lib.call("rpm_krylov_eval", _lib.ptr(self._spectra), len(pairs), reqs, float(self.safety_factor),
-                  float(state_norm), _lib.ptr(gram) if gram is not None else None,
+        _lib.call("rpm_krylov_coefficients", _lib.ptr(self._alpha), _lib.ptr(self._beta), int(kry.size), len(pairs),
+                  reqs, float(self.safety_factor), float(state_norm), _lib.ptr(gram) if gram is not None else None,
                   int(gram.shape[1]) if gram is not None else 0, _lib.ptr(coef), _lib.RPM_MAX_KRYLOV,
                   _lib.dptr(err), _lib.dptr(val), _lib.stream_handle())
         return coef, err, val
