@@ -252,6 +252,13 @@ enum Slot : int {
   SLOT_PLAIN = 5,     // basis and step buffers of the device-driven plain propagation
 };
 void* system_scratch(rpm_system* sys, int slot, size_t bytes);
+// Stream-ordered scratch of one call, from a memory pool of the library's own
+// (one per device) that keeps up to kPoolKeep bytes mapped between calls; the
+// default pool unmaps its memory at every synchronisation, which made a small
+// allocation cost half a millisecond.  Trimmed when the last system goes.
+constexpr size_t kPoolKeep = (size_t)64 << 20;  // (the driver maps 32 MB at a time)
+void* pool_alloc(size_t bytes, cudaStream_t stream);
+void pool_free(void* p, cudaStream_t stream);
 // H psi launchers (hpsi.cu).  `scale_dev`, when non-null, multiplies the input
 // by 1/scale_dev[0] on load (used to fold normalisation into H psi).
 template <class T>

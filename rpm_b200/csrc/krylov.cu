@@ -427,17 +427,19 @@ __global__ void __launch_bounds__(kThreads) k_combine(const double2* __restrict_
   }
 }
 
-// Per-vector reductions over a batch: kind 0 = ||x||^2, kind 1 = singlet population.
+// Per-vector reductions over a batch: kind 0 = ||x||^2, kind 1 = singlet
+// population; block partials of vector blockIdx.y at out[vector * gridDim.x].
 __global__ void __launch_bounds__(kThreads) k_batch_reduce(const double2* __restrict__ x, long long n, long long ld,
                                                           int kind, double* out) {
   __shared__ double red[kThreads / 32];
-  const double2* v = x + (long long)blockIdx.x * ld;
+  const double2* v = x + (long long)blockIdx.y * ld;
   double acc = 0.0;
+  const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
   if (kind == 0) {
-    for (long long i = threadIdx.x; i < n; i += blockDim.x) acc = fma(v[i].x, v[i].x, fma(v[i].y, v[i].y, acc));
+    for (long long i = first; i < n; i += stride) acc = fma(v[i].x, v[i].x, fma(v[i].y, v[i].y, acc));
   } else {
     const long long q = n / 4;
-    for (long long i = threadIdx.x; i < q; i += blockDim.x) {
+    for (long long i = first; i < q; i += stride) {
       const double2 a = v[q + i], b = v[2 * q + i];
       const double re = a.x - b.x, im = a.y - b.y;
       acc = fma(re, re, fma(im, im, acc));
@@ -450,7 +452,7 @@ __global__ void __launch_bounds__(kThreads) k_batch_reduce(const double2* __rest
   if (threadIdx.x == 0) {
     double s = 0.0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
-    out[blockIdx.x] = s;
+    out[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = s;
   }
 }
 
@@ -1138,8 +1140,7 @@ int rpm_tridiag_spectra(const double* alpha_dev, const double* beta_dev, int ndi
     for (int k = 0; k < ndims; ++k)
       if (dims_host[k] < 1 || dims_host[k] > RPM_MAX_KRYLOV) fail(RPM_E_UNSUPPORTED, "Krylov dimension must be in [1, 128]");
     auto st = static_cast<cudaStream_t>(stream);
-    int* d_dims = nullptr;
-    check_cuda(cudaMallocAsync(&d_dims, sizeof(int) * ndims, st), "cudaMallocAsync(dims)");
+    auto* d_dims = static_cast<int*>(pool_alloc(sizeof(int) * ndims, st));
     check_cuda(cudaMemcpyAsync(d_dims, dims_host, sizeof(int) * ndims, cudaMemcpyHostToDevice, st), "copy dims");
     const size_t smem = sizeof(double) * (RPM_MAX_KRYLOV * RPM_MAX_KRYLOV + 2 * RPM_MAX_KRYLOV) +
                         sizeof(double2) * RPM_MAX_KRYLOV;
@@ -1147,7 +1148,7 @@ int rpm_tridiag_spectra(const double* alpha_dev, const double* beta_dev, int ndi
                "cudaFuncSetAttribute(spectra)");
     k_tridiag_spectra<<<ndims, 128, smem, st>>>(alpha_dev, beta_dev, d_dims, spectra_dev);
     check_launch("k_tridiag_spectra");
-    check_cuda(cudaFreeAsync(d_dims, st), "cudaFreeAsync(dims)");
+    pool_free(d_dims, st);
   });
 }
 
@@ -1159,8 +1160,7 @@ int rpm_krylov_eval(const double* spectra_dev, int nreq, const rpm_krylov_req* r
     if (gram_dev && !value_host) fail(RPM_E_INVALID, "value_host required with a Gram matrix");
     auto st = static_cast<cudaStream_t>(stream);
     const size_t req_bytes = sizeof(rpm_krylov_req) * nreq;
-    void* dbuf = nullptr;
-    check_cuda(cudaMallocAsync(&dbuf, req_bytes + sizeof(double) * 2 * nreq, st), "cudaMallocAsync(eval)");
+    void* dbuf = pool_alloc(req_bytes + sizeof(double) * 2 * nreq, st);
     auto* d_req = static_cast<rpm_krylov_req*>(dbuf);
     auto* d_err = reinterpret_cast<double*>(static_cast<char*>(dbuf) + req_bytes);
     double* d_val = d_err + nreq;
@@ -1172,7 +1172,7 @@ int rpm_krylov_eval(const double* spectra_dev, int nreq, const rpm_krylov_req* r
     check_cuda(cudaMemcpyAsync(err_host, d_err, sizeof(double) * nreq, cudaMemcpyDeviceToHost, st), "copy err");
     if (gram_dev)
       check_cuda(cudaMemcpyAsync(value_host, d_val, sizeof(double) * nreq, cudaMemcpyDeviceToHost, st), "copy values");
-    check_cuda(cudaFreeAsync(dbuf, st), "cudaFreeAsync(eval)");
+    pool_free(dbuf, st);
     check_cuda(cudaStreamSynchronize(st), "eval sync");
   });
 }
@@ -1191,8 +1191,7 @@ int rpm_krylov_coefficients(const double* alpha_dev, const double* beta_dev, int
         fail(RPM_E_INVALID, "bad coefficient request");
     auto st = static_cast<cudaStream_t>(stream);
     const size_t req_bytes = sizeof(rpm_krylov_req) * nreq;
-    void* dbuf = nullptr;
-    check_cuda(cudaMallocAsync(&dbuf, req_bytes + sizeof(double) * 2 * nreq, st), "cudaMallocAsync(coefficients)");
+    void* dbuf = pool_alloc(req_bytes + sizeof(double) * 2 * nreq, st);
     auto* d_req = static_cast<rpm_krylov_req*>(dbuf);
     auto* d_err = reinterpret_cast<double*>(static_cast<char*>(dbuf) + req_bytes);
     double* d_val = d_err + nreq;
@@ -1205,7 +1204,7 @@ int rpm_krylov_coefficients(const double* alpha_dev, const double* beta_dev, int
     check_cuda(cudaMemcpyAsync(err_host, d_err, sizeof(double) * nreq, cudaMemcpyDeviceToHost, st), "copy err");
     if (gram_dev)
       check_cuda(cudaMemcpyAsync(value_host, d_val, sizeof(double) * nreq, cudaMemcpyDeviceToHost, st), "copy values");
-    check_cuda(cudaFreeAsync(dbuf, st), "cudaFreeAsync(coefficients)");
+    pool_free(dbuf, st);
     check_cuda(cudaStreamSynchronize(st), "coefficients sync");
   });
 }
@@ -1278,13 +1277,25 @@ static int batch_reduce(long long n, const void* psi, int batch, long long ld, i
     if (!psi || !host || batch < 1 || n < 1 || ld < n) fail(RPM_E_INVALID, "bad arguments");
     if (kind == 1 && n % 4 != 0) fail(RPM_E_INVALID, "The first two axes must be the two electron spins.");
     auto st = static_cast<cudaStream_t>(stream);
-    double* d_out = nullptr;
-    check_cuda(cudaMallocAsync(&d_out, sizeof(double) * batch, st), "cudaMallocAsync(reduce)");
-    k_batch_reduce<<<batch, kThreads, 0, st>>>(static_cast<const double2*>(psi), n, ld, kind, d_out);
-    check_launch("k_batch_reduce");
-    check_cuda(cudaMemcpyAsync(host, d_out, sizeof(double) * batch, cudaMemcpyDeviceToHost, st), "copy reduce");
-    check_cuda(cudaFreeAsync(d_out, st), "cudaFreeAsync(reduce)");
+    // a few blocks per vector (one left the full system's norm at 55 us), at
+    // most 65535 vectors a launch; the host adds the block partials in order
+    const int nb = (int)std::max<long long>(1, std::min<long long>(64, n / (4 * kThreads)));
+    std::vector<double> part((size_t)batch * nb);
+    auto* d_out = static_cast<double*>(pool_alloc(sizeof(double) * part.size(), st));
+    for (int b0 = 0; b0 < batch; b0 += 65535) {
+      k_batch_reduce<<<dim3(nb, std::min(65535, batch - b0)), kThreads, 0, st>>>(
+          static_cast<const double2*>(psi) + (long long)b0 * ld, n, ld, kind, d_out + (size_t)b0 * nb);
+      check_launch("k_batch_reduce");
+    }
+    check_cuda(cudaMemcpyAsync(part.data(), d_out, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, st),
+               "copy reduce");
+    pool_free(d_out, st);
     check_cuda(cudaStreamSynchronize(st), "reduce sync");
+    for (int b = 0; b < batch; ++b) {
+      double s = 0.0;
+      for (int k = 0; k < nb; ++k) s += part[(size_t)b * nb + k];
+      host[b] = s;
+    }
   });
 }
 
@@ -1354,13 +1365,12 @@ extern "C" int rpm_apply_local_operator(const int* dims, int ndims, int axis, co
     const int d = dims[axis];
     if (d > RPM_MAX_LOCAL_DIM) fail(RPM_E_UNSUPPORTED, "axis dimension above 64");
     auto st = static_cast<cudaStream_t>(stream);
-    double2* d_op = nullptr;
-    check_cuda(cudaMallocAsync(&d_op, sizeof(double2) * d * d, st), "cudaMallocAsync(op)");
+    auto* d_op = static_cast<double2*>(pool_alloc(sizeof(double2) * d * d, st));
     check_cuda(cudaMemcpyAsync(d_op, op_host, sizeof(double2) * d * d, cudaMemcpyHostToDevice, st), "copy op");
     const int blocks = (int)std::min<long long>((n + 255) / 256, 4096);
     k_apply_local<<<dim3(blocks, batch), 256, 0, st>>>(static_cast<const double2*>(in_dev),
                                                        static_cast<double2*>(out_dev), n, ld, stride, d, d_op);
     check_launch("k_apply_local");
-    check_cuda(cudaFreeAsync(d_op, st), "cudaFreeAsync(op)");
+    pool_free(d_op, st);
   });
 }

@@ -5,10 +5,12 @@
 // split), re-designed as host-built CSR + offset tables consumed by the
 // sm_100a H psi kernels in hpsi.cu.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <numeric>
 #include <set>
 
@@ -45,6 +47,50 @@ void* system_scratch(rpm_system* sys, int slot, size_t bytes) {
   check_cuda(cudaMemset(sys->scratch[slot], 0, grown), "cudaMemset(scratch)");
   sys->scratch_bytes[slot] = grown;
   return sys->scratch[slot];
+}
+
+// The library's memory pools, one per device, and the number of live systems.
+static std::mutex g_pool_mutex;
+static std::vector<std::pair<int, cudaMemPool_t>> g_pools;
+static std::atomic<long long> g_live_systems{0};
+
+void* pool_alloc(size_t bytes, cudaStream_t stream) {
+  int dev = 0;
+  check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+  cudaMemPool_t pool = nullptr;
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    for (const auto& p : g_pools)
+      if (p.first == dev) pool = p.second;
+    if (!pool) {
+      cudaMemPoolProps props{};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      check_cuda(cudaMemPoolCreate(&pool, &props), "cudaMemPoolCreate");
+      unsigned long long keep = kPoolKeep;
+      check_cuda(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
+      g_pools.emplace_back(dev, pool);
+    }
+  }
+  void* p = nullptr;
+  const cudaError_t err = cudaMallocFromPoolAsync(&p, std::max<size_t>(bytes, 16), pool, stream);
+  if (err == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    fail(RPM_E_NOMEM, "device allocation failed");
+  }
+  check_cuda(err, "cudaMallocFromPoolAsync");
+  return p;
+}
+
+void pool_free(void* p, cudaStream_t stream) { check_cuda(cudaFreeAsync(p, stream), "cudaFreeAsync(pool)"); }
+
+// Gives the pools' idle memory back when the last system has gone.
+static void system_gone() {
+  if (--g_live_systems > 0) return;
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  for (const auto& p : g_pools) cudaMemPoolTrimTo(p.second, 0);
+  cudaGetLastError();
 }
 
 // Row-major tensor strides.
@@ -556,6 +602,7 @@ int rpm_system_create(const int* dims, int ndims, const rpm_term* terms, int nte
     *out = nullptr;
     *out = rpm::create_system(dims, ndims, terms, nterms, left_axes, nleft, right_axes, nright, hermitian_tolerance,
                               host_only);
+    ++rpm::g_live_systems;
   });
 }
 
@@ -564,6 +611,7 @@ int rpm_system_destroy(rpm_system* sys) {
     if (!sys) return;
     rpm::free_system(sys);
     delete sys;
+    rpm::system_gone();
   });
 }
 
