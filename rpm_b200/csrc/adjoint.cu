@@ -41,10 +41,12 @@
 // point; with the complex128 basis it gives FP64-accurate checkpoints and
 // populations on a fixed schedule (smooth in the parameters).
 #include "hpsi.cuh"
+#include "hpsi_direct.cuh"
 
 #include <algorithm>
 #include <cmath>
 #include <complex>
+#include <type_traits>
 #include <vector>
 
 namespace rpm {
@@ -54,6 +56,16 @@ constexpr int kAdjMaxNodes = 4;
 constexpr int kAdjThreads = 256;
 constexpr int kAdjBlocksPerVector = 32;
 constexpr int kAdjWarps = kAdjThreads / 32;
+constexpr int kAdjSums = 36;  // 4 x 4 densities (complex), Taylor norms, energy
+
+// Blocks per vector of the kernels that read the whole Taylor basis: about six
+// per SM over the batch, no more than there are elements for (32 per vector
+// left 4 vectors of 221,184 at 218 and 232 us per interval, of which 80 and 35
+// at the HBM rate).
+int adj_blocks(long long n, int B) {
+  const long long want = std::max<long long>(kAdjBlocksPerVector, 6LL * sm_count() / B);
+  return (int)std::max<long long>(1, std::min(want, (n + kAdjThreads - 1) / kAdjThreads));
+}
 
 template <class T>
 struct AdjCoef {
@@ -115,11 +127,12 @@ __global__ void k_adj_source(const double2* __restrict__ xp, double2* __restrict
 
 // One backward interval (see the file comment).  U: degree + 1 slots of 2B
 // vectors (lambda part first); slot 0 is rewritten with the new [lambda_k; psi_k].
+// energy (complex128 basis, or null): <lambda| u_1> = dt <lambda| H psi> is added.
 template <class T, int Q>
 __global__ void __launch_bounds__(kAdjThreads) k_adj_combine(
     T* U, double2* __restrict__ xl, double2* __restrict__ xp, T* __restrict__ nodes_p, T* __restrict__ nodes_l,
-    double* __restrict__ density, int dens_stride, double* __restrict__ tail, const AdjCoef<T> cf, int degree, int B,
-    long long ld, long long n4, double src_weight) {
+    double* __restrict__ density, int dens_stride, double* __restrict__ tail, double* __restrict__ energy, int e_stride,
+    const AdjCoef<T> cf, int degree, int B, long long ld, long long n4, double src_weight) {
   using R = typename Real<T>::type;
   const int b = blockIdx.y;
   const int lane = threadIdx.x & 31, e = threadIdx.x & 3, base = lane & ~3;
@@ -129,7 +142,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_combine(
   double m[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) m[k] = 0.0;
-  double tl[2] = {0.0, 0.0};
+  double tl[4] = {0.0, 0.0, 0.0, 0.0};  // |last term|^2, |psi|^2, <lambda| u_1> (energy)
   const long long per_round = (long long)gridDim.x * blockDim.x / 4;
   const long long first = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   const long long rounds = (n4 + per_round - 1) / per_round;
@@ -143,6 +156,8 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_combine(
       lq[q] = czero<T>();
       pq[q] = czero<T>();
     }
+    T a0 = czero<T>();
+#pragma unroll 4
     for (int j = 0; j <= degree; ++j) {
       const T a = act ? ul0[(long long)j * slot + at] : czero<T>();
       const T c = act ? up0[(long long)j * slot + at] : czero<T>();
@@ -155,7 +170,15 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_combine(
         ls = cfma(cf.start[j], a, ls);
         ps = cfma(cf.start[j], c, ps);
       }
-      if (j == 0) tl[1] += norm2(c);
+      if (j == 0) {
+        tl[1] += norm2(c);
+        a0 = a;
+      }
+      if (j == 1 && energy) {
+        const T t = cconj_mul(a0, c);
+        tl[2] += (double)t.x;
+        tl[3] += (double)t.y;
+      }
       if (j == degree) tl[0] += norm2(c);
     }
     // row e of M: conj(lambda_q[e]) psi_q[c] for c = 0..3 (psi_q[c] from lane base + c)
@@ -204,26 +227,26 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_combine(
 #pragma unroll
   for (int k = 0; k < 8; ++k)
     for (int o = 4; o < 32; o <<= 1) m[k] += __shfl_xor_sync(0xffffffffu, m[k], o);
-  for (int o = 1; o < 32; o <<= 1) {
-    tl[0] += __shfl_xor_sync(0xffffffffu, tl[0], o);
-    tl[1] += __shfl_xor_sync(0xffffffffu, tl[1], o);
-  }
-  __shared__ double part[kAdjWarps][34];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    for (int o = 1; o < 32; o <<= 1) tl[k] += __shfl_xor_sync(0xffffffffu, tl[k], o);
+  __shared__ double part[kAdjWarps][kAdjSums];
   const int warp = threadIdx.x >> 5;
   if (lane < 4) {
 #pragma unroll
     for (int k = 0; k < 8; ++k) part[warp][lane * 8 + k] = m[k];
   }
   if (lane == 0) {
-    part[warp][32] = tl[0];
-    part[warp][33] = tl[1];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) part[warp][32 + k] = tl[k];
   }
   __syncthreads();
-  if (threadIdx.x < 34) {
+  if (threadIdx.x < kAdjSums) {
     double s = 0.0;
     for (int w = 0; w < kAdjWarps; ++w) s += part[w][threadIdx.x];
     if (threadIdx.x < 32) atomicAdd(density + (long long)b * dens_stride + threadIdx.x, s);
-    else atomicAdd(tail + 2 * b + (threadIdx.x - 32), s);
+    else if (threadIdx.x < 34) atomicAdd(tail + 2 * b + (threadIdx.x - 32), s);
+    else if (energy) atomicAdd(energy + (long long)b * e_stride + (threadIdx.x - 34), s);
   }
 }
 
@@ -247,6 +270,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_forward(T* U, double2* __re
     const bool act = i < n4;
     const long long at = (long long)e * n4 + (act ? i : 0);
     T ps = czero<T>();
+#pragma unroll 4
     for (int j = 0; j <= degree; ++j) {
       const T c = act ? up0[(long long)j * slot + at] : czero<T>();
       if (j >= 1) ps = cfma(cf.start[j], c, ps);
@@ -491,11 +515,91 @@ double read_tail(rpm_adjoint* a, size_t need, cudaStream_t st) {
   return worst;
 }
 
+// All Taylor terms of one complex128 vector per block: u_t stays in shared
+// memory from term to term (ping-pong), one launch per interval where the
+// direct H psi took one of about 5 us per term for a state of this size.
+constexpr int kTaylorThreads = 384;
+constexpr size_t kTaylorSmem = 200 * 1024;
+
+__global__ void __launch_bounds__(kTaylorThreads) k_adj_taylor(const CubeView<double2>* __restrict__ view,
+                                                              double2* __restrict__ U, int groups, long long ld,
+                                                              long long slot, const double* __restrict__ scales,
+                                                              int degree) {
+  using namespace direct;
+  __shared__ Tables tb;
+  extern __shared__ __align__(16) double2 tsm[];
+  const int hr = view->half_r, hl = view->half_l;
+  double2* tab = tsm;
+  HRec* lrec = reinterpret_cast<HRec*>(tab + view->L.ntab + view->R.ntab);
+  HRec* rrec = lrec + hl;
+  double2* cur = reinterpret_cast<double2*>(rrec + hr);
+  double2* nxt = cur + 4 * groups;
+  load_tables(view, tb, tab);
+  constexpr int W = sizeof(HRec) / sizeof(double2);
+  for (int k = threadIdx.x; k < hl * W; k += blockDim.x)
+    reinterpret_cast<double2*>(lrec)[k] = static_cast<const double2*>(view->lrec)[k];
+  for (int k = threadIdx.x; k < hr * W; k += blockDim.x)
+    reinterpret_cast<double2*>(rrec)[k] = static_cast<const double2*>(view->rrec)[k];
+  double2* u = U + (long long)blockIdx.x * ld;
+  for (int k = threadIdx.x; k < 4 * groups; k += blockDim.x) cur[k] = u[k];
+  __syncthreads();
+  for (int t = 0; t < degree; ++t) {
+    const double s = scales[t];
+    double2* out = u + (long long)(t + 1) * slot;
+    for (int g = threadIdx.x; g < groups; g += blockDim.x) {
+      const int l = g / hr, r = g - l * hr;
+      const double2* v = cur + g;
+      double2 x[4], o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[e] = v[e * groups];
+      apply_group(
+          tb, tab, lrec[l], rrec[r], x,
+          [&](int delta, double2(&y)[4]) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) y[e] = v[e * groups + delta];
+          },
+          o);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const double2 w = make_double2(s * o[e].x, s * o[e].y);
+        nxt[e * groups + g] = w;
+        out[e * (long long)groups + g] = w;
+      }
+    }
+    __syncthreads();
+    double2* swap = cur;
+    cur = nxt;
+    nxt = swap;
+  }
+}
+
+// Whether a system's Taylor terms run in one launch: the direct H psi covers it
+// and two copies of a vector fit in shared memory (up to about 6,000 components).
+size_t taylor_smem(const rpm_system* h) {
+  return sizeof(double2) * (size_t)(h->cube_l.ntab + h->cube_r.ntab + 2 * h->n) +
+         sizeof(direct::HRec) * (size_t)(h->half_l + h->half_r);
+}
+
+bool taylor_one_launch(rpm_adjoint* a, rpm_system* h, int count, cudaStream_t st) {
+  if (!direct_usable(h) || h->non_hermitian || h->cube64.inner_l < 1 || h->cube64.inner_r < 1 ||
+      taylor_smem(h) > kTaylorSmem)
+    return false;
+  const int groups = (int)(h->n / 4);
+  check_cuda(cudaFuncSetAttribute(k_adj_taylor, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTaylorSmem),
+             "adjoint Taylor smem attr");
+  const int threads = std::min(kTaylorThreads, (groups + 31) / 32 * 32);
+  k_adj_taylor<<<count, threads, taylor_smem(h), st>>>(h->cube64_dev, static_cast<double2*>(a->U), groups, a->ld,
+                                                       2LL * a->B * a->ld, a->scales, a->degree);
+  check_launch("k_adj_taylor");
+  return true;
+}
+
 // Taylor basis u_{t+1} = H (u_t * dt / (t + 1)) of `count` vectors per slot.
 template <class T>
 void taylor_basis(rpm_adjoint* a, rpm_system* h, int count, cudaStream_t st) {
   T* U = static_cast<T*>(a->U);
   const long long slot = 2LL * a->B * a->ld;
+  if (std::is_same<T, double2>::value && taylor_one_launch(a, h, count, st)) return;
   for (int t = 0; t < a->degree; ++t)
     launch_hpsi_scaled<T>(h, U + t * slot, U + (t + 1) * slot, count, a->ld, a->scales + t, st);
 }
@@ -518,12 +622,15 @@ void sweep_impl(rpm_adjoint* a, rpm_system* const* systems, int nseg, rpm_system
   for (int k = 0; k < nseg * nder; ++k) any_der = any_der || dsys[k] != nullptr;
   T* np = any_der ? static_cast<T*>(a->node_p) : nullptr;
   T* nl = any_der ? static_cast<T*>(a->node_l) : nullptr;
-  const dim3 grid(kAdjBlocksPerVector, B);
+  const dim3 grid(adj_blocks(a->n, B), B);
+  constexpr bool kWide = std::is_same<T, double2>::value;
   for (int j = nint - 1; j >= 0; --j) {
     const int s = seg_of[j];
     rpm_system* h = systems[s];
-    if (energy) {
-      // <lambda(tau)| H |psi(tau)> is constant over the interval: FP64 once
+    // <lambda(tau)| H |psi(tau)> is constant over the interval: FP64 once (the
+    // complex128 basis holds dt H psi already, and the combine sums it)
+    double* wide_energy = kWide && energy ? energy + 2 * s : nullptr;
+    if (energy && !kWide) {
       launch_hpsi<double2>(h, xp, a->hpsi64, B, a->ld, st);
       k_adj_energy<<<dim3(kAdjBlocksPerVector * 4, B), kAdjThreads, 0, st>>>(xl, a->hpsi64, B, a->n, a->ld, dt,
                                                                              energy + 2 * s, 2 * nseg);
@@ -535,20 +642,20 @@ void sweep_impl(rpm_adjoint* a, rpm_system* const* systems, int nseg, rpm_system
     const long long n4 = a->n / 4;
     switch (a->nodes) {
       case 1:
-        k_adj_combine<T, 1><<<grid, kAdjThreads, 0, st>>>(U, xl, xp, np, nl, dens, 32 * nseg, tail, cf, a->degree, B,
-                                                          a->ld, n4, weights[j]);
+        k_adj_combine<T, 1><<<grid, kAdjThreads, 0, st>>>(U, xl, xp, np, nl, dens, 32 * nseg, tail, wide_energy,
+                                                          2 * nseg, cf, a->degree, B, a->ld, n4, weights[j]);
         break;
       case 2:
-        k_adj_combine<T, 2><<<grid, kAdjThreads, 0, st>>>(U, xl, xp, np, nl, dens, 32 * nseg, tail, cf, a->degree, B,
-                                                          a->ld, n4, weights[j]);
+        k_adj_combine<T, 2><<<grid, kAdjThreads, 0, st>>>(U, xl, xp, np, nl, dens, 32 * nseg, tail, wide_energy,
+                                                          2 * nseg, cf, a->degree, B, a->ld, n4, weights[j]);
         break;
       case 3:
-        k_adj_combine<T, 3><<<grid, kAdjThreads, 0, st>>>(U, xl, xp, np, nl, dens, 32 * nseg, tail, cf, a->degree, B,
-                                                          a->ld, n4, weights[j]);
+        k_adj_combine<T, 3><<<grid, kAdjThreads, 0, st>>>(U, xl, xp, np, nl, dens, 32 * nseg, tail, wide_energy,
+                                                          2 * nseg, cf, a->degree, B, a->ld, n4, weights[j]);
         break;
       default:
-        k_adj_combine<T, 4><<<grid, kAdjThreads, 0, st>>>(U, xl, xp, np, nl, dens, 32 * nseg, tail, cf, a->degree, B,
-                                                          a->ld, n4, weights[j]);
+        k_adj_combine<T, 4><<<grid, kAdjThreads, 0, st>>>(U, xl, xp, np, nl, dens, 32 * nseg, tail, wide_energy,
+                                                          2 * nseg, cf, a->degree, B, a->ld, n4, weights[j]);
         break;
     }
     check_launch("adjoint combine");
@@ -581,7 +688,7 @@ void forward_impl(rpm_adjoint* a, rpm_system* const* systems, const int* seg_of,
   const AdjCoef<T> cf = make_coef<T>(a->degree, 1, dt, -1);
   for (int j = 0; j < nint; ++j) {
     taylor_basis<T>(a, systems[seg_of[j]], B, st);
-    k_adj_forward<T><<<dim3(kAdjBlocksPerVector, B), kAdjThreads, 0, st>>>(
+    k_adj_forward<T><<<dim3(adj_blocks(a->n, B), B), kAdjThreads, 0, st>>>(
         U, xp, pops + j, pop_ld, a->tail + (size_t)j * 2 * B, cf, a->degree, B, a->ld, a->n / 4);
     check_launch("adjoint forward step");
   }

@@ -190,6 +190,9 @@ struct CubeView {
   // radical the records of the direct H psi (hpsi_direct.cuh); else null
   const void* lrec;
   const void* rrec;
+  // complex128: bit k set when nucleus k of the radical has any transition to
+  // another level (its block of the table is not diagonal in the nucleus)
+  unsigned moves_l, moves_r;
 };
 
 }  // namespace rpm

@@ -4,9 +4,13 @@
 namespace rpm {
 namespace {
 
+// Bound by the load / store pipe (61 % of its wavefronts at 28 % occupancy, FP64
+// pipe 32 %, DRAM 6 %: ncu, 8 vectors of 221,184).  Six blocks of 128 threads
+// per SM (80 registers): 181 us for 32 vectors, against 187 us at 92
+// registers and 202 us at 64, which spills.
 constexpr int kDirectThreads = 128;
 
-__global__ void __launch_bounds__(kDirectThreads) k_hpsi_direct(const CubeView<double2>* __restrict__ view,
+__global__ void __launch_bounds__(kDirectThreads, 6) k_hpsi_direct(const CubeView<double2>* __restrict__ view,
                                                                const double2* __restrict__ in,
                                                                double2* __restrict__ out, int groups, long long ld,
                                                                const double* __restrict__ scale) {

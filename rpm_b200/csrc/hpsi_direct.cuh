@@ -28,9 +28,11 @@ constexpr int kMaxPartners = 64;   // sum of (dimension - 1) over a radical's nu
 constexpr int kMaxDigit = 16;      // largest nuclear dimension (four bits)
 constexpr int kMaxTables = 1024;   // coefficients of both radicals staged in shared memory
 
-// Partner t = 1 .. d - 1 of one nucleus: its value is (m + t) mod d.
-struct Partner {
-  int shift, t, d, stride, offx;
+// Partner t = 1 .. d - 1 of one nucleus: its value is (m + t) mod d.  One
+// 16-byte shared-memory read: the load / store pipe is what bounds the kernel.
+struct __align__(16) Partner {
+  unsigned char shift, t, d, pad;
+  int stride, offx, pad2;
 };
 
 struct Tables {
@@ -49,12 +51,16 @@ __device__ __forceinline__ void load_tables(const CubeView<double2>* view, Table
   for (int k = threadIdx.x; k < 2 * kCubeMaxDigits; k += blockDim.x) {
     const int side = k / kCubeMaxDigits, q = k % kCubeMaxDigits;
     const CubeSide& s = side ? view->R : view->L;
+    // nuclei without transitions (a quadrupole system's spin-1/2 ones) have no partners
+    const unsigned moves = side ? view->moves_r : view->moves_l;
     if (q < s.K) {
       int at = 0;
-      for (int p = 0; p < q; ++p) at += s.dim[p] - 1;
-      const int d = s.dim[q];
+      for (int p = 0; p < q; ++p) at += (moves >> p) & 1u ? s.dim[p] - 1 : 0;
+      const int d = (moves >> q) & 1u ? s.dim[q] : 1;
       for (int t = 1; t < d; ++t)
-        tb.part[side][at + t - 1] = Partner{4 * q, t, d, s.gs[q] * (side ? 1 : view->half_r), s.offX[q] + (side ? nl : 0)};
+        tb.part[side][at + t - 1] =
+            Partner{(unsigned char)(4 * q), (unsigned char)t, (unsigned char)d, 0,
+                    s.gs[q] * (side ? 1 : view->half_r), s.offX[q] + (side ? nl : 0), 0};
       if (q == s.K - 1) tb.np[side] = at + d - 1;
     }
   }
@@ -93,7 +99,9 @@ __device__ __forceinline__ void apply_group(const Tables& tb, const double2* tab
     // partner p + 1 is on its way while partner p is applied
     double2 y[4];
     auto fetch = [&](int p, double2 (&v)[4], const double2*& cf, int& d) {
-      const Partner q = tb.part[side][p];
+      const int4 raw = *reinterpret_cast<const int4*>(&tb.part[side][p]);
+      Partner q;
+      memcpy(&q, &raw, sizeof(q));
       const int m = (int)(digits >> q.shift) & 15;
       int mp = m + q.t;
       if (mp >= q.d) mp -= q.d;

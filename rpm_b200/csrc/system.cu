@@ -307,6 +307,20 @@ static std::vector<direct::HRec> direct_records(const CubeSide& side, const std:
   return out;
 }
 
+// Bit k: nucleus k has a nonzero entry between two of its levels.
+static unsigned moving_digits(const CubeSide& side, const std::vector<double2>& tab) {
+  unsigned out = 0;
+  for (int k = 0; k < side.K; ++k) {
+    const int d = side.dim[k];
+    for (int row = 0; row < 2 * d; ++row)
+      for (int col = 0; col < 2 * d; ++col) {
+        const double2 x = tab[side.offX[k] + row * 2 * d + col];
+        if (row % d != col % d && (x.x != 0.0 || x.y != 0.0)) out |= 1u << k;
+      }
+  }
+  return out;
+}
+
 // Standard layout psi[eA][eB][l][r] within the direct H psi's limits.
 static bool direct_layout(const rpm_system* sys) {
   int partners[2] = {0, 0}, side = 0;
@@ -411,6 +425,9 @@ static void upload_system(rpm_system* sys) {
         c32.orec_bytes_l = (int)(rl.size() * sizeof(float));  // records (padded to 16 bytes) + 128 pair bytes
       }
       c64.lrec = c64.rrec = c32.lrec = c32.rrec = nullptr;
+      c32.moves_l = c32.moves_r = 0;
+      c64.moves_l = moving_digits(cl, tl64);
+      c64.moves_r = moving_digits(cr, tr64);
       if (direct_layout(sys)) {
         const auto lr = direct_records(cl, tl64), rr = direct_records(cr, tr64);
         c64.lrec = upload<direct::HRec>(sys, lr.data(), lr.size() * sizeof(direct::HRec));
