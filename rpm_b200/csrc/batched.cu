@@ -29,6 +29,7 @@
 
 #include "common.cuh"
 #include "hpsi.cuh"
+#include "hpsi_cube.cuh"
 #include "krylov.cuh"
 
 namespace rpm {
@@ -1251,6 +1252,7 @@ __global__ void __launch_bounds__(256) k_b_observe(BatchDev B) {
 }  // namespace rpm
 
 #include "gram_tc.cuh"
+#include "lanczos_small.cuh"
 
 struct rpm_batch {
   std::vector<rpm_system*> systems;
@@ -1498,6 +1500,16 @@ static void record_step(rpm_batch* Bh, const BatchDev& B, const Layout& L, cudaS
     npers = 0;
   }
   const bool all_pers = npers == (int)Bh->groups.size();
+  // groups of small states on the general cube kernels: one block per
+  // trajectory for the whole step (not between reorthogonalisations)
+  std::vector<small::Shape> gshape(Bh->groups.size());
+  std::vector<char> gsmall(Bh->groups.size(), 0);
+  int nsmall = 0;
+  for (size_t g = 0; g < Bh->groups.size(); ++g) {
+    gsmall[g] = reo == 0 && !gfused[g] && small::shape_of(Bh->groups[g].plan, Bh->groups[g].nb, gshape[g]);
+    nsmall += gsmall[g];
+  }
+  const bool whole_step = npers + nsmall == (int)Bh->groups.size();  // no launch per iteration is left
   auto reorth_after = [&](int j) { return reo > 0 && (j + 1) % reo == 0 && j + 1 < m; };
   auto reorthogonalise = [&](int j) {
     for (int pass = 1; pass <= 2; ++pass) {
@@ -1507,7 +1519,11 @@ static void record_step(rpm_batch* Bh, const BatchDev& B, const Layout& L, cudaS
     check_launch("batched reorthogonalisation");
   };
   const int nseg = reo > 0 ? (m + reo - 1) / reo : 1;  // segments of the persistent launches
-  if (all_pers) check_cuda(cudaEventRecordWithFlags(Bh->probe0, st, probe_flags), "probe record");
+  if (whole_step) check_cuda(cudaEventRecordWithFlags(Bh->probe0, st, probe_flags), "probe record");
+  for (size_t g = 0; g < Bh->groups.size(); ++g)
+    if (gsmall[g])
+      small::launch(B, Bh->views_dev, reinterpret_cast<const int*>(base + L.sysof), Bh->groups[g].b0,
+                    Bh->groups[g].nb, Bh->groups[g].plan, gshape[g], st);
   for (int seg = 0; seg < nseg && npers > 0; ++seg) {
     const int j0 = reo > 0 ? seg * reo : 0;
     const int j1 = reo > 0 ? std::min(m, (seg + 1) * reo) : m;
@@ -1564,13 +1580,13 @@ static void record_step(rpm_batch* Bh, const BatchDev& B, const Layout& L, cudaS
     }
     if (all_pers && reorth_after(j1 - 1)) reorthogonalise(j1 - 1);
   }
-  if (all_pers) {
+  if (whole_step) {
     check_cuda(cudaEventRecordWithFlags(Bh->probe1, st, probe_flags), "probe record");
     Bh->probe_iters = m;
   } else {
     Bh->probe_iters = 1;
   }
-  for (int j = 0; j < m && !all_pers; ++j) {
+  for (int j = 0; j < m && !whole_step; ++j) {
     a.in = B.V + (size_t)j * B.ld;
     a.out = B.V + (size_t)(j + 1) * B.ld;
     // While capturing, external records become event-record nodes of the graph.
@@ -1595,7 +1611,7 @@ static void record_step(rpm_batch* Bh, const BatchDev& B, const Layout& L, cudaS
     z.istride = kStateInts;
     z.breakdown_rel = B.breakdown_rel;
     for (size_t g = 0; g < Bh->groups.size(); ++g) {
-      if (gpers[g]) continue;
+      if (gpers[g] || gsmall[g]) continue;
       const auto& G = Bh->groups[g];
       HpsiArgs<float2> ak = group_args(a, G.b0, D);
       float2* yk = ya + (size_t)G.b0 * B.ld;
@@ -1617,9 +1633,9 @@ static void record_step(rpm_batch* Bh, const BatchDev& B, const Layout& L, cudaS
   Bh->persistent = all_pers;
   int per_iter_rest = 0;
   for (size_t g = 0; g < Bh->groups.size(); ++g)
-    if (!gpers[g]) per_iter_rest += gfused[g] ? 2 : 3;
+    if (!gpers[g] && !gsmall[g]) per_iter_rest += gfused[g] ? 2 : 3;
   const int nreo = reo > 0 ? (m - 1) / reo : 0;  // iterations j = P-1, 2P-1, ... <= m-2
-  Bh->launches_per_step = 1 + npers * nseg + per_iter_rest * m + 4 * nreo + 4;
+  Bh->launches_per_step = 1 + nsmall + npers * nseg + per_iter_rest * m + 4 * nreo + 4;
   const size_t ctl_smem = sizeof(double) * 2 * kRecDoubles;
   check_cuda(cudaEventRecord(Bh->ev_fork, st), "fork record");
   check_cuda(cudaStreamWaitEvent(Bh->side, Bh->ev_fork, 0), "fork wait");
@@ -1771,6 +1787,7 @@ static void run_batch(rpm_batch* Bh, int ntraj, const int* sys_of, void* psi, co
   check_cuda(cudaFuncSetAttribute(k_b_observe, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(sizeof(double2) * kBMaxK * kBMaxK)),
              "observe attr");
+  for (const auto& G : Bh->groups) small::prepare(G.plan);
 
   const bool use_graph = cfg.use_graph != 0;
   if (use_graph) {

@@ -31,6 +31,7 @@
 
 #include "common.cuh"
 #include "hpsi.cuh"
+#include "hpsi_cube.cuh"
 #include "hpsi_direct.cuh"
 
 namespace rpm {
@@ -119,209 +120,6 @@ __device__ void finish_dot(const HpsiArgs<T>& a, int b, double mine) {
     for (int k = 0; k < (int)gridDim.x; ++k) s += __ldcg(a.dot_part + (long long)b * gridDim.x + k);
     a.dot_out[(long long)b * a.dot_stride] = s;
     a.dot_count[b] = 0;
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Cube form
-// ---------------------------------------------------------------------------
-// Complex multiply-accumulate of the cube kernels: four FMAs per complex
-// product in the state precision (FP32 for complex64, FP64 for complex128).
-template <class T> struct CubeArith;
-
-template <>
-struct CubeArith<double2> {
-  using Coef = double2;
-  using R = double;
-  __device__ static double2 prep(double2 x) { return x; }
-  __device__ static double2 mac(const double2& c, double2 x, double2, double2 acc) { return cfma(c, x, acc); }
-  __device__ static double2 rmac(double d, double2 x, double2 acc) {
-    acc.x = fma(d, x.x, acc.x);
-    acc.y = fma(d, x.y, acc.y);
-    return acc;
-  }
-  __device__ static double2 add(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-  __device__ static double2 from_complex(double2 v) { return v; }
-  __device__ static double re(const double2& c) { return c.x; }
-};
-
-template <>
-struct CubeArith<float2> {
-  using Coef = float2;
-  using R = float;
-  __device__ static float2 prep(float2 x) { return x; }
-  __device__ static float2 mac(const float2& c, float2 x, float2, float2 acc) { return cfma(c, x, acc); }
-  __device__ static float2 rmac(float d, float2 x, float2 acc) {
-    acc.x = fmaf(d, x.x, acc.x);
-    acc.y = fmaf(d, x.y, acc.y);
-    return acc;
-  }
-  __device__ static float2 add(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-  __device__ static float2 from_complex(float2 v) { return v; }
-  __device__ static float re(const float2& c) { return c.x; }
-};
-
-// Per outer index o (all group digits except the NI inner ones), built once
-// per CTA in shared memory: the outer digits packed 4 bits each and the
-// diagonal / electron-flip coefficients merged over Z and the outer digits.
-// Group index g = e * half + C * o + i  (C = 2^NI, i = inner digits).
-template <class T>
-struct OuterRec {
-  typename CubeArith<T>::Coef f[2];
-  typename CubeArith<T>::R d[2];
-  unsigned lo, hi;
-};
-
-__device__ __forceinline__ int align16(int bytes) { return (bytes + 15) & ~15; }
-
-// Asynchronous global -> shared copy of one complex element (cp.async).
-template <class T>
-__device__ __forceinline__ void async_copy(T* smem_dst, const T* gmem_src) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
-  if constexpr (sizeof(T) == 16) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem_src) : "memory");
-  } else {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem_src) : "memory");
-  }
-}
-__device__ __forceinline__ void async_wait_all() {
-  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-}
-
-// Copy one group's CubeSide and its coefficient table into shared memory.
-template <class Coef>
-__device__ __forceinline__ void load_side(const CubeSide& src, const Coef* tab_src, CubeSide& side, Coef* tab) {
-  const int* s = reinterpret_cast<const int*>(&src);
-  int* d = reinterpret_cast<int*>(&side);
-  for (int k = threadIdx.x; k < (int)(sizeof(CubeSide) / sizeof(int)); k += blockDim.x) d[k] = s[k];
-  __syncthreads();
-  for (int k = threadIdx.x; k < side.ntab; k += blockDim.x) tab[k] = tab_src[k];
-}
-
-template <class T, int NI>
-__device__ __forceinline__ void build_outer(const CubeSide& side, const typename CubeArith<T>::Coef* tab,
-                                            OuterRec<T>* otab, int n_outer) {
-  using A = CubeArith<T>;
-  const int nout = side.K - NI;
-  for (int o = threadIdx.x; o < n_outer; o += blockDim.x) {
-    OuterRec<T> rec;
-    rec.d[0] = A::re(tab[0]);
-    rec.d[1] = A::re(tab[1]);
-    rec.f[0] = tab[2];
-    rec.f[1] = tab[3];
-    int rem = o;
-    unsigned lo = 0, hi = 0;
-    for (int k = nout - 1; k >= 0; --k) {
-      const int d = side.dim[k];
-      const int m = rem % d;
-      rem /= d;
-      if (k < 8) lo |= (unsigned)m << (4 * k);
-      else hi |= (unsigned)m << (4 * (k - 8));
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        rec.d[e] += A::re(tab[side.offD[k] + e * d + m]);
-        rec.f[e] = A::add(rec.f[e], tab[side.offF[k] + e * d + m]);
-      }
-    }
-    rec.lo = lo;
-    rec.hi = hi;
-    otab[o] = rec;
-  }
-}
-
-// Diagonal and electron-flip coefficients contributed by the inner digits:
-// the same for every cube of a CTA, so computed once per thread.
-template <class T, int NI>
-struct InnerConst {
-  typename CubeArith<T>::R d[2][1 << NI];
-  typename CubeArith<T>::Coef f[2][1 << NI];
-  __device__ InnerConst(const CubeSide& side, const typename CubeArith<T>::Coef* tab) {
-    using A = CubeArith<T>;
-#pragma unroll
-    for (int e = 0; e < 2; ++e)
-#pragma unroll
-      for (int i = 0; i < (1 << NI); ++i) {
-        // first inner digit, then the others
-        typename A::Coef fl = tab[side.offF[side.K - NI] + e * 2 + ((i >> (NI - 1)) & 1)];
-        typename A::R dg = A::re(tab[side.offD[side.K - NI] + e * 2 + ((i >> (NI - 1)) & 1)]);
-#pragma unroll
-        for (int q = 1; q < NI; ++q) {
-          const int k = side.K - NI + q;
-          const int bit = (i >> (NI - 1 - q)) & 1;
-          dg += A::re(tab[side.offD[k] + e * 2 + bit]);
-          fl = A::add(fl, tab[side.offF[k] + e * 2 + bit]);
-        }
-        d[e][i] = dg;
-        f[e][i] = fl;
-      }
-  }
-};
-
-// Register-cube update shared by both passes.  `at(e, i, delta)` returns the
-// element (electron e, inner i) of the cube whose outer index is shifted by
-// `delta` (delta = 0: the thread's own cube).
-template <class T, int NI, class At>
-__device__ __forceinline__ void cube_apply(const CubeSide& side, const typename CubeArith<T>::Coef* tab,
-                                           const InnerConst<T, NI>& ic, const OuterRec<T>& rec,
-                                           const typename CubeArith<T>::R (&dout)[2],
-                                           const typename CubeArith<T>::Coef (&fout)[2], const T (&x)[2][1 << NI],
-                                           T (&acc)[2][1 << NI], At at) {
-  using A = CubeArith<T>;
-  constexpr int C = 1 << NI;
-  const int K = side.K;
-  T xs[2][C];
-#pragma unroll
-  for (int e = 0; e < 2; ++e)
-#pragma unroll
-    for (int i = 0; i < C; ++i) xs[e][i] = A::prep(x[e][i]);
-#pragma unroll
-  for (int e = 0; e < 2; ++e)
-#pragma unroll
-    for (int i = 0; i < C; ++i) {
-      acc[e][i] = A::rmac(dout[e] + ic.d[e][i], x[e][i], acc[e][i]);
-      acc[e][i] = A::mac(A::add(fout[e], ic.f[e][i]), x[1 - e][i], xs[1 - e][i], acc[e][i]);
-    }
-#pragma unroll
-  for (int q = 0; q < NI; ++q) {
-    const typename A::Coef* X = tab + side.offX[K - NI + q];
-#pragma unroll
-    for (int i = 0; i < C; ++i) {
-      const int bit = (i >> (NI - 1 - q)) & 1;
-      const int ip = i ^ (1 << (NI - 1 - q));
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        acc[e][i] = A::mac(X[(e * 2 + bit) * 4 + (1 - bit)], x[0][ip], xs[0][ip], acc[e][i]);
-        acc[e][i] = A::mac(X[(e * 2 + bit) * 4 + 2 + (1 - bit)], x[1][ip], xs[1][ip], acc[e][i]);
-      }
-    }
-  }
-  const int nout = K - NI;
-  for (int k = 0; k < nout; ++k) {
-    const int d = side.dim[k];
-    const int m = (int)(((k < 8) ? (rec.lo >> (4 * k)) : (rec.hi >> (4 * (k - 8)))) & 15u);
-    const int ostride = side.gs[k] >> NI;
-    const typename A::Coef* X = tab + side.offX[k] + (size_t)m * 2 * d;
-    for (int mp = 0; mp < d; ++mp) {
-      if (mp == m) continue;
-      const int delta = (mp - m) * ostride;
-      T y[2][C];
-#pragma unroll
-      for (int e = 0; e < 2; ++e)
-#pragma unroll
-        for (int i = 0; i < C; ++i) y[e][i] = at(e, i, delta);
-#pragma unroll
-      for (int ep = 0; ep < 2; ++ep) {
-        // coefficients of output electron e from input electron ep
-        const typename A::Coef c0 = X[(0 * d) * 2 * d + ep * d + mp];
-        const typename A::Coef c1 = X[(1 * d) * 2 * d + ep * d + mp];
-#pragma unroll
-        for (int i = 0; i < C; ++i) {
-          const T ys = A::prep(y[ep][i]);
-          acc[0][i] = A::mac(c0, y[ep][i], ys, acc[0][i]);
-          acc[1][i] = A::mac(c1, y[ep][i], ys, acc[1][i]);
-        }
-      }
-    }
   }
 }
 
@@ -743,25 +541,44 @@ static void cube_l_dispatch(const HpsiArgs<T>& a, const CubePlan& p, T* ya, int 
   fail(RPM_E_UNSUPPORTED, "radical group too large for the cube kernel");
 }
 
+// Rows per pass-R tile for a batch: the largest tile (of a power of two of at
+// most 16 rows) that still gives about two CTAs per SM and fits in shared
+// memory, 0 when none fits; an explicit choice (autotuner) comes first.
+template <class T, int NI>
+static int cube_r_rows(const CubePlan& p, int batch, int tuned_tl) {
+  const int n_outer = NI == 1 ? p.n_outer_r1 : p.n_outer_r2;
+  auto fits = [&](int tl) {
+    return (size_t)cube_smem_prefix<T>(p.tab_cap, n_outer, tl, p.nr) + (size_t)2 * tl * p.nr * sizeof(T) <= kMaxSmem;
+  };
+  for (int tl = 16; tl >= 1; tl /= 2)
+    if (tl == tuned_tl && fits(tl)) return tl;
+  const int want = 2 * sm_count();
+  for (int tl = 16; tl >= 4; tl /= 2)
+    if (((p.nl + tl - 1) / tl) * batch >= want && fits(tl)) return tl;
+  return fits(2) ? 2 : fits(1) ? 1 : 0;
+}
+
 template <class T, int NI>
 static void cube_r_dispatch(const HpsiArgs<T>& a, const CubePlan& p, const T* ya, int batch, cudaStream_t st,
                             int tuned_tl) {
-  switch (tuned_tl) {
-    case 16: if (try_cube_r<T, NI, 16>(a, p, ya, batch, st)) return; break;
-    case 8: if (try_cube_r<T, NI, 8>(a, p, ya, batch, st)) return; break;
-    case 4: if (try_cube_r<T, NI, 4>(a, p, ya, batch, st)) return; break;
-    case 2: if (try_cube_r<T, NI, 2>(a, p, ya, batch, st)) return; break;
-    case 1: if (try_cube_r<T, NI, 1>(a, p, ya, batch, st)) return; break;
+  bool done = false;
+  switch (cube_r_rows<T, NI>(p, batch, tuned_tl)) {
+    case 16: done = try_cube_r<T, NI, 16>(a, p, ya, batch, st); break;
+    case 8: done = try_cube_r<T, NI, 8>(a, p, ya, batch, st); break;
+    case 4: done = try_cube_r<T, NI, 4>(a, p, ya, batch, st); break;
+    case 2: done = try_cube_r<T, NI, 2>(a, p, ya, batch, st); break;
+    case 1: done = try_cube_r<T, NI, 1>(a, p, ya, batch, st); break;
     default: break;
   }
-  const int want = 2 * sm_count();
-  auto ctas = [&](int tl) { return ((p.nl + tl - 1) / tl) * batch; };
-  if (ctas(16) >= want && try_cube_r<T, NI, 16>(a, p, ya, batch, st)) return;
-  if (ctas(8) >= want && try_cube_r<T, NI, 8>(a, p, ya, batch, st)) return;
-  if (ctas(4) >= want && try_cube_r<T, NI, 4>(a, p, ya, batch, st)) return;
-  if (try_cube_r<T, NI, 2>(a, p, ya, batch, st)) return;
-  if (try_cube_r<T, NI, 1>(a, p, ya, batch, st)) return;
-  fail(RPM_E_UNSUPPORTED, "radical group too large for the cube kernel");
+  if (!done) fail(RPM_E_UNSUPPORTED, "radical group too large for the cube kernel");
+}
+
+// Pass-R tile rows of launch_cube<float2> (complex64) for a batch, and 0 when
+// an explicit cube-kernel variant is set.
+int cube_rows_c64(const CubePlan& p, int batch) {
+  const CubeTuning tu = cube_tuning();
+  if (tu.ni_l || tu.ni_r || tu.tr || tu.tl) return 0;
+  return p.ni_r >= 2 ? cube_r_rows<float2, 2>(p, batch, 0) : cube_r_rows<float2, 1>(p, batch, 0);
 }
 
 template <class T>

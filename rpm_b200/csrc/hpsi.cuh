@@ -136,6 +136,9 @@ template <class T>
 bool launch_cube_fast(const HpsiArgs<T>& a, const CubePlan& p, T* ya, int batch, cudaStream_t stream);
 template <class T>
 bool cube_fast_usable(const HpsiArgs<T>& a, const CubePlan& p, const T* ya);
+// Rows per pass-R tile that launch_cube<float2> takes for a batch (0: an
+// explicit variant is set); the tiles fix the order of its fused sums.
+int cube_rows_c64(const CubePlan& p, int batch);
 // Two passes: pass L into `ya` (batch x ld scratch), pass R into a.out.
 template <class T>
 void launch_cube(const HpsiArgs<T>& a, const CubePlan& p, T* ya, int batch, cudaStream_t stream);
