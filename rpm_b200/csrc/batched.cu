@@ -281,79 +281,87 @@ __global__ void __launch_bounds__(kEwThreads) k_b_update(BatchDev B, int j, int 
 }
 
 // ---------------------------------------------------------------------------
-// Per-trajectory controller (one CTA of four warps per trajectory)
+// Per-trajectory controller (one CTA of 16 warps per trajectory)
 // ---------------------------------------------------------------------------
-// One warp: c = exp(-i T_hi t) e1 (into `c` when non-null) and the embedded
-// error safety * norm * |c_hi(t) - [c_lo(t); 0]| (0 when `exact`), the
-// reference's estimate (rpm_statevector_engine.py:690-715).  ph: 2 * kBMaxK
-// warp-private scratch.  Records: [0] size, [1] status, [2, 2 + kBMaxK)
-// eigenvalues, then the eigenvectors by columns (tridiag_qr_warp_cols, ld kBMaxK).
-__device__ double warp_step_error(const double* rec_hi, const double* rec_lo, bool exact, double t, double safety,
-                                  double norm, double2* ph, double2* c) {
+// One warp: c = exp(-i T t) e1 into `c` from a spectra record ([0] size, [1]
+// status, [2, 2 + kBMaxK) eigenvalues, then the eigenvectors by columns).  ph:
+// warp-private scratch.
+__device__ void warp_exponential(const double* rec, double t, double2* ph, double2* c) {
   const int lane = threadIdx.x & 31;
-  const int mh = (int)rec_hi[0], ml = exact ? 0 : (int)rec_lo[0];
-  const double* lh = rec_hi + 2;
-  const double* zh = rec_hi + 2 + kBMaxK;
-  const double* ll = rec_lo + 2;
-  const double* zl = rec_lo + 2 + kBMaxK;
-  for (int k = lane; k < mh + ml; k += 32) {
-    const bool hi = k < mh;
-    const int kk = hi ? k : k - mh;
+  const int m = (int)rec[0];
+  const double* lam = rec + 2;
+  const double* z = rec + 2 + kBMaxK;
+  for (int k = lane; k < m; k += 32) {
     double sv, cv;
-    sincos((hi ? lh : ll)[kk] * t, &sv, &cv);
-    const double w = (hi ? zh : zl)[kk * kBMaxK];  // first component of eigenvector kk
+    sincos(lam[k] * t, &sv, &cv);
+    const double w = z[k * kBMaxK];  // first component of eigenvector k
     ph[k] = make_double2(cv * w, -sv * w);
   }
   __syncwarp();
-  double acc = 0.0;
-  for (int i = lane; i < mh; i += 32) {
-    double2 ch = make_double2(0.0, 0.0), cl = make_double2(0.0, 0.0);
-    for (int k = 0; k < mh; ++k) {
-      const double zz = zh[k * kBMaxK + i];
-      ch.x = fma(zz, ph[k].x, ch.x);
-      ch.y = fma(zz, ph[k].y, ch.y);
+  for (int i = lane; i < m; i += 32) {
+    double2 acc = make_double2(0.0, 0.0);
+#pragma unroll 8
+    for (int k = 0; k < m; ++k) {
+      const double zz = z[k * kBMaxK + i];
+      acc.x = fma(zz, ph[k].x, acc.x);
+      acc.y = fma(zz, ph[k].y, acc.y);
     }
-    if (c) c[i] = ch;
-    if (i < ml) {
-      for (int k = 0; k < ml; ++k) {
-        const double zz = zl[k * kBMaxK + i];
-        cl.x = fma(zz, ph[mh + k].x, cl.x);
-        cl.y = fma(zz, ph[mh + k].y, cl.y);
-      }
-    }
-    const double dx = ch.x - cl.x, dy = ch.y - cl.y;
-    acc = fma(dx, dx, fma(dy, dy, acc));
+    c[i] = acc;
   }
-  acc = warp_sum(acc);
   __syncwarp();
-  return exact ? 0.0 : safety * norm * sqrt(acc);
 }
 
-// Per trajectory: spectra of T_M and T_{M-offset} (one warp each), the
-// largest step dt <= dt_max with err(dt) <= budget * dt / T (bracket, then
-// 5-way multisection in log dt with four trial steps per round, one per
-// warp, to a relative width of 5e-4), and the coefficient rows of the
-// step's observation points (one point per warp at a time).
-// Dynamic shared memory: two spectra records (hi, lo) of the krylov.cuh layout.
-__global__ void __launch_bounds__(128) k_b_control(BatchDev B) {
+// |c_hi - [c_lo; 0]|^2 over one warp.
+__device__ double warp_difference(const double2* ch, int mh, const double2* cl, int ml) {
+  double acc = 0.0;
+  for (int i = threadIdx.x & 31; i < mh; i += 32) {
+    const double2 lo = i < ml ? cl[i] : make_double2(0.0, 0.0);
+    const double dx = ch[i].x - lo.x, dy = ch[i].y - lo.y;
+    acc = fma(dx, dx, fma(dy, dy, acc));
+  }
+  return warp_sum(acc);
+}
+
+__device__ __forceinline__ void pair_sync(int pair) { asm volatile("bar.sync %0, 64;\n" ::"r"(pair + 1) : "memory"); }
+
+// Per trajectory: spectra of T_M and T_{M-offset} (a chase warp and up to two
+// row warps each), the largest step dt <= dt_max with err(dt) <= budget * dt /
+// T (bracket, then 5-way multisection in log dt with four trial steps per
+// round to a relative width of 5e-4), and the coefficient rows of the step's
+// observation points.  err is the reference's estimate safety * norm *
+// |c_hi(t) - [c_lo(t); 0]| (rpm_statevector_engine.py:690-715); a pair of warps
+// evaluates one time, hi and lo side by side, eight times at once.
+// Latency-bound FP64 chains: with four warps in all, every warp applying its
+// own rotations and evaluating hi and lo one after the other, a step took 233
+// us at M = 30 and 472 us at M = 40.
+// Dynamic shared memory: two spectra records (hi, lo).
+constexpr int kCtlWarps = 16;
+constexpr int kCtlPairs = kCtlWarps / 2;
+
+__global__ void __launch_bounds__(kCtlWarps * 32) k_b_control(BatchDev B) {
   extern __shared__ double sm[];
-  __shared__ double2 ph[4][2 * kBMaxK];
-  __shared__ double2 rot[2][kBMaxK];
+  __shared__ RotRing ring[2];
+  __shared__ double2 ph[kCtlWarps][kBMaxK], cf[kCtlWarps][kBMaxK];
   __shared__ double dd[2][kBMaxK], ee[2][kBMaxK];
   __shared__ double cand[4];
   __shared__ int okf[4];
   __shared__ double s_dt, s_lo, s_hi;
-  __shared__ int s_state, s_np;
+  __shared__ int s_state;
   const int b = blockIdx.x;
   TrajState& s = B.st[b];
   if (s.done) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int pair = warp >> 1;
+  const bool is_hi = (warp & 1) == 0;
   double* rec_hi = sm;
   double* rec_lo = sm + kRecDoubles;
   const int M = s.msize;
   const bool exact = s.stop != 0;
   const int ML = max(1, M - B.offset);
-  if (warp < (exact ? 1 : 2)) {
+  const int solves = exact ? 1 : 2;
+  if (threadIdx.x < solves) rot_ring_init(ring[threadIdx.x], (threadIdx.x == 0 ? M : ML) > 32 ? 2 : 1);
+  __syncthreads();
+  if (warp < solves) {  // chase warps
     const int dim = warp == 0 ? M : ML;
     double* rec = warp == 0 ? rec_hi : rec_lo;
     for (int i = lane; i < dim; i += 32) {
@@ -361,13 +369,19 @@ __global__ void __launch_bounds__(128) k_b_control(BatchDev B) {
       ee[warp][i] = (i + 1 < dim) ? s.beta[i] : 0.0;
     }
     __syncwarp();
-    const int bad = tridiag_qr_warp_cols(dim, dd[warp], ee[warp], rec + 2 + kBMaxK, kBMaxK, rot[warp]);
+    const int bad = tridiag_chase_warp(dim, dd[warp], ee[warp], ring[warp], B.kstatus);
     for (int i = lane; i < dim; i += 32) rec[2 + i] = dd[warp][i];
     if (lane == 0) {
       rec[0] = dim;
       rec[1] = bad;
       if (bad) s.status = 2;
     }
+  } else if (warp >= 2 && warp < 6) {  // row warps
+    const int which = (warp - 2) >> 1, half = (warp - 2) & 1;
+    const int dim = which == 0 ? M : ML;
+    if (which < solves && 32 * half < dim)
+      tridiag_rows_warp(dim, 32 * half + lane, (which == 0 ? rec_hi : rec_lo) + 2 + kBMaxK, kBMaxK, ring[which],
+                        B.kstatus);
   }
   __syncthreads();
   const double t_now = s.t_now;
@@ -388,11 +402,14 @@ __global__ void __launch_bounds__(128) k_b_control(BatchDev B) {
   }
   __syncthreads();
   for (int round = 0; round < 64; ++round) {
-    {
-      const double err = warp_step_error(rec_hi, rec_lo, exact, cand[warp], B.safety, norm, ph[warp], nullptr);
-      if (lane == 0) okf[warp] = err <= B.budget * cand[warp] / B.t_end;
+    if (pair < 4 && (is_hi || !exact)) warp_exponential(is_hi ? rec_hi : rec_lo, cand[pair], ph[warp], cf[warp]);
+    __syncthreads();
+    if (pair < 4 && is_hi) {
+      const double err = exact ? 0.0 : B.safety * norm * sqrt(warp_difference(cf[warp], M, cf[warp + 1], ML));
+      if (lane == 0) okf[pair] = err <= B.budget * cand[pair] / B.t_end;
     }
     __syncthreads();
+    int split = 0;
     if (threadIdx.x == 0) {
       int st = s_state;
       if (st == 0 && okf[0]) {
@@ -436,11 +453,18 @@ __global__ void __launch_bounds__(128) k_b_control(BatchDev B) {
           s_dt = s_lo;
           st = 3;
         } else {
-          const double l0 = log(s_lo), w = log(s_hi) - l0;
-          for (int k = 0; k < 4; ++k) cand[k] = exp(l0 + w * (k + 1) / 5.0);
+          split = 1;
         }
       }
       s_state = st;
+    }
+    if (warp == 0) {
+      split = __shfl_sync(0xffffffffu, split, 0);  // (orders lane 0's bracket before the reads)
+      __syncwarp();
+      if (split && lane < 4) {
+        const double l0 = log(s_lo), w = log(s_hi) - l0;
+        cand[lane] = exp(l0 + w * (lane + 1) / 5.0);
+      }
     }
     __syncthreads();
     if (s_state >= 3) break;
@@ -457,31 +481,31 @@ __global__ void __launch_bounds__(128) k_b_control(BatchDev B) {
   double dt = s_dt;
   if (remaining - dt < 1e-12) dt = remaining;
   double2* rows = B.coef + (size_t)b * (kMaxPts + 1) * kBMaxK;
-  // observation points inside (t_now, t_now + dt]
-  if (threadIdx.x == 0) {
-    int np = 0;
-    const double t_end_step = t_now + dt;
-    while (s.cursor + np < B.ntimes && np < kMaxPts && B.times[s.cursor + np] <= t_end_step + 1e-13) ++np;
-    s_np = np;
-  }
-  __syncthreads();
-  const int np = s_np;
+  // observation points inside (t_now, t_now + dt] (the times increase)
+  static_assert(kMaxPts <= kCtlWarps * 32, "one thread per possible observation point");
+  const int at = s.cursor + (int)threadIdx.x;
+  const int np = __syncthreads_count((int)threadIdx.x < kMaxPts && at < B.ntimes && B.times[at] <= t_now + dt + 1e-13);
   // point p < np: row p; p == np: the endpoint (row kMaxPts)
-  for (int p = warp; p <= np; p += 4) {
+  for (int p = pair; p <= np; p += kCtlPairs) {
     const bool endpoint = p == np;
     const double tau = endpoint ? dt : B.times[s.cursor + p] - t_now;
     double2* row = rows + (size_t)(endpoint ? kMaxPts : p) * kBMaxK;
-    const double err = warp_step_error(rec_hi, rec_lo, exact, tau, B.safety, norm, ph[warp], row);
-    for (int i = M + lane; i < kBMaxK; i += 32) row[i] = make_double2(0.0, 0.0);
-    if (lane == 0) {
-      if (endpoint) {
-        s.dt = dt;
-        s.step_err = err;
-        s.npts = np;
-      } else {
-        B.perr[(size_t)b * kMaxPts + p] = err;
+    if (is_hi || !exact) warp_exponential(is_hi ? rec_hi : rec_lo, tau, ph[warp], cf[warp]);
+    pair_sync(pair);
+    if (is_hi) {
+      const double err = exact ? 0.0 : B.safety * norm * sqrt(warp_difference(cf[warp], M, cf[warp + 1], ML));
+      for (int i = lane; i < kBMaxK; i += 32) row[i] = i < M ? cf[warp][i] : make_double2(0.0, 0.0);
+      if (lane == 0) {
+        if (endpoint) {
+          s.dt = dt;
+          s.step_err = err;
+          s.npts = np;
+        } else {
+          B.perr[(size_t)b * kMaxPts + p] = err;
+        }
       }
     }
+    pair_sync(pair);  // the coefficients are free for the pair's next point
   }
 }
 
@@ -1641,7 +1665,7 @@ static void record_step(rpm_batch* Bh, const BatchDev& B, const Layout& L, cudaS
   check_cuda(cudaStreamWaitEvent(Bh->side, Bh->ev_fork, 0), "fork wait");
   launch_gram(Bh, B);
   check_cuda(cudaEventRecord(Bh->ev_join, Bh->side), "join record");
-  k_b_control<<<B.ntraj, 128, ctl_smem, st>>>(B);
+  k_b_control<<<B.ntraj, kCtlWarps * 32, ctl_smem, st>>>(B);
   k_b_rebuild<<<ew, kEwThreads, 0, st>>>(B);
   check_cuda(cudaStreamWaitEvent(st, Bh->ev_join, 0), "join wait");
   k_b_observe<<<B.ntraj, 256, sizeof(double2) * kBMaxK * kBMaxK, st>>>(B);

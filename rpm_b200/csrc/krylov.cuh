@@ -4,6 +4,7 @@
 #include <cfloat>
 
 #include "common.cuh"
+#include "ptx.cuh"
 
 namespace rpm {
 
@@ -146,27 +147,39 @@ static __device__ int tridiag_qr(int m, double* d, double* e, double* z, int ldz
 }
 
 // ---------------------------------------------------------------------------
-// Tridiagonal eigen-decomposition by one warp
+// Tridiagonal eigen-decomposition by a chase warp and row warps
 // ---------------------------------------------------------------------------
 // Implicit symmetric tridiagonal QR with Wilkinson shifts (Golub & Van Loan,
-// section 8.3) run by ONE warp: every lane tests its off-diagonal entries
-// for deflation and the active block [p, q] comes from two ballots; lane 0
-// computes the shift and chases the bulge; every lane applies the sweep's
-// rotations to its rows of the eigenvector matrix.  d, e: diagonal and
-// off-diagonal (d -> eigenvalues); m <= 64.  z: m x m eigenvector matrix
-// stored by columns, z[k * ldz + i] = component i of eigenvector k, so that
-// the lanes' row updates touch consecutive addresses.  The rotations are
-// normalised with rsqrt and carry the entries the next rotation reads in
-// registers.  Returns 0 on convergence.
-static __device__ int tridiag_qr_warp_cols(int m, double* d, double* e, double* z, int ldz, double2* rot) {
-  const int lane = threadIdx.x & 31;
-  for (int idx = lane; idx < m * m; idx += 32) {
-    const int k = idx / m, i = idx - k * m;
-    z[k * ldz + i] = (i == k) ? 1.0 : 0.0;
+// section 8.3).  One warp runs the sweeps: every lane tests its off-diagonal
+// entries for deflation, the active block [p, q] comes from two ballots, lane
+// 0 computes the shift and chases the bulge (rotations normalised with rsqrt,
+// the entries the next rotation reads carried in registers).  The chase never
+// reads the eigenvectors, so it does not wait for them: it leaves each sweep's
+// rotations in a ring of slots, and row warps (32 rows each) apply them
+// meanwhile.  d, e: diagonal and off-diagonal (d -> eigenvalues); m <= 64.
+// z: eigenvectors by columns, z[k * ldz + i] = component i of eigenvector k, so
+// that the lanes' row updates touch consecutive addresses.
+constexpr int kRotSlots = 4;
+struct RotRing {
+  double2 rot[kRotSlots][64];
+  int p[kRotSlots], q[kRotSlots];  // q == 0: the end
+  unsigned long long full[kRotSlots], empty[kRotSlots];
+};
+
+// By one thread, before a block barrier.
+static __device__ void rot_ring_init(RotRing& r, int row_warps) {
+  for (int s = 0; s < kRotSlots; ++s) {
+    ptx::mbar_init(&r.full[s], 1);
+    ptx::mbar_init(&r.empty[s], row_warps);
   }
-  __syncwarp();
+  asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+}
+
+// The chase warp.  Returns 0 on convergence; status: wait-timeout word.
+static __device__ int tridiag_chase_warp(int m, double* d, double* e, RotRing& ring, int* status) {
+  const int lane = threadIdx.x & 31;
   int sweeps = 0;
-  while (true) {
+  for (int it = 0;; ++it) {
     // deflation: e[i] negligible against its neighbours on the diagonal
     bool nz[2];
 #pragma unroll
@@ -184,11 +197,23 @@ static __device__ int tridiag_qr_warp_cols(int m, double* d, double* e, double* 
     __syncwarp();
     // q - 1: the last nonzero off-diagonal; p: the start of its unreduced block
     const int q = nzm ? 64 - __clzll(nzm) : 0;
-    if (q == 0) return 0;
-    if (++sweeps > 40 * m) return 1;
+    const int slot = it % kRotSlots;
+    int ok = 1;
+    if (it >= kRotSlots && lane == 0)
+      ok = ptx::mbar_wait(&ring.empty[slot], (unsigned)((it / kRotSlots - 1) & 1), status) ? 1 : 0;
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+    if (q == 0 || ++sweeps > 40 * m || !ok) {
+      if (lane == 0) {
+        ring.q[slot] = 0;
+        ptx::mbar_arrive(&ring.full[slot]);
+      }
+      __syncwarp();
+      return q == 0 ? 0 : 1;
+    }
     const unsigned long long below = q >= 2 ? (~nzm) & ((1ull << (q - 1)) - 1ull) : 0ull;
     const int p = below ? 64 - __clzll(below) : 0;
     if (lane == 0) {
+      double2* rot = ring.rot[slot];
       const double delta = 0.5 * (d[q - 1] - d[q]);
       const double eq = e[q - 1];
       const double denom = delta + copysign(hypot(delta, eq), delta);
@@ -222,19 +247,56 @@ static __device__ int tridiag_qr_warp_cols(int m, double* d, double* e, double* 
         a = dk1;
         rot[k] = make_double2(c, sn);
       }
+      ring.p[slot] = p;
+      ring.q[slot] = q;
+      ptx::mbar_arrive(&ring.full[slot]);
     }
     __syncwarp();
-    for (int i = lane; i < m; i += 32) {
-      double zk = z[p * ldz + i];
-      for (int k = p; k < q; ++k) {
+  }
+}
+
+// A row warp: row `row` of the eigenvector matrix per lane (rows >= m idle).
+static __device__ void tridiag_rows_warp(int m, int row, double* z, int ldz, RotRing& ring, int* status) {
+  const int lane = threadIdx.x & 31;
+  if (row < m)
+    for (int k = 0; k < m; ++k) z[k * ldz + row] = k == row ? 1.0 : 0.0;
+  for (int it = 0;; ++it) {
+    const int slot = it % kRotSlots;
+    int ok = 1;
+    if (lane == 0) ok = ptx::mbar_wait(&ring.full[slot], (unsigned)((it / kRotSlots) & 1), status) ? 1 : 0;
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+    const int p = ring.p[slot], q = ring.q[slot];
+    if (!ok || q == 0) return;
+    if (row < m) {
+      const double2* rot = ring.rot[slot];
+      double* zr = z + row;
+      double zk = zr[p * ldz];
+      int k = p;
+      for (; k + 4 <= q; k += 4) {  // four rotations' operands ahead of their use
+        double2 cs[4];
+        double zn[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          cs[u] = rot[k + u];
+          zn[u] = zr[(k + u + 1) * ldz];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const double zk1 = zn[u];
+          zr[(k + u) * ldz] = cs[u].x * zk + cs[u].y * zk1;
+          zk = -cs[u].y * zk + cs[u].x * zk1;
+        }
+      }
+      for (; k < q; ++k) {
         const double2 cs = rot[k];
-        const double zk1 = z[(k + 1) * ldz + i];
-        z[k * ldz + i] = cs.x * zk + cs.y * zk1;
+        const double zk1 = zr[(k + 1) * ldz];
+        zr[k * ldz] = cs.x * zk + cs.y * zk1;
         zk = -cs.y * zk + cs.x * zk1;
       }
-      z[q * ldz + i] = zk;
+      zr[q * ldz] = zk;
     }
     __syncwarp();
+    if (lane == 0) ptx::mbar_arrive(&ring.empty[slot]);
   }
 }
 
