@@ -523,18 +523,20 @@ __global__ void __launch_bounds__(kCtlWarps * 32) k_b_control(BatchDev B) {
 // warps, the blocks), because a projection's last bit reaches FP32 elements;
 // the order is the one of a per-vector loop with two warp sums per vector,
 // which took 240 us per call on the uneven mix (6 vectors of 221,184, 10 of
-// 13,824 and 16 of 864 elements, 20 basis vectors on average).  Here a thread
-// loads kArnVec basis vectors' elements before it uses them, the warp sums of
-// kArnVec vectors share one transposed butterfly (9 exchanges instead of 40),
-// the last block stages the partials through shared memory, and blocks past a
-// trajectory's end leave at once.
-constexpr int kArnVec = 4;      // basis vectors per round
+// 13,824 and 16 of 864 elements, 20 basis vectors on average).  Here the next
+// two basis vectors' elements are on their way while two are summed, the warp
+// sums of two vectors share one transposed butterfly (6 exchanges instead of
+// 20), the vectors are split over kArnSplit blocks, the last block stages the
+// partials through shared memory, and every shape group has a launch of its
+// own size.
+constexpr int kArnVec = 2;      // basis vectors per round
+constexpr int kArnSplit = 3;    // blocks (grid z) that share a chunk's basis vectors
 constexpr int kArnFinish = 32;  // block partials staged per round of the final sum
 
 // Blocks that hold elements of a trajectory of n components.
 __device__ __forceinline__ int ew_blocks(long long n) { return (int)((n + kEwChunk - 1) / kEwChunk); }
 
-// As traj_last_block for the first `blocks` blocks of a trajectory.
+// As traj_last_block for `blocks` blocks of a trajectory.
 __device__ __forceinline__ bool traj_last_of(unsigned* counter, int blocks) {
   __shared__ bool is_last;
   __threadfence();
@@ -545,42 +547,49 @@ __device__ __forceinline__ bool traj_last_of(unsigned* counter, int blocks) {
   return is_last;
 }
 
-// Warp sums of eight values per lane by halving the set at each of the first
-// three butterfly levels: lane l ends with the sum of v[(l >> 2) & 7] (bit 4
-// selects v[4..7], bit 3 the upper pair, bit 2 the upper one).  The pairs that
-// are added are those of warp_sum, so the bits are too.
-__device__ __forceinline__ double warp_sum8(double (&v)[8]) {
+// Warp sums of four values per lane by halving the set at the first two
+// butterfly levels: lane l ends with the sum of v[(l >> 3) & 3] (bit 4 selects
+// v[2..3], bit 3 the odd one).  The pairs that are added are those of
+// warp_sum, so the bits are too.
+__device__ __forceinline__ double warp_sum4(const double (&v)[4]) {
   const int lane = threadIdx.x & 31;
+  const bool up = (lane & 16) != 0, odd = (lane & 8) != 0;
+  const double a = (up ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, up ? v[0] : v[2], 16);
+  const double b = (up ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, up ? v[1] : v[3], 16);
+  double t = (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
 #pragma unroll
-  for (int half = 4, o = 16; half >= 1; half >>= 1, o >>= 1) {
-    const bool up = (lane & o) != 0;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      if (c < half) {
-        const double keep = up ? v[c + half] : v[c];
-        const double give = up ? v[c] : v[c + half];
-        v[c] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-      }
-    }
-  }
-  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
-  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-  return v[0];
+  for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
 }
 
-__global__ void __launch_bounds__(kEwThreads, 2) k_b_arn_dots(BatchDev B, int j, int pass) {
+__global__ void __launch_bounds__(kEwThreads, 2) k_b_arn_dots(BatchDev B, int j, int pass, int b0) {
   // warp sums [warp][vector]; then the staged block partials [block][vector]
   __shared__ double2 red[kArnFinish][kBMaxK];
   __shared__ double rn[kEwThreads / 32];
   static_assert(kArnFinish >= kEwThreads / 32, "staging buffer holds the warp sums");
-  const int b = blockIdx.y;
+  const int b = b0 + blockIdx.y;
   TrajState& s = B.st[b];
   const long long n = s.n;
   const int blocks = ew_blocks(n);
   if ((int)blockIdx.x >= blocks || s.skip || (pass == 2 && s.cgs_done)) return;
+  // this block's basis vectors [i0, i1)
+  const int per = (j + kArnSplit) / kArnSplit;
+  const int v0 = min((int)blockIdx.z * per, j + 1), v1 = min(v0 + per, j + 1);
   const float2* base = B.V + (size_t)b * (B.m + 1) * B.ld;
   const float2* w = base + (size_t)(j + 1) * B.ld;
   const long long i0 = (long long)blockIdx.x * kEwChunk + threadIdx.x;
+  const bool whole = (long long)(blockIdx.x + 1) * kEwChunk <= n;  // no element past the end
+  auto fetch = [&](int i, float2 (&q)[kArnVec][kEwPer]) {
+#pragma unroll
+    for (int c = 0; c < kArnVec; ++c) {
+      const float2* v = base + (size_t)min(i + c, j) * B.ld + i0;
+#pragma unroll
+      for (int k = 0; k < kEwPer; ++k)
+        q[c][k] = whole || i0 + k * kEwThreads < n ? v[k * kEwThreads] : make_float2(0.f, 0.f);
+    }
+  };
+  float2 qa[kArnVec][kEwPer], qb[kArnVec][kEwPer];
+  if (v0 < v1) fetch(v0, qa);
   double2 wv[kEwPer];
 #pragma unroll
   for (int k = 0; k < kEwPer; ++k) {
@@ -588,24 +597,14 @@ __global__ void __launch_bounds__(kEwThreads, 2) k_b_arn_dots(BatchDev B, int j,
     wv[k] = e < n ? to_d2(w[e]) : make_double2(0.0, 0.0);
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (pass == 1) {  // |w|^2 before the projection (second-pass criterion)
+  if (pass == 1 && blockIdx.z == 0) {  // |w|^2 before the projection (second-pass criterion)
     double nn = 0.0;
 #pragma unroll
     for (int k = 0; k < kEwPer; ++k) nn = fma(wv[k].x, wv[k].x, fma(wv[k].y, wv[k].y, nn));
     nn = warp_sum(nn);
     if (lane == 0) rn[warp] = nn;
   }
-  for (int i = 0; i <= j; i += kArnVec) {
-    float2 q[kArnVec][kEwPer];
-#pragma unroll
-    for (int c = 0; c < kArnVec; ++c) {
-      const float2* v = base + (size_t)min(i + c, j) * B.ld;
-#pragma unroll
-      for (int k = 0; k < kEwPer; ++k) {
-        const long long e = i0 + (long long)k * kEwThreads;
-        q[c][k] = e < n ? v[e] : make_float2(0.f, 0.f);
-      }
-    }
+  auto project = [&](int i, const float2 (&q)[kArnVec][kEwPer]) {
     double acc[2 * kArnVec];
 #pragma unroll
     for (int c = 0; c < kArnVec; ++c) {
@@ -619,24 +618,30 @@ __global__ void __launch_bounds__(kEwThreads, 2) k_b_arn_dots(BatchDev B, int j,
       acc[2 * c] = ax;
       acc[2 * c + 1] = ay;
     }
-    const double t = warp_sum8(acc);
-    const int at = (lane >> 2) & 7;  // value of this lane: component at & 1 of vector i + at / 2
-    if ((lane & 3) == 0 && i + (at >> 1) <= j)
-      reinterpret_cast<double*>(&red[warp][i + (at >> 1)])[at & 1] = t;
+    const double t = warp_sum4(acc);
+    const int at = (lane >> 3) & 3;  // value of this lane: component at & 1 of vector i + at / 2
+    if ((lane & 7) == 0 && i + (at >> 1) < v1) reinterpret_cast<double*>(&red[warp][i + (at >> 1)])[at & 1] = t;
+  };
+  for (int i = v0; i < v1; i += 2 * kArnVec) {
+    if (i + kArnVec < v1) fetch(i + kArnVec, qb);
+    project(i, qa);
+    if (i + kArnVec >= v1) break;
+    if (i + 2 * kArnVec < v1) fetch(i + 2 * kArnVec, qa);
+    project(i + kArnVec, qb);
   }
   __syncthreads();
   double2* part = B.adots + ((size_t)b * B.nblk + blockIdx.x) * kBMaxK;
-  for (int i = threadIdx.x; i <= j; i += blockDim.x) {
+  for (int i = v0 + threadIdx.x; i < v1; i += blockDim.x) {
     double2 t = make_double2(0.0, 0.0);
     for (int w2 = 0; w2 < kEwThreads / 32; ++w2) t = cadd(t, red[w2][i]);
     part[i] = t;
   }
-  if (pass == 1 && threadIdx.x == 0) {
+  if (pass == 1 && blockIdx.z == 0 && threadIdx.x == 0) {
     double t = 0.0;
     for (int w2 = 0; w2 < kEwThreads / 32; ++w2) t += rn[w2];
     B.part[((size_t)b * B.nblk + blockIdx.x) * 2 + 1] = t;
   }
-  if (traj_last_of(B.count + b, blocks)) {
+  if (traj_last_of(B.count + b, blocks * kArnSplit)) {
     // partials of all blocks, added in block order
     const double2* parts = B.adots + (size_t)b * B.nblk * kBMaxK;
     const double* norms = B.part + (size_t)b * B.nblk * 2 + 1;
@@ -690,10 +695,10 @@ __global__ void __launch_bounds__(kEwThreads) k_b_arn_scale(BatchDev B, int j, i
 // that k_b_arn_dots read last are found in L2; a thread sums its elements side
 // by side (each element's sum runs over i in ascending order): 135 us per call
 // on the uneven mix before, with one element's chain of loads at a time.
-__global__ void __launch_bounds__(kEwThreads) k_b_arn_axpy(BatchDev B, int j, int pass) {
+__global__ void __launch_bounds__(kEwThreads) k_b_arn_axpy(BatchDev B, int j, int pass, int b0) {
   __shared__ float2 hc[kBMaxK];
   __shared__ double red[32];
-  const int b = gridDim.y - 1 - blockIdx.y;
+  const int b = b0 + gridDim.y - 1 - blockIdx.y;
   TrajState& s = B.st[b];
   const long long n = s.n;
   const int blocks = ew_blocks(n);
@@ -901,20 +906,22 @@ __device__ void cmatmul(int n, const double2* A, const double2* X, double2* C) {
 // matrix at most 1/2: truncation below 1e-22).  P, Q, R: n x n scratch.
 __device__ void hessenberg_expm(const double2* hess, int n, double h, double2* P, double2* Q, double2* R,
                                 double2* out) {
-  __shared__ double s_norm;
+  __shared__ double s_norm, s_col[kBMaxK];
   for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
     const int r = idx / n, c = idx - r * n;
     const double2 v = hess[(size_t)r * kBMaxK + c];
     P[idx] = make_double2(v.y * h, -v.x * h);  // -i h H
   }
   __syncthreads();
+  for (int c = threadIdx.x; c < n; c += blockDim.x) {
+    double col = 0.0;
+    for (int r = 0; r < n; ++r) col += hypot(P[r * n + c].x, P[r * n + c].y);
+    s_col[c] = col;
+  }
+  __syncthreads();
   if (threadIdx.x == 0) {
     double best = 0.0;
-    for (int c = 0; c < n; ++c) {
-      double col = 0.0;
-      for (int r = 0; r < n; ++r) col += hypot(P[r * n + c].x, P[r * n + c].y);
-      best = fmax(best, col);
-    }
+    for (int c = 0; c < n; ++c) best = fmax(best, s_col[c]);
     s_norm = best;
   }
   __syncthreads();
@@ -955,7 +962,10 @@ __device__ void hessenberg_expm(const double2* hess, int n, double h, double2* P
 // whose embedded error (the reference's estimate, rpm_statevector_engine.py:
 // 690-715) meets budget * k h / T.  Every grid point of the step is an
 // observation point.  Dynamic shared memory: three kBMaxK^2 complex buffers.
-__global__ void __launch_bounds__(128) k_b_control_arn(BatchDev B) {
+// The matrix products are the time: 16 warps share their elements (742 us per
+// step at M = 40 with four, and the norm's columns summed by one thread).
+constexpr int kArnCtlThreads = 512;
+__global__ void __launch_bounds__(kArnCtlThreads) k_b_control_arn(BatchDev B) {
   extern __shared__ double2 scratch[];
   __shared__ double2 chi[kBMaxK], clo[kBMaxK], nhi[kBMaxK], nlo[kBMaxK];
   __shared__ double red[32];
@@ -1321,8 +1331,14 @@ struct rpm_batch {
     int b0, nb;
     rpm::CubePlan plan;
     bool records;  // every member carries the outer-index records of the persistent kernel
+    int blocks;    // blocks of kEwChunk components per trajectory
+    long long work() const { return (long long)blocks * nb; }
   };
   std::vector<ShapeGroup> groups;
+  // Arnoldi: one stream and join event per shape group (as many as the largest
+  // number of groups so far)
+  std::vector<cudaStream_t> gstreams;
+  std::vector<cudaEvent_t> gevents;
   int dot_stride = 1;  // partial-sum slots per trajectory
   std::vector<int> caps;  // Krylov cap per system (0: the batch's dimension)
 };
@@ -1422,6 +1438,18 @@ static HpsiArgs<float2> group_args(const HpsiArgs<float2>& a, int b0, int dstrid
   return c;
 }
 
+// Streams and events for every shape group.
+static void group_streams(rpm_batch* Bh) {
+  while (Bh->gstreams.size() < Bh->groups.size()) {
+    cudaStream_t st = nullptr;
+    cudaEvent_t ev = nullptr;
+    check_cuda(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "create group stream");
+    Bh->gstreams.push_back(st);
+    check_cuda(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "create group event");
+    Bh->gevents.push_back(ev);
+  }
+}
+
 static void record_step(rpm_batch* Bh, const BatchDev& B, const Layout& L, cudaStream_t st) {
   char* base = static_cast<char*>(Bh->buf);
   const int m = B.m;
@@ -1461,6 +1489,16 @@ static void record_step(rpm_batch* Bh, const BatchDev& B, const Layout& L, cudaS
   int per_iter = 0;
   for (size_t g = 0; g < Bh->groups.size(); ++g) per_iter += gfused[g] ? 2 : 3;
   if (B.arnoldi) {
+    // The shape groups are independent until the controller: each runs its
+    // iterations on a stream of its own beside the largest one (the small
+    // groups' launches were 22 of 280 us per iteration of the uneven mix).
+    size_t lead = 0;
+    for (size_t g = 1; g < Bh->groups.size(); ++g)
+      if (Bh->groups[g].work() > Bh->groups[lead].work()) lead = g;
+    group_streams(Bh);
+    check_cuda(cudaEventRecord(Bh->ev_fork, st), "group fork record");
+    for (size_t g = 0; g < Bh->groups.size(); ++g)
+      if (g != lead) check_cuda(cudaStreamWaitEvent(Bh->gstreams[g], Bh->ev_fork, 0), "group fork wait");
     for (int j = 0; j < m; ++j) {
       a.in = B.V + (size_t)j * B.ld;
       a.out = B.V + (size_t)(j + 1) * B.ld;
@@ -1471,35 +1509,43 @@ static void record_step(rpm_batch* Bh, const BatchDev& B, const Layout& L, cudaS
       z.j = j;
       a.dot_out = nullptr;
       a.dot_part = nullptr;
-      if (j == probe_j) check_cuda(cudaEventRecordWithFlags(Bh->probe0, st, probe_flags), "probe record");
       for (size_t g = 0; g < Bh->groups.size(); ++g) {
         const auto& G = Bh->groups[g];
+        cudaStream_t sg = g == lead ? st : Bh->gstreams[g];
         HpsiArgs<float2> ak = group_args(a, G.b0, D);
         float2* yk = ya + (size_t)G.b0 * B.ld;
+        if (g == lead && j == probe_j)
+          check_cuda(cudaEventRecordWithFlags(Bh->probe0, st, probe_flags), "probe record");
         if (gfused[g]) {
           ak.lz.on = 2;  // pass R scales v_j (written back) while staging
-          if (!launch_cube_fast(ak, G.plan, yk, G.nb, st)) fail(RPM_E_INVALID, "H psi passes unavailable");
+          if (!launch_cube_fast(ak, G.plan, yk, G.nb, sg)) fail(RPM_E_INVALID, "H psi passes unavailable");
         } else {
           // one shape per launch: H (scale V_j), then V_j *= scale
-          launch_cube<float2>(ak, G.plan, yk, G.nb, st);
-          k_b_arn_scale<<<dim3(B.nblk, G.nb), kEwThreads, 0, st>>>(B, j, G.b0);
+          launch_cube<float2>(ak, G.plan, yk, G.nb, sg);
+          k_b_arn_scale<<<dim3(G.blocks, G.nb), kEwThreads, 0, sg>>>(B, j, G.b0);
+        }
+        if (g == lead && j == probe_j)
+          check_cuda(cudaEventRecordWithFlags(Bh->probe1, st, probe_flags), "probe record");
+        for (int pass = 1; pass <= 2; ++pass) {
+          k_b_arn_dots<<<dim3(G.blocks, G.nb, kArnSplit), kEwThreads, 0, sg>>>(B, j, pass, G.b0);
+          k_b_arn_axpy<<<dim3(G.blocks, G.nb), kEwThreads, 0, sg>>>(B, j, pass, G.b0);
         }
       }
-      if (j == probe_j) check_cuda(cudaEventRecordWithFlags(Bh->probe1, st, probe_flags), "probe record");
-      for (int pass = 1; pass <= 2; ++pass) {
-        k_b_arn_dots<<<ew, kEwThreads, 0, st>>>(B, j, pass);
-        k_b_arn_axpy<<<ew, kEwThreads, 0, st>>>(B, j, pass);
-      }
+    }
+    for (size_t g = 0; g < Bh->groups.size(); ++g) {
+      if (g == lead) continue;
+      check_cuda(cudaEventRecord(Bh->gevents[g], Bh->gstreams[g]), "group join record");
+      check_cuda(cudaStreamWaitEvent(st, Bh->gevents[g], 0), "group join wait");
     }
     Bh->fused = false;
     Bh->persistent = false;
     Bh->probe_iters = 1;
-    Bh->launches_per_step = 1 + (per_iter + 4) * m + 4;
+    Bh->launches_per_step = 1 + (per_iter + 4 * (int)Bh->groups.size()) * m + 4;
     check_cuda(cudaEventRecord(Bh->ev_fork, st), "fork record");
     check_cuda(cudaStreamWaitEvent(Bh->side, Bh->ev_fork, 0), "fork wait");
     launch_gram(Bh, B);
     check_cuda(cudaEventRecord(Bh->ev_join, Bh->side), "join record");
-    k_b_control_arn<<<B.ntraj, 128, kArnCtlSmem, st>>>(B);
+    k_b_control_arn<<<B.ntraj, kArnCtlThreads, kArnCtlSmem, st>>>(B);
     k_b_rebuild<<<ew, kEwThreads, 0, st>>>(B);
     check_cuda(cudaStreamWaitEvent(st, Bh->ev_join, 0), "join wait");
     k_b_observe<<<B.ntraj, 256, sizeof(double2) * kBMaxK * kBMaxK, st>>>(B);
@@ -1708,7 +1754,8 @@ static void run_batch(rpm_batch* Bh, int ntraj, const int* sys_of, void* psi, co
     }
     bool records = true;
     for (const rpm_system* sk : members) records = records && sk->cube32.orecR && sk->cube32.orecL;
-    Bh->groups.push_back({b, e - b, cube_plan(members.data(), (int)members.size()), records});
+    const int blocks = (int)((Bh->systems[sys_of[b]]->n + kEwChunk - 1) / kEwChunk);
+    Bh->groups.push_back({b, e - b, cube_plan(members.data(), (int)members.size()), records, blocks});
     b = e;
   }
   // partial-sum slots per trajectory: general pass R (grid.x <= nl) or fused pass L (3 per block)
@@ -1875,8 +1922,11 @@ static void release_batch(rpm_batch* batch) {
   free_graph(batch);
   if (batch->work) cudaStreamSynchronize(batch->work);
   if (batch->side) cudaStreamSynchronize(batch->side);
+  for (cudaStream_t st : batch->gstreams) cudaStreamSynchronize(st);
   if (batch->buf) cudaFree(batch->buf);
   if (batch->views_dev) cudaFree(batch->views_dev);
+  for (cudaEvent_t ev : batch->gevents) cudaEventDestroy(ev);
+  for (cudaStream_t st : batch->gstreams) cudaStreamDestroy(st);
   if (batch->ev_fork) cudaEventDestroy(batch->ev_fork);
   if (batch->ev_join) cudaEventDestroy(batch->ev_join);
   if (batch->side) cudaStreamDestroy(batch->side);
