@@ -74,6 +74,7 @@ struct BatchDev {
   double* part;     // [traj][nblk][2]
   unsigned* count;  // [traj] completion counters (elementwise reductions)
   double2* gpart;   // [traj][gblk][kBMaxK * kBMaxK]
+  double2* gram;    // [traj][kBMaxK * kBMaxK] sum over the blocks
   double* values;   // [traj][ntimes]
   double* errs;     // [traj][ntimes]
   int nblk, gblk;
@@ -1221,20 +1222,29 @@ __global__ void __launch_bounds__(256) k_b_gram(BatchDev B) {
   }
 }
 
+// Gram of a trajectory's basis: its blocks' partials added in block order
+// (M x M, on the Gram's stream beside the rebuild).
+__global__ void __launch_bounds__(256) k_b_gram_sum(BatchDev B) {
+  const int b = blockIdx.y;
+  const TrajState& s = B.st[b];
+  if (s.done) return;
+  const int pr = blockIdx.x * blockDim.x + threadIdx.x;
+  if (pr >= s.msize * s.msize) return;
+  double2 t = make_double2(0.0, 0.0);
+  const double2* p = B.gpart + (size_t)b * B.gblk * kBMaxK * kBMaxK + pr;
+#pragma unroll 8
+  for (int k = 0; k < B.gblk; ++k) t = cadd(t, p[(size_t)k * kBMaxK * kBMaxK]);
+  B.gram[(size_t)b * kBMaxK * kBMaxK + pr] = t;
+}
+
 // Populations at the step's observation points and the controller update.
-__global__ void __launch_bounds__(256) k_b_observe(BatchDev B) {
+__global__ void __launch_bounds__(512) k_b_observe(BatchDev B) {
   extern __shared__ double2 G[];  // M x M
   const int b = blockIdx.x;
   TrajState& s = B.st[b];
   if (s.done) return;
   const int M = s.msize;
-  const int pairs = M * M;
-  for (int pr = threadIdx.x; pr < pairs; pr += blockDim.x) {
-    double2 t = make_double2(0.0, 0.0);
-    const double2* p = B.gpart + (size_t)b * B.gblk * kBMaxK * kBMaxK + pr;
-    for (int k = 0; k < B.gblk; ++k) t = cadd(t, p[(size_t)k * kBMaxK * kBMaxK]);
-    G[pr] = t;
-  }
+  for (int pr = threadIdx.x; pr < M * M; pr += blockDim.x) G[pr] = B.gram[(size_t)b * kBMaxK * kBMaxK + pr];
   __syncthreads();
   const double n2 = s.norm * s.norm;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -1245,6 +1255,7 @@ __global__ void __launch_bounds__(256) k_b_observe(BatchDev B) {
     for (int i = lane; i < M; i += 32) {
       // (G c)_i with G Hermitian-symmetrised on the fly
       double2 gc = make_double2(0.0, 0.0);
+#pragma unroll 4
       for (int k = 0; k < M; ++k) {
         const double2 g1 = G[i * M + k], g2 = G[k * M + i];
         const double2 g = make_double2(0.5 * (g1.x + g2.x), 0.5 * (g1.y - g2.y));
@@ -1349,8 +1360,13 @@ namespace rpm {
 // k_b_gram, 1 the tensor-core k_b_gram_tc where the batch allows it.
 static std::atomic<int> g_gram_kernel{1};
 
-// The singlet Gram of the step's basis, on the side stream (it overlaps the
-// controller and the rebuild).
+// The singlet Gram of the step's basis, on the side stream.  It is launched
+// after the controller: its blocks take whole SMs, and a controller queued
+// behind them started when the last of them had left (48 trajectories of
+// 221,184: Gram 951, controller 393 and rebuild 596 us one after the other;
+// now 1040 us for the first two; 30 of 13,824: 300 -> 218 us).  Node priorities
+// that let the rebuild in between gained nothing more (each of the two fills
+// the SMs), nor did a Gram of 128 registers beside the rebuild (it spills).
 static void launch_gram(const rpm_batch* Bh, const BatchDev& B) {
   if (Bh->gram_tc) {
     const CUtensorMap map = basis_rows_map(B.V, (long long)B.ntraj * (B.m + 1), B.ld, gramtc::kGC, B.m + 1);
@@ -1358,6 +1374,7 @@ static void launch_gram(const rpm_batch* Bh, const BatchDev& B) {
   }
   else
     k_b_gram<<<dim3(B.gblk, B.ntraj), 256, 0, Bh->side>>>(B);
+  k_b_gram_sum<<<dim3((B.m * B.m + 255) / 256, B.ntraj), 256, 0, Bh->side>>>(B);
 }
 
 static void free_graph(rpm_batch* B) {
@@ -1369,7 +1386,7 @@ static void free_graph(rpm_batch* B) {
 }
 
 struct Layout {
-  size_t st, V, coef, perr, part, count, gpart, ya, dotpart, dotcount, times, sysof, nof, active, hess, hcur, adots,
+  size_t st, V, coef, perr, part, count, gpart, gram, ya, dotpart, dotcount, times, sysof, nof, active, hess, hcur, adots,
       expm, prog, pcnt, ppart, work, kstatus, capof, total;
 };
 
@@ -1390,6 +1407,7 @@ static Layout layout(const rpm_batch* B, int ntraj, int ntimes, int nblk, int gb
   L.part = take(sizeof(double) * (size_t)ntraj * nblk * 2);
   L.count = take(sizeof(unsigned) * ntraj);
   L.gpart = take(sizeof(double2) * (size_t)ntraj * gblk * kBMaxK * kBMaxK);
+  L.gram = take(sizeof(double2) * (size_t)ntraj * kBMaxK * kBMaxK);
   L.ya = take(sizeof(float2) * (size_t)ntraj * B->ld);
   L.dotpart = take(sizeof(double) * (size_t)ntraj * dot_blocks);
   L.dotcount = take(sizeof(unsigned) * ntraj);
@@ -1540,15 +1558,15 @@ static void record_step(rpm_batch* Bh, const BatchDev& B, const Layout& L, cudaS
     Bh->fused = false;
     Bh->persistent = false;
     Bh->probe_iters = 1;
-    Bh->launches_per_step = 1 + (per_iter + 4 * (int)Bh->groups.size()) * m + 4;
+    Bh->launches_per_step = 1 + (per_iter + 4 * (int)Bh->groups.size()) * m + 5;
     check_cuda(cudaEventRecord(Bh->ev_fork, st), "fork record");
+    k_b_control_arn<<<B.ntraj, kArnCtlThreads, kArnCtlSmem, st>>>(B);
     check_cuda(cudaStreamWaitEvent(Bh->side, Bh->ev_fork, 0), "fork wait");
     launch_gram(Bh, B);
     check_cuda(cudaEventRecord(Bh->ev_join, Bh->side), "join record");
-    k_b_control_arn<<<B.ntraj, kArnCtlThreads, kArnCtlSmem, st>>>(B);
     k_b_rebuild<<<ew, kEwThreads, 0, st>>>(B);
     check_cuda(cudaStreamWaitEvent(st, Bh->ev_join, 0), "join wait");
-    k_b_observe<<<B.ntraj, 256, sizeof(double2) * kBMaxK * kBMaxK, st>>>(B);
+    k_b_observe<<<B.ntraj, 512, sizeof(double2) * kBMaxK * kBMaxK, st>>>(B);
     check_launch("batched Arnoldi step");
     return;
   }
@@ -1705,16 +1723,16 @@ static void record_step(rpm_batch* Bh, const BatchDev& B, const Layout& L, cudaS
   for (size_t g = 0; g < Bh->groups.size(); ++g)
     if (!gpers[g] && !gsmall[g]) per_iter_rest += gfused[g] ? 2 : 3;
   const int nreo = reo > 0 ? (m - 1) / reo : 0;  // iterations j = P-1, 2P-1, ... <= m-2
-  Bh->launches_per_step = 1 + nsmall + npers * nseg + per_iter_rest * m + 4 * nreo + 4;
+  Bh->launches_per_step = 1 + nsmall + npers * nseg + per_iter_rest * m + 4 * nreo + 5;
   const size_t ctl_smem = sizeof(double) * 2 * kRecDoubles;
   check_cuda(cudaEventRecord(Bh->ev_fork, st), "fork record");
+  k_b_control<<<B.ntraj, kCtlWarps * 32, ctl_smem, st>>>(B);
   check_cuda(cudaStreamWaitEvent(Bh->side, Bh->ev_fork, 0), "fork wait");
   launch_gram(Bh, B);
   check_cuda(cudaEventRecord(Bh->ev_join, Bh->side), "join record");
-  k_b_control<<<B.ntraj, kCtlWarps * 32, ctl_smem, st>>>(B);
   k_b_rebuild<<<ew, kEwThreads, 0, st>>>(B);
   check_cuda(cudaStreamWaitEvent(st, Bh->ev_join, 0), "join wait");
-  k_b_observe<<<B.ntraj, 256, sizeof(double2) * kBMaxK * kBMaxK, st>>>(B);
+  k_b_observe<<<B.ntraj, 512, sizeof(double2) * kBMaxK * kBMaxK, st>>>(B);
   check_launch("batched step");
 }
 
@@ -1807,6 +1825,7 @@ static void run_batch(rpm_batch* Bh, int ntraj, const int* sys_of, void* psi, co
   B.part = reinterpret_cast<double*>(base + L.part);
   B.count = reinterpret_cast<unsigned*>(base + L.count);
   B.gpart = reinterpret_cast<double2*>(base + L.gpart);
+  B.gram = reinterpret_cast<double2*>(base + L.gram);
   B.values = values;
   B.errs = errs;
   B.nblk = nblk;
