@@ -186,8 +186,8 @@ struct CubeView {
   const void* orecR;
   const void* orecL;
   int orec_bytes_r, orec_bytes_l;
-  // complex128 views of standard-layout systems: per group index of each
-  // radical the records of the direct H psi (hpsi_direct.cuh); else null
+  // standard-layout systems: per group index of each radical the records of
+  // the direct H psi (hpsi_direct.cuh, hpsi_direct32.cu); else null
   const void* lrec;
   const void* rrec;
   // complex128: bit k set when nucleus k of the radical has any transition to

@@ -721,6 +721,18 @@ static bool try_direct(rpm_system* sys, const T* in, T* out, int batch, long lon
   return false;
 }
 
+// rpm_hpsi's complex64 calls take the direct form too (never the batched
+// propagation and the adjoint, whose results keep the passes' order of
+// additions).
+static bool try_direct32(rpm_system* sys, const float2* in, float2* out, int batch, long long ld, cudaStream_t stream) {
+  const CubeTuning tu = cube_tuning();
+  if (tu.ni_l || tu.ni_r || tu.tr || tu.tl || batch < 1 || batch > 65535 || !sys->on_device ||
+      !direct32_usable(sys, in, out, ld))
+    return false;
+  launch_direct32(sys, in, out, batch, ld, stream);
+  return true;
+}
+
 template <class T>
 void launch_hpsi(rpm_system* sys, const T* in, T* out, int batch, long long ld, cudaStream_t stream) {
   if (!sys->on_device) fail(RPM_E_INVALID, "system was created host-only");
@@ -805,7 +817,9 @@ extern "C" int rpm_hpsi(rpm_system* sys, int precision, const void* psi_dev, voi
     if (precision == RPM_PREC_C128) {
       rpm::launch_hpsi<double2>(sys, static_cast<const double2*>(psi_dev), static_cast<double2*>(out_dev), batch, ld, st);
     } else if (precision == RPM_PREC_C64) {
-      rpm::launch_hpsi<float2>(sys, static_cast<const float2*>(psi_dev), static_cast<float2*>(out_dev), batch, ld, st);
+      const auto* x = static_cast<const float2*>(psi_dev);
+      auto* y = static_cast<float2*>(out_dev);
+      if (!rpm::try_direct32(sys, x, y, batch, ld, st)) rpm::launch_hpsi<float2>(sys, x, y, batch, ld, st);
     } else {
       rpm::fail(RPM_E_INVALID, "precision must be 64 or 128");
     }
@@ -871,6 +885,9 @@ static void launch_hpsi_noalloc(rpm_system* sys, const T* in, T* out, int batch,
   // the kernel choice of launch_hpsi: the direct form (no scratch), the cube
   // form, else the CSR passes, else the per-term kernel (no scratch)
   if (try_direct<T>(sys, in, out, batch, ld, nullptr, stream)) return;
+  if constexpr (std::is_same<T, float2>::value) {
+    if (try_direct32(sys, in, out, batch, ld, stream)) return;
+  }
   T* ya = static_cast<T*>(noalloc_scratch());
   if (sys->cube && sys->cube64.inner_l >= 1 && sys->cube64.inner_r >= 1) {
     HpsiArgs<T> a{};

@@ -147,5 +147,10 @@ bool direct_usable(const rpm_system* sys);
 // null for 1).  No scratch.
 void launch_direct(rpm_system* sys, const double2* in, double2* out, int batch, long long ld, const double* scale_dev,
                    cudaStream_t stream);
+// The complex64 form (hpsi_direct32.cu): the same layout with a spin-1/2 as
+// fastest right nucleus, 16-byte aligned pointers and an even stride.
+bool direct32_usable(const rpm_system* sys, const float2* in, const float2* out, long long ld);
+void launch_direct32(rpm_system* sys, const float2* in, float2* out, int batch, long long ld, cudaStream_t stream);
+std::vector<unsigned char> direct32_records(const CubeSide& side, const std::vector<cd>& tab);
 
 }  // namespace rpm

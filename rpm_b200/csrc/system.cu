@@ -432,6 +432,11 @@ static void upload_system(rpm_system* sys) {
         const auto lr = direct_records(cl, tl64), rr = direct_records(cr, tr64);
         c64.lrec = upload<direct::HRec>(sys, lr.data(), lr.size() * sizeof(direct::HRec));
         c64.rrec = upload<direct::HRec>(sys, rr.data(), rr.size() * sizeof(direct::HRec));
+        if (cr.dim[cr.K - 1] == 2) {
+          const auto l32 = direct32_records(cl, sys->cube_tab_l), r32 = direct32_records(cr, sys->cube_tab_r);
+          c32.lrec = upload<unsigned char>(sys, l32.data(), l32.size());
+          c32.rrec = upload<unsigned char>(sys, r32.data(), r32.size());
+        }
       }
       sys->cube64_dev = upload<CubeView<double2>>(sys, &c64, sizeof(c64));
       sys->cube32_dev = upload<CubeView<float2>>(sys, &c32, sizeof(c32));

@@ -101,3 +101,50 @@ def test_full_size_action_matches_general_kernels():
     finally:
         _lib.call("rpm_set_cube_tuning", 0, 0, 0, 0)
     assert float(torch.linalg.vector_norm(a - b) / torch.linalg.vector_norm(b)) < REL
+
+
+# fastest right nucleus a spin-1/2 (the complex64 form's condition): a lone
+# right nucleus, index-pair counts below, at and around one 128-thread block,
+# spins above 1/2 before it
+SHAPES32 = [((2,), (2,)), ((3,), (2, 2)), ((5, 3), (7, 2)), ((16,), (8, 2)), ((2, 3, 4), (4, 3, 2, 2)),
+            ((3, 2, 2, 2), (3, 2, 2, 2, 2, 2))]
+
+
+@pytest.mark.parametrize("case", range(len(SHAPES32)))
+@pytest.mark.parametrize("batch,rates", [(1, None), (3, (1.0, 2.5))])
+@pytest.mark.parametrize("offset,pad", [(0, 6), (1, 6), (0, 5)])
+def test_complex64_action_matches_dense(case, batch, rates, offset, pad):
+    """offset 1 (8-byte aligned) and the odd stride take the general passes.
+
+    Bar 2e-6 of the norm: fewer than 200 products of rounding 6e-8, as a random sum 200^0.5 x 6e-8 = 0.9e-6.
+    """
+    import torch
+
+    import rpm_b200 as rb
+    from rpm_b200 import _lib
+
+    left, right = SHAPES32[case]
+    dims = (2, 2) + left + right
+    rng = np.random.default_rng(200 + case)
+    terms = _terms(rb, rng, left, right, pair=case % 2 == 0)
+    h = rb.CompiledFullPairHamiltonian(dims, terms, left_axes=(0,) + tuple(range(2, 2 + len(left))),
+                                       right_axes=(1,) + tuple(range(2 + len(left), len(dims))))
+    n = h.dimension
+    x = (rng.normal(size=(n, batch)) + 1j * rng.normal(size=(n, batch))).astype(np.complex64)
+    ref = _dense_apply(dims, terms, x.astype(np.complex128))
+    if rates is not None:
+        h.set_recombination_rates(*rates)
+        ps = np.zeros((4, 4))
+        ps[1:3, 1:3] = [[0.5, -0.5], [-0.5, 0.5]]
+        extra = rb.LocalTerm((0, 1), -0.5j * (rates[1] - rates[0]) * (np.eye(4) - ps))
+        ref = ref + _dense_apply(dims, [extra], x)
+    ld = n + pad
+    store = torch.full((2, offset + batch * ld), 7.0, dtype=torch.complex64, device="cuda")
+    xs, out = (store[k, offset:].view(batch, ld) for k in range(2))
+    xs.fill_(float("nan"))
+    xs[:, :n] = torch.from_numpy(np.ascontiguousarray(x.T))
+    _lib.call("rpm_hpsi", h._system.handle, _lib.PREC_C64, _lib.ptr(xs), _lib.ptr(out), batch, ld,
+              _lib.stream_handle())
+    got = out.cpu().numpy()
+    assert np.linalg.norm(got[:, :n].T - ref) <= 2e-6 * np.linalg.norm(ref)
+    assert np.all(got[:, n:] == 7.0)
