@@ -334,7 +334,8 @@ __device__ __forceinline__ void pair_sync(int pair) { asm volatile("bar.sync %0,
 // evaluates one time, hi and lo side by side, eight times at once.
 // Latency-bound FP64 chains: with four warps in all, every warp applying its
 // own rotations and evaluating hi and lo one after the other, a step took 233
-// us at M = 30 and 472 us at M = 40.
+// us at M = 30 and 472 us at M = 40; with branches in each rotation of the
+// chase 197 and 340 us; now 171 us at M = 30.
 // Dynamic shared memory: two spectra records (hi, lo).
 constexpr int kCtlWarps = 16;
 constexpr int kCtlPairs = kCtlWarps / 2;
@@ -343,7 +344,7 @@ __global__ void __launch_bounds__(kCtlWarps * 32) k_b_control(BatchDev B) {
   extern __shared__ double sm[];
   __shared__ RotRing ring[2];
   __shared__ double2 ph[kCtlWarps][kBMaxK], cf[kCtlWarps][kBMaxK];
-  __shared__ double dd[2][kBMaxK], ee[2][kBMaxK];
+  __shared__ double dd[2][kBMaxK + 2], ee[2][kBMaxK + 3];  // padded for the chase
   __shared__ double cand[4];
   __shared__ int okf[4];
   __shared__ double s_dt, s_lo, s_hi;
@@ -365,12 +366,13 @@ __global__ void __launch_bounds__(kCtlWarps * 32) k_b_control(BatchDev B) {
   if (warp < solves) {  // chase warps
     const int dim = warp == 0 ? M : ML;
     double* rec = warp == 0 ? rec_hi : rec_lo;
-    for (int i = lane; i < dim; i += 32) {
-      dd[warp][i] = s.alpha[i];
-      ee[warp][i] = (i + 1 < dim) ? s.beta[i] : 0.0;
+    double* ew = ee[warp] + 1;
+    for (int i = lane; i < dim + 2; i += 32) {
+      dd[warp][i] = i < dim ? s.alpha[i] : 0.0;
+      ew[i] = (i + 1 < dim) ? s.beta[i] : 0.0;
     }
     __syncwarp();
-    const int bad = tridiag_chase_warp(dim, dd[warp], ee[warp], ring[warp], B.kstatus);
+    const int bad = tridiag_chase_warp(dim, dd[warp], ew, ring[warp], B.kstatus);
     for (int i = lane; i < dim; i += 32) rec[2 + i] = dd[warp][i];
     if (lane == 0) {
       rec[0] = dim;

@@ -156,7 +156,9 @@ static __device__ int tridiag_qr(int m, double* d, double* e, double* z, int ldz
 // the entries the next rotation reads carried in registers).  The chase never
 // reads the eigenvectors, so it does not wait for them: it leaves each sweep's
 // rotations in a ring of slots, and row warps (32 rows each) apply them
-// meanwhile.  d, e: diagonal and off-diagonal (d -> eigenvalues); m <= 64.
+// meanwhile.  d, e: diagonal and off-diagonal (d -> eigenvalues); m <= 64;
+// d[m .. m + 1] and e[-1], e[m - 1 .. m + 1] are padding, e's zero: a rotation
+// takes no branch (its last and first are not treated apart).
 // z: eigenvectors by columns, z[k * ldz + i] = component i of eigenvector k, so
 // that the lanes' row updates touch consecutive addresses.
 constexpr int kRotSlots = 4;
@@ -218,35 +220,33 @@ static __device__ int tridiag_chase_warp(int m, double* d, double* e, RotRing& r
       const double eq = e[q - 1];
       const double denom = delta + copysign(hypot(delta, eq), delta);
       const double mu = d[q] - eq * eq / denom;
-      double x = d[p] - mu, y = e[p];
       double a = d[p], bb = e[p];  // d[k] and e[k] as the previous rotation left them
+      double x = a - mu, y = bb;
+      double cc = d[p + 1], en = e[p + 1];  // e[q] = 0; the padding behind it is never used
       for (int k = p; k < q; ++k) {
-        const double cc = d[k + 1];
-        const double en = k + 1 < q ? e[k + 1] : 0.0;
-        double c = 1.0, sn = 0.0, r = 0.0;
+        // the next rotation's operands, ahead of this one's stores
+        const double cn = d[k + 2], en2 = e[k + 2];
         const double rr = fma(x, x, y * y);
-        if (rr > 0.0) {
-          const double inv = rsqrt(rr);
-          c = x * inv;
-          sn = y * inv;
-          r = rr * inv;
-        }
-        if (k > p) e[k - 1] = r;
+        const double inv = rsqrt(rr);
+        const bool turn = rr > 0.0;
+        const double c = turn ? x * inv : 1.0, sn = turn ? y * inv : 0.0, r = turn ? rr * inv : 0.0;
         const double dk = c * c * a + 2.0 * c * sn * bb + sn * sn * cc;
         const double dk1 = sn * sn * a - 2.0 * c * sn * bb + c * c * cc;
         const double ek = c * sn * (cc - a) + (c * c - sn * sn) * bb;
-        d[k] = dk;
-        d[k + 1] = dk1;
-        e[k] = ek;
-        if (k + 1 < q) {
-          x = ek;
-          y = sn * en;
-          bb = c * en;
-          e[k + 1] = bb;
-        }
+        x = ek;
+        y = sn * en;
+        bb = c * en;
         a = dk1;
+        e[k - 1] = r;  // e[p - 1]: put back below
+        d[k] = dk;
+        e[k + 1] = bb;
         rot[k] = make_double2(c, sn);
+        cc = cn;
+        en = en2;
       }
+      d[q] = a;
+      e[q - 1] = x;
+      e[p - 1] = 0.0;
       ring.p[slot] = p;
       ring.q[slot] = q;
       ptx::mbar_arrive(&ring.full[slot]);
