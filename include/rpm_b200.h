@@ -358,6 +358,27 @@ int rpm_batch_lanczos_kind(const rpm_batch* batch, int* kind);
  * work_dev: rpm_he_eigh_workspace bytes.  Synchronises the stream. */
 int rpm_he_eigh_workspace(int n, int batch, long long* bytes);
 int rpm_he_eigh(int n, int batch, void* a_dev, double* w_dev, void* v_dev, void* work_dev, cudaStream_t stream);
+/* The two radicals' matrices in the same launches: `batch` of each size,
+ * symmetrised first (0.5 (A + A^H)); work_dev: the sum of both
+ * rpm_he_eigh_workspace sizes, 2 <= na, nb <= 1024, batch <= 32767. */
+int rpm_he_eigh_pair(int na, int nb, int batch, void* a_dev, void* b_dev, double* wa_dev, double* wb_dev, void* va_dev,
+                     void* vb_dev, void* work_dev, cudaStream_t stream);
+/* Lifetime sums from the eigensystems (replaces solve_orientation and
+ * convolved_correlation_spectrum, :172-240): for each of `batch` orientations
+ * the spin operators of both radicals, the nine binned transition spectra of
+ * each on a grid of spacing `delta` with half_a[b], half_b[b] bins either side
+ * of zero (host arrays), their convolution and
+ *   out_dev[b][0] = 1/4 + sum Re conv, out_dev[b][1 + t] = 1/4 + sum Re (conv k / (k - i w)),
+ * k = 1 / lifetimes[t] (host array, nlife >= 1).  lam: ascending eigenvalues,
+ * v: eigenvectors as columns (electron digit slowest, even da, db).
+ * *bad_dev is raised when a line falls outside its grid.  work_dev:
+ * rpm_factorized_workspace bytes.  Asynchronous on the stream. */
+int rpm_factorized_workspace(int da, int db, int batch, const long long* half_a, const long long* half_b, int nlife,
+                             long long* bytes);
+int rpm_factorized_yields(int da, int db, int batch, const double* lam_a_dev, const void* va_dev,
+                          const double* lam_b_dev, const void* vb_dev, double delta, const long long* half_a,
+                          const long long* half_b, const double* lifetimes, int nlife, double* out_dev, int* bad_dev,
+                          void* work_dev, cudaStream_t stream);
 /* C = A^H B for `batch` square complex128 matrices (row-major): the
  * eigenbasis spin operators of diagonalize_radical (:127-170). */
 int rpm_zgemm_hn(int n, int batch, const void* a_dev, const void* b_dev, void* c_dev, cudaStream_t stream);

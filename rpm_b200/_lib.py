@@ -107,6 +107,9 @@ SIGNATURES: dict[str, list] = {
     "rpm_bin_transition_lines": [_P, _P, _P, _I, _D, _D, _LL, _P, _P, _P],
     "rpm_he_eigh_workspace": [_I, _I, _P],
     "rpm_he_eigh": [_I, _I, _P, _P, _P, _P, _P],
+    "rpm_he_eigh_pair": [_I, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P],
+    "rpm_factorized_workspace": [_I, _I, _I, _P, _P, _I, _P],
+    "rpm_factorized_yields": [_I, _I, _I, _P, _P, _P, _P, _D, _P, _P, _P, _I, _P, _P, _P, _P],
     "rpm_zgemm_hn": [_I, _I, _P, _P, _P, _P],
     "rpm_fft_pow2": [_I, _I, _P, _P, _I, _P],
     "rpm_spectrum_mac": [_LL, _P, _P, _P, _P],

@@ -1,19 +1,19 @@
 // Kernels of the factorized exact oracle (rpm_quantum_needle_reproduction.py:
 // 93-240): batched Hermitian eigen-decompositions of the radical
 // Hamiltonians (FAD 576, TrpH 384 dimensions; one matrix per field
-// orientation), eigenbasis spin operators (complex products A^H B) and the
-// FFT convolution of the binned transition spectra.  All FP64.
+// orientation), complex products A^H B and FFTs.  All FP64.  The binned
+// spectra, their convolution and the lifetime sums are in factorized_yields.cu.
 //
-// Eigen-decomposition (one CTA per matrix):
+// Eigen-decomposition; both radicals' matrices share each launch:
 //   k_he_tridiag  Householder reduction Q^H A Q = T with a real symmetric
 //                 tridiagonal T (the reflectors of LAPACK's zlarfg / zhetd2,
 //                 lower form: H = I - tau v v^H, v[0] = 1, H^H [a; x] = [b; 0]
 //                 with b real), the full trailing matrix updated by the
-//                 Hermitian rank-2 update;
+//                 Hermitian rank-2 update; one CTA per matrix;
 //   k_he_tridiag_eig  implicit symmetric tridiagonal QR with Wilkinson shifts
-//                 (krylov.cuh tridiag_qr) with the eigenvectors of T;
-//   k_he_back     V = Q Z, the reflectors applied to Z in reverse order, 32
-//                 columns per CTA.
+//                 with the eigenvectors of T;
+//   k_he_back     V = Q Z, the reflectors applied to Z in reverse order, two
+//                 columns per warp.
 // Eigenvalues come out in QR order and are sorted ascending with their
 // vectors (k_he_sort), as LAPACK returns them.
 #include <algorithm>
@@ -21,7 +21,7 @@
 #include <vector>
 
 #include "common.cuh"
-#include "krylov.cuh"
+#include "ptx.cuh"
 
 namespace rpm {
 namespace {
@@ -56,22 +56,71 @@ __device__ double block_reduce_sum(double v, double* red) {
   return red[0];
 }
 
+// One size's share of a call; two radicals' matrices run in the same launches.
+struct HePart {
+  int n = 0;
+  double2 *a = nullptr, *v = nullptr, *tau = nullptr, *house = nullptr;
+  double *w = nullptr, *d = nullptr, *e = nullptr, *z = nullptr;
+  int *perm = nullptr, *status = nullptr;
+  int rows = 0;  // eigenvector rows per CTA of k_he_tridiag_eig
+};
+struct HePair {
+  HePart part[2];
+  int batch;
+  __device__ const HePart& of(int item, int* b) const {
+    const int second = item >= batch;
+    *b = item - (second ? batch : 0);
+    return part[second];
+  }
+};
+
+constexpr int kHeSmem = 200 * 1024;    // rows of eigenvectors
+constexpr int kHeMatSmem = 193 * 1024; // the matrix, beside 33 KB of vectors
+
+// 0.5 (A + A^H) in place.
+__global__ void __launch_bounds__(256) k_he_symmetrise(HePair p) {
+  int b;
+  const HePart& h = p.of(blockIdx.y, &b);
+  const int n = h.n;
+  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= (long long)n * n) return;
+  const int i = (int)(idx / n), j = (int)(idx - (long long)i * n);
+  if (i > j) return;
+  double2* a = h.a + (size_t)b * n * n;
+  const double2 x = a[(size_t)i * n + j], y = a[(size_t)j * n + i];
+  const double2 m = make_double2(0.5 * (x.x + y.x), 0.5 * (x.y - y.y));
+  a[(size_t)i * n + j] = m;
+  a[(size_t)j * n + i] = cconj(m);
+}
+
 // Householder reduction of matrix b: a (n x n, row-major, overwritten), d, e
 // (n, n - 1 real), house (n x n: row k holds v_k, v_k[j] for j > k, v_k[k+1]
-// = 1), tau (n - 1 complex).
-__global__ void __launch_bounds__(kHeThreads) k_he_tridiag(double2* a_all, int n, double* d_all, double* e_all,
-                                                          double2* house_all, double2* tau_all) {
+// = 1), tau (n - 1 complex).  Bound by the barriers and latencies of its n - 1
+// serial steps.  A matrix that fits is worked on in shared memory (n <= 111),
+// and rows go to warps, without a division per element: 6 x 72 and 6 x 48 took
+// 313 + 172 us from global memory, one size after the other; now 290 us together
+// (512 threads 275, but 288 x 288 8.7 ms against 6.4; 256 threads 330).
+__global__ void __launch_bounds__(kHeThreads) k_he_tridiag(HePair p) {
   __shared__ double2 v[kHeMaxN], w[kHeMaxN];
   __shared__ double red[32];
   __shared__ double2 s_tau;
   __shared__ double s_beta;
+  extern __shared__ double2 he_smem[];
+  int b;
+  const HePart& h = p.of(blockIdx.x, &b);
+  const int n = h.n;
   const size_t nn = (size_t)n * n;
-  double2* a = a_all + blockIdx.x * nn;
-  double* d = d_all + (size_t)blockIdx.x * n;
-  double* e = e_all + (size_t)blockIdx.x * n;
-  double2* house = house_all + blockIdx.x * nn;
-  double2* tau = tau_all + (size_t)blockIdx.x * n;
+  double2* a = h.a + b * nn;
+  double* d = h.d + (size_t)b * n;
+  double* e = h.e + (size_t)b * n;
+  double2* house = h.house + b * nn;
+  double2* tau = h.tau + (size_t)b * n;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if (nn * sizeof(double2) <= kHeMatSmem) {
+    for (int k = threadIdx.x; k < (int)nn; k += blockDim.x) he_smem[k] = a[k];
+    a = he_smem;
+    __syncthreads();
+  }
   for (int k = 0; k + 1 < n; ++k) {
     const int m = n - k - 1;  // trailing size
     // x = A[k+1:, k] = conj(A[k, k+1:]) (A Hermitian, full storage)
@@ -100,7 +149,6 @@ __global__ void __launch_bounds__(kHeThreads) k_he_tridiag(double2* a_all, int n
     const double2 t = s_tau;
     const bool reflect = t.x != 0.0 || t.y != 0.0;
     const double2 scale = w[0];
-    __syncthreads();
     for (int j = threadIdx.x; j < m; j += blockDim.x) {
       double2 vj = make_double2(1.0, 0.0);
       if (j > 0) vj = reflect ? cmul(cconj(a[(size_t)k * n + k + 1 + j]), scale) : make_double2(0.0, 0.0);
@@ -119,37 +167,40 @@ __global__ void __launch_bounds__(kHeThreads) k_he_tridiag(double2* a_all, int n
         const double2* row = a + (size_t)(k + 1 + i) * n + k + 1;
         double sx = 0.0, sy = 0.0;
         for (int j = lane; j < m; j += 32) {
-          const double2 p = cmul(row[j], v[j]);
-          sx += p.x;
-          sy += p.y;
+          const double2 q = cmul(row[j], v[j]);
+          sx += q.x;
+          sy += q.y;
         }
         sx = warp_reduce(sx);
         sy = warp_reduce(sy);
         if (lane == 0) w[i] = cmul(t, make_double2(sx, sy));
       }
       __syncthreads();
-      // alpha = -1/2 tau (w^H v); w += alpha v
-      double px = 0.0, py = 0.0;
-      for (int j = threadIdx.x; j < m; j += blockDim.x) {
-        const double2 p = cmul(cconj(w[j]), v[j]);
-        px += p.x;
-        py += p.y;
+      // alpha = -1/2 tau (w^H v), by every warp for itself; w += alpha v
+      double wx = 0.0, wy = 0.0;
+      for (int j = lane; j < m; j += 32) {
+        const double2 q = cmul(cconj(w[j]), v[j]);
+        wx += q.x;
+        wy += q.y;
       }
-      const double wx = block_reduce_sum(px, red);
-      const double wy = block_reduce_sum(py, red);
+      wx = warp_reduce(wx);
+      wy = warp_reduce(wy);
       const double2 al = cmul(make_double2(-0.5 * t.x, -0.5 * t.y), make_double2(wx, wy));
+      __syncthreads();
       for (int j = threadIdx.x; j < m; j += blockDim.x) {
-        const double2 p = cmul(al, v[j]);
-        w[j] = make_double2(w[j].x + p.x, w[j].y + p.y);
+        const double2 q = cmul(al, v[j]);
+        w[j] = make_double2(w[j].x + q.x, w[j].y + q.y);
       }
       __syncthreads();
       // A22 -= v w^H + w v^H (full storage)
-      for (size_t idx = threadIdx.x; idx < (size_t)m * m; idx += blockDim.x) {
-        const int i = (int)(idx / m), j = (int)(idx - (size_t)i * m);
-        const double2 p = cmul(v[i], cconj(w[j]));
-        const double2 q = cmul(w[i], cconj(v[j]));
-        double2& x = a[(size_t)(k + 1 + i) * n + k + 1 + j];
-        x = make_double2(x.x - p.x - q.x, x.y - p.y - q.y);
+      for (int i = warp; i < m; i += nw) {
+        double2* row = a + (size_t)(k + 1 + i) * n + k + 1;
+        const double2 vi = v[i], wi = w[i];
+        for (int j = lane; j < m; j += 32) {
+          const double2 q = cmul(vi, cconj(w[j])), u = cmul(wi, cconj(v[j]));
+          const double2 x = row[j];
+          row[j] = make_double2(x.x - q.x - u.x, x.y - q.y - u.y);
+        }
       }
       __syncthreads();
     }
@@ -157,32 +208,231 @@ __global__ void __launch_bounds__(kHeThreads) k_he_tridiag(double2* a_all, int n
   if (threadIdx.x == 0) d[n - 1] = a[(size_t)(n - 1) * n + n - 1].x;
 }
 
-// Eigenvalues and eigenvectors of the tridiagonal T of matrix b: z (n x n,
-// row i = component i), eigenvalues into d (QR order), status[b] = 0 on
-// convergence.
-__global__ void __launch_bounds__(256) k_he_tridiag_eig(double* d_all, double* e_all, double* z_all, int n,
-                                                       int* status) {
-  __shared__ double ds[kHeMaxN], es[kHeMaxN];
-  __shared__ double2 rot[kHeMaxN];
-  double* d = d_all + (size_t)blockIdx.x * n;
-  const double* e = e_all + (size_t)blockIdx.x * n;
-  double* z = z_all + (size_t)blockIdx.x * n * n;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    ds[i] = d[i];
+// Eigenvalues and eigenvectors of the tridiagonal T of matrix b (implicit
+// symmetric QR with Wilkinson shifts, Golub & Van Loan, section 8.3): z (n x n,
+// row i = component i), eigenvalues into d (QR order), status[b] raised when it
+// does not converge.
+//
+// Bound by the serial chase of the bulge (n^2 rotations or so, each a chain of
+// dependent FP64 operations).  Warp 0 chases and does nothing else: it leaves
+// the rotations, 64 at a time, in a ring of slots that row warps work off, one
+// eigenvector-matrix row per lane in shared memory, by columns.  Where the rows
+// of a matrix do not fit, several CTAs each take a part of them and repeat the
+// same chase.  A rotation takes no branch and loads the next one's operands
+// before it stores: 275 cycles with the sweep's share of deflation and shift,
+// 490 with its first and last iteration and its fallback treated apart.
+// 6 x 72 and 6 x 48 dimensions, one size after the other with the rows in
+// global memory behind each sweep: 3,600 + 1,560 us; now 770 us together.
+// 192, 288, 384 dimensions: 30, 87, 170 -> 5.2, 10.3, 18 ms.
+constexpr int kEigSlots = 8, kEigChunk = 64, kEigPad = 5;
+constexpr int kEigFirst = 1, kEigLast = 2, kEigEnd = 4;
+struct EigRing {
+  double2 rot[kEigSlots][kEigChunk];
+  int k0[kEigSlots], count[kEigSlots], flags[kEigSlots];
+  unsigned long long full[kEigSlots], empty[kEigSlots];
+};
+
+// d, e: one entry of padding before e and two behind each
+__device__ __forceinline__ void eig_chase(int n, double* d, double* e, EigRing& ring, int* status) {
+  const int lane = threadIdx.x & 31;
+  unsigned it = 0;  // slots filled (lane 0)
+  int hi = n - 1;   // off-diagonal entries from hi on are zero
+  auto slot_free = [&] {
+    return it < kEigSlots || ptx::mbar_wait(&ring.empty[it % kEigSlots], (it / kEigSlots - 1) & 1u, status);
+  };
+  for (int sweeps = 0;; ++sweeps) {
+    // deflation, from the top: the last unreduced block is [p, q]
+    int q = 0, p = 0;
+    for (int base = (hi - 1) & ~31; base >= 0; base -= 32) {
+      const int i = base + lane;
+      bool nz = false;
+      if (i < hi) {
+        const double ei = e[i];
+        if (fabs(ei) <= DBL_EPSILON * (fabs(d[i]) + fabs(d[i + 1])) || fabs(ei) < DBL_MIN) e[i] = 0.0;
+        else nz = true;
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, nz);
+      unsigned zero = ~m;
+      if (q == 0) {
+        if (!m) continue;
+        const int top = 31 - __clz(m);
+        q = base + top + 1;
+        zero &= (1u << top) - 1u;
+      }
+      if (zero) {
+        p = base + 32 - __clz(zero);
+        break;
+      }
+    }
+    __syncwarp();
+    hi = q;
+    int ok = 1;
+    if (q == 0 || sweeps >= 40 * n) {
+      if (lane == 0) {
+        if (q != 0) atomicExch(status, 1);
+        slot_free();
+        ring.flags[it % kEigSlots] = kEigEnd;
+        ptx::mbar_arrive(&ring.full[it % kEigSlots]);
+      }
+      return;
+    }
+    if (lane == 0) {
+      const double delta = 0.5 * (d[q - 1] - d[q]);
+      const double eq = e[q - 1];
+      const double mu = d[q] - eq * eq / (delta + copysign(hypot(delta, eq), delta));
+      double a = d[p], bb = e[p];  // d[k] and e[k] as the previous rotation left them
+      double x = a - mu, y = bb;
+      double cc = d[p + 1], en = e[p + 1];  // e[q] = 0, the padding behind it is never used
+      for (int k0 = p; k0 < q; k0 += kEigChunk) {
+        ok = slot_free() ? 1 : 0;
+        if (!ok) break;
+        const int slot = it % kEigSlots, k1 = min(q, k0 + kEigChunk);
+        double2* rot = ring.rot[slot];
+        for (int k = k0; k < k1; ++k) {
+          // the next rotation's operands, ahead of this one's stores
+          const double cn = d[k + 2], en2 = e[k + 2];
+          // [d_k e_k; e_k d_k+1] turned by (c, s) = (x, y) / r: the sums over x
+          // and y are formed beside 1 / r, not behind c and s
+          const double xx = x * x, yy = y * y, xy = x * y;
+          const double rr = xx + yy;
+          const double nk = fma(xx, a, fma(2.0 * xy, bb, yy * cc));
+          const double nk1 = fma(yy, a, fma(-2.0 * xy, bb, xx * cc));
+          const double ne = fma(xy, cc - a, (xx - yy) * bb);
+          const double inv = rsqrt(rr), inv2 = inv * inv;
+          double ek = ne * inv2, dk1 = nk1 * inv2, dk = nk * inv2, c = x * inv, sn = y * inv, r = rr * inv;
+          if (__builtin_expect(!(rr > 1e-150 && rr < 1e150), 0)) {
+            r = hypot(x, y);
+            c = r > 0.0 ? x / r : 1.0;
+            sn = r > 0.0 ? y / r : 0.0;
+            ek = c * sn * (cc - a) + (c * c - sn * sn) * bb;
+            dk1 = sn * sn * a - 2.0 * c * sn * bb + c * c * cc;
+            dk = c * c * a + 2.0 * c * sn * bb + sn * sn * cc;
+          }
+          x = ek;
+          y = sn * en;
+          bb = c * en;
+          a = dk1;
+          e[k - 1] = r;  // e[p - 1]: put back below
+          d[k] = dk;
+          e[k + 1] = bb;
+          rot[k - k0] = make_double2(c, sn);
+          cc = cn;
+          en = en2;
+        }
+        ring.k0[slot] = k0;
+        ring.count[slot] = k1 - k0;
+        ring.flags[slot] = (k0 == p ? kEigFirst : 0) | (k1 == q ? kEigLast : 0);
+        ptx::mbar_arrive(&ring.full[slot]);
+        ++it;
+      }
+      d[q] = a;
+      e[q - 1] = x;
+      e[p - 1] = 0.0;
+    }
+    __syncwarp();
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+    if (!ok) return;  // status is raised: the row warps' waits end on it
+  }
+}
+
+// One row per lane (row < 0: none); z[k * ld + row].
+__device__ __forceinline__ void eig_rows(double* z, int ld, int row, EigRing& ring, int* status) {
+  const int lane = threadIdx.x & 31;
+  double zk = 0.0;
+  for (unsigned it = 0;; ++it) {
+    const int slot = it % kEigSlots;
+    int ok = 1;
+    if (lane == 0) ok = ptx::mbar_wait(&ring.full[slot], (it / kEigSlots) & 1u, status) ? 1 : 0;
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+    if (!ok) return;
+    const int flags = ring.flags[slot];
+    if (flags & kEigEnd) return;
+    if (row >= 0) {
+      const int count = ring.count[slot];
+      const double2* rot = ring.rot[slot];
+      double* zr = z + row + (size_t)ring.k0[slot] * ld;
+      if (flags & kEigFirst) zk = zr[0];
+      int k = 0;
+      for (; k + 4 <= count; k += 4) {  // four rotations' operands ahead of their use
+        double2 cs[4];
+        double zn[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          cs[u] = rot[k + u];
+          zn[u] = zr[(k + u + 1) * ld];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          zr[(k + u) * ld] = cs[u].x * zk + cs[u].y * zn[u];
+          zk = -cs[u].y * zk + cs[u].x * zn[u];
+        }
+      }
+      for (; k < count; ++k) {
+        const double2 cs = rot[k];
+        const double zn = zr[(k + 1) * ld];
+        zr[k * ld] = cs.x * zk + cs.y * zn;
+        zk = -cs.y * zk + cs.x * zn;
+      }
+      if (flags & kEigLast) zr[count * ld] = zk;
+    }
+    __syncwarp();
+    if (lane == 0) ptx::mbar_arrive(&ring.empty[slot]);
+  }
+}
+
+__global__ void __launch_bounds__(1024) k_he_tridiag_eig(HePair p) {
+  __shared__ EigRing ring;
+  extern __shared__ double eig_smem[];
+  int b;
+  const HePart& h = p.of(blockIdx.y, &b);
+  const int n = h.n, ld = h.rows, row0 = blockIdx.x * ld;
+  if (row0 >= n) return;
+  const int rows = min(ld, n - row0);
+  double* ds = eig_smem;
+  double* es = ds + n + 3;  // es[-1] .. es[n + 1], ds[0] .. ds[n + 1]
+  double* z = es + n + 2;
+  double* d = h.d + (size_t)b * n;
+  const double* e = h.e + (size_t)b * n;
+  int* status = h.status + b;
+  const int row_warps = (rows + 31) / 32, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < n + 2; i += blockDim.x) {
+    ds[i] = i < n ? d[i] : 0.0;
     es[i] = i + 1 < n ? e[i] : 0.0;
   }
+  for (int k = threadIdx.x; k < n * ld; k += blockDim.x) z[k] = k / ld == row0 + k % ld ? 1.0 : 0.0;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kEigSlots; ++s) {
+      ptx::mbar_init(&ring.full[s], 1);
+      ptx::mbar_init(&ring.empty[s], row_warps);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
   __syncthreads();
-  const int bad = tridiag_qr(n, ds, es, z, n, rot);
-  for (int i = threadIdx.x; i < n; i += blockDim.x) d[i] = ds[i];
-  if (threadIdx.x == 0) status[blockIdx.x] = bad;
+  if (warp == 0) {
+    eig_chase(n, ds, es, ring, status);
+  } else if (warp <= row_warps) {
+    const int row = (warp - 1) * 32 + (threadIdx.x & 31);
+    eig_rows(z, ld, row < rows ? row : -1, ring, status);
+  }
+  __syncthreads();
+  double* zo = h.z + (size_t)b * n * n + (size_t)row0 * n;
+  for (int k = threadIdx.x; k < rows * n; k += blockDim.x) zo[k] = z[(k % n) * ld + k / n];
+  // d is read by every CTA of the matrix: the values go out through w
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < n; i += blockDim.x) h.w[(size_t)b * n + i] = ds[i];
 }
 
 // Ascending order of the eigenvalues: perm[r] = index of the r-th smallest
-// (ties by index), sorted values into w.
-__global__ void __launch_bounds__(256) k_he_sort(const double* d_all, int n, int* perm_all, double* w_all) {
-  const double* d = d_all + (size_t)blockIdx.x * n;
-  int* perm = perm_all + (size_t)blockIdx.x * n;
-  double* w = w_all + (size_t)blockIdx.x * n;
+// (ties by index), sorted values into w (which holds them in QR order).
+__global__ void __launch_bounds__(256) k_he_sort(HePair p) {
+  __shared__ double d[kHeMaxN];
+  int b;
+  const HePart& h = p.of(blockIdx.x, &b);
+  const int n = h.n;
+  int* perm = h.perm + (size_t)b * n;
+  double* w = h.w + (size_t)b * n;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) d[i] = w[i];
+  __syncthreads();
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const double x = d[i];
     int r = 0;
@@ -195,49 +445,58 @@ __global__ void __launch_bounds__(256) k_he_sort(const double* d_all, int n, int
   }
 }
 
-// V = Q Z[:, perm]: 32 output columns per CTA (lanes), 8 row groups (warps);
-// the reflectors H_k = I - tau_k v_k v_k^H applied for k = n-2 .. 0.
-__global__ void __launch_bounds__(256) k_he_back(const double* z_all, const int* perm_all, const double2* house_all,
-                                                const double2* tau_all, int n, double2* v_all) {
-  __shared__ double2 part[8][32];
+// V = Q Z[:, perm]: the reflectors H_k = I - tau_k v_k v_k^H applied for
+// k = n-2 .. 0, two columns per warp in shared memory, so that a step's sum
+// needs no block barrier: 125 + 62 us for 6 x 72 and 6 x 48 dimensions with
+// eight warps per column, now 78 us together.
+constexpr int kBackWarps = 4, kBackCols = 2;
+__global__ void __launch_bounds__(32 * kBackWarps) k_he_back(HePair p) {
+  extern __shared__ double2 he_smem[];
+  int b;
+  const HePart& h = p.of(blockIdx.y, &b);
+  const int n = h.n;
   const size_t nn = (size_t)n * n;
-  const int b = blockIdx.y;
-  const double* z = z_all + b * nn;
-  const int* perm = perm_all + (size_t)b * n;
-  const double2* house = house_all + b * nn;
-  const double2* tau = tau_all + (size_t)b * n;
-  double2* v = v_all + b * nn;
-  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
-  const int c = blockIdx.x * 32 + lane;
-  const bool col = c < n;
-  const int src = col ? perm[c] : 0;
-  for (int i = g; i < n; i += 8)
-    if (col) v[(size_t)i * n + c] = make_double2(z[(size_t)i * n + src], 0.0);
-  __syncthreads();
+  const double* z = h.z + b * nn;
+  const int* perm = h.perm + (size_t)b * n;
+  const double2* house = h.house + b * nn;
+  const double2* tau = h.tau + (size_t)b * n;
+  double2* v = h.v + b * nn;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c0 = (blockIdx.x * kBackWarps + warp) * kBackCols;
+  if (c0 >= n) return;
+  const int nc = min(kBackCols, n - c0);
+  double2* x0 = he_smem + (size_t)warp * kBackCols * n;
+  double2* x1 = x0 + n;
+  const int s0 = perm[c0], s1 = perm[c0 + nc - 1];  // nc = 1: the same column twice
+  for (int i = lane; i < n; i += 32) {
+    x0[i] = make_double2(z[(size_t)i * n + s0], 0.0);
+    x1[i] = make_double2(z[(size_t)i * n + s1], 0.0);
+  }
   for (int k = n - 2; k >= 0; --k) {
     const double2 t = tau[k];
-    if (t.x == 0.0 && t.y == 0.0) continue;  // uniform: H_k = I
+    if (t.x == 0.0 && t.y == 0.0) continue;  // H_k = I
     const double2* hv = house + (size_t)k * n;
-    double2 s = make_double2(0.0, 0.0);
-    if (col)
-      for (int i = k + 1 + g; i < n; i += 8) {
-        const double2 p = cmul(cconj(hv[i]), v[(size_t)i * n + c]);
-        s.x += p.x;
-        s.y += p.y;
-      }
-    part[g][lane] = s;
-    __syncthreads();
-    double2 tot = make_double2(0.0, 0.0);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) tot = make_double2(tot.x + part[q][lane].x, tot.y + part[q][lane].y);
-    const double2 ts = cmul(t, tot);
-    if (col)
-      for (int i = k + 1 + g; i < n; i += 8) {
-        const double2 p = cmul(hv[i], ts);
-        double2& x = v[(size_t)i * n + c];
-        x = make_double2(x.x - p.x, x.y - p.y);
-      }
-    __syncthreads();
+    double2 a0 = make_double2(0.0, 0.0), a1 = a0;
+    __syncwarp();
+    for (int i = k + 1 + lane; i < n; i += 32) {
+      const double2 u = cconj(hv[i]);
+      const double2 p0 = cmul(u, x0[i]), p1 = cmul(u, x1[i]);
+      a0 = make_double2(a0.x + p0.x, a0.y + p0.y);
+      a1 = make_double2(a1.x + p1.x, a1.y + p1.y);
+    }
+    a0 = cmul(t, make_double2(warp_reduce(a0.x), warp_reduce(a0.y)));
+    a1 = cmul(t, make_double2(warp_reduce(a1.x), warp_reduce(a1.y)));
+    for (int i = k + 1 + lane; i < n; i += 32) {
+      const double2 u = hv[i];
+      const double2 p0 = cmul(u, a0), p1 = cmul(u, a1);
+      x0[i] = make_double2(x0[i].x - p0.x, x0[i].y - p0.y);
+      x1[i] = make_double2(x1[i].x - p1.x, x1[i].y - p1.y);
+    }
+  }
+  __syncwarp();
+  for (int i = lane; i < n; i += 32) {
+    v[(size_t)i * n + c0] = x0[i];
+    if (nc == 2) v[(size_t)i * n + c0 + 1] = x1[i];
   }
 }
 
@@ -306,6 +565,76 @@ __global__ void k_fft_mac(double2* acc, const double2* x, const double2* y, long
 
 int grid_for(long long work) { return (int)std::max(1LL, std::min((work + 255) / 256, 65535LL * 4)); }
 
+template <class K>
+void set_smem(K kern, size_t bytes) {
+  check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "eigh shared memory");
+}
+
+long long eigh_bytes(int n, int batch) {
+  const long long nn = (long long)n * n;
+  // d, e, perm (as double), tau (2 doubles), status; house (complex) and z (real)
+  return (long long)batch * ((3 * n + 2 * n + 1) * 8 + nn * 16 + nn * 8) + 7 * 256;  // + alignment of 7 parts
+}
+
+char* eigh_part(HePart& h, int n, int batch, void* a, double* w, void* v, char* p) {
+  const long long nn = (long long)n * n;
+  auto take = [&](long long bytes) {
+    char* q = p;
+    p += (bytes + 255) / 256 * 256;
+    return q;
+  };
+  h.n = n;
+  h.a = static_cast<double2*>(a);
+  h.w = w;
+  h.v = static_cast<double2*>(v);
+  h.d = reinterpret_cast<double*>(take((long long)batch * n * 8));
+  h.e = reinterpret_cast<double*>(take((long long)batch * n * 8));
+  h.perm = reinterpret_cast<int*>(take((long long)batch * n * 8));
+  h.tau = reinterpret_cast<double2*>(take((long long)batch * n * 16));
+  h.status = reinterpret_cast<int*>(take((long long)batch * 8));
+  h.house = reinterpret_cast<double2*>(take((long long)batch * nn * 16));
+  h.z = reinterpret_cast<double*>(take((long long)batch * nn * 8));
+  // as many rows per CTA as fit beside d and e (n = 1024: 23)
+  h.rows = std::min({n, 31 * 32, (kHeSmem / 8 - 2 * n - kEigPad) / n});
+  return p;
+}
+
+// `parts` sizes of `batch` matrices each.
+void eigh_run(HePair& p, int parts, bool symmetrise, cudaStream_t stream) {
+  int nmax = 0, row_blocks = 1, row_threads = 0;
+  size_t eig_smem = 0, red_smem = 0;
+  for (int k = 0; k < parts; ++k) {
+    const HePart& h = p.part[k];
+    nmax = std::max(nmax, h.n);
+    row_blocks = std::max(row_blocks, (h.n + h.rows - 1) / h.rows);
+    row_threads = std::max(row_threads, (h.rows + 31) / 32 * 32);
+    eig_smem = std::max(eig_smem, sizeof(double) * (size_t)(2 * h.n + kEigPad + h.n * h.rows));
+    const size_t mat = sizeof(double2) * (size_t)h.n * h.n;
+    if (mat <= (size_t)kHeMatSmem) red_smem = std::max(red_smem, mat);
+    check_cuda(cudaMemsetAsync(h.status, 0, sizeof(int) * p.batch, stream), "eigh status");
+  }
+  const int items = p.batch * parts;
+  if (symmetrise)
+    k_he_symmetrise<<<dim3((unsigned)(((long long)nmax * nmax + 255) / 256), items), 256, 0, stream>>>(p);
+  const size_t back_smem = sizeof(double2) * (size_t)kBackWarps * kBackCols * nmax;
+  set_smem(k_he_tridiag, red_smem);
+  set_smem(k_he_tridiag_eig, eig_smem);
+  set_smem(k_he_back, back_smem);
+  k_he_tridiag<<<items, kHeThreads, red_smem, stream>>>(p);
+  k_he_tridiag_eig<<<dim3(row_blocks, items), 32 + row_threads, eig_smem, stream>>>(p);
+  k_he_sort<<<items, 256, 0, stream>>>(p);
+  const int per = kBackWarps * kBackCols;
+  k_he_back<<<dim3((nmax + per - 1) / per, items), 32 * kBackWarps, back_smem, stream>>>(p);
+  check_launch("eigh");
+  std::vector<int> st((size_t)items);
+  for (int k = 0; k < parts; ++k)
+    check_cuda(cudaMemcpyAsync(st.data() + (size_t)k * p.batch, p.part[k].status, sizeof(int) * p.batch,
+                               cudaMemcpyDeviceToHost, stream), "eigh status");
+  check_cuda(cudaStreamSynchronize(stream), "eigh sync");
+  for (int s : st)
+    if (s) fail(RPM_E_NUMERIC, "eigh: the tridiagonal QR did not converge");
+}
+
 }  // namespace
 }  // namespace rpm
 
@@ -316,9 +645,7 @@ extern "C" {
 int rpm_he_eigh_workspace(int n, int batch, long long* bytes) {
   return guarded([&] {
     if (n < 2 || n > kHeMaxN || batch < 1 || !bytes) fail(RPM_E_INVALID, "eigh: need 2 <= n <= 1024, batch >= 1");
-    const long long nn = (long long)n * n;
-    // d, e, perm (as double), tau (2 doubles), status; house (complex) and z (real)
-    *bytes = (long long)batch * ((3 * n + 2 * n + 1) * 8 + nn * 16 + nn * 8) + 7 * 256;  // + alignment of 7 parts
+    *bytes = eigh_bytes(n, batch);
   });
 }
 
@@ -327,31 +654,27 @@ int rpm_he_eigh(int n, int batch, void* a_dev, double* w_dev, void* v_dev, void*
     long long need = 0;
     if (rpm_he_eigh_workspace(n, batch, &need) != RPM_OK) fail(RPM_E_INVALID, "eigh: bad sizes");
     if (!a_dev || !w_dev || !v_dev || !work_dev) fail(RPM_E_INVALID, "eigh: null pointer");
-    const long long nn = (long long)n * n;
-    char* p = static_cast<char*>(work_dev);
-    auto take = [&](long long bytes) {
-      char* q = p;
-      p += (bytes + 255) / 256 * 256;
-      return q;
-    };
-    double* d = reinterpret_cast<double*>(take((long long)batch * n * 8));
-    double* e = reinterpret_cast<double*>(take((long long)batch * n * 8));
-    int* perm = reinterpret_cast<int*>(take((long long)batch * n * 8));
-    double2* tau = reinterpret_cast<double2*>(take((long long)batch * n * 16));
-    int* status = reinterpret_cast<int*>(take((long long)batch * 8));
-    double2* house = reinterpret_cast<double2*>(take((long long)batch * nn * 16));
-    double* z = reinterpret_cast<double*>(take((long long)batch * nn * 8));
-    (void)need;
-    k_he_tridiag<<<batch, kHeThreads, 0, stream>>>(static_cast<double2*>(a_dev), n, d, e, house, tau);
-    k_he_tridiag_eig<<<batch, 256, 0, stream>>>(d, e, z, n, status);
-    k_he_sort<<<batch, 256, 0, stream>>>(d, n, perm, w_dev);
-    k_he_back<<<dim3((n + 31) / 32, batch), 256, 0, stream>>>(z, perm, house, tau, n, static_cast<double2*>(v_dev));
-    check_launch("eigh");
-    std::vector<int> st(batch);
-    check_cuda(cudaMemcpyAsync(st.data(), status, sizeof(int) * batch, cudaMemcpyDeviceToHost, stream), "eigh status");
-    check_cuda(cudaStreamSynchronize(stream), "eigh sync");
-    for (int b = 0; b < batch; ++b)
-      if (st[b]) fail(RPM_E_NUMERIC, "eigh: the tridiagonal QR did not converge");
+    HePair p;
+    p.batch = batch;
+    eigh_part(p.part[0], n, batch, a_dev, w_dev, v_dev, static_cast<char*>(work_dev));
+    eigh_run(p, 1, false, stream);
+  });
+}
+
+int rpm_he_eigh_pair(int na, int nb, int batch, void* a_dev, void* b_dev, double* wa_dev, double* wb_dev, void* va_dev,
+                     void* vb_dev, void* work_dev, cudaStream_t stream) {
+  return guarded([&] {
+    long long need = 0;
+    if (rpm_he_eigh_workspace(na, batch, &need) != RPM_OK || rpm_he_eigh_workspace(nb, batch, &need) != RPM_OK ||
+        batch > 32767)
+      fail(RPM_E_INVALID, "eigh: bad sizes");
+    if (!a_dev || !b_dev || !wa_dev || !wb_dev || !va_dev || !vb_dev || !work_dev)
+      fail(RPM_E_INVALID, "eigh: null pointer");
+    HePair p;
+    p.batch = batch;
+    char* rest = eigh_part(p.part[0], na, batch, a_dev, wa_dev, va_dev, static_cast<char*>(work_dev));
+    eigh_part(p.part[1], nb, batch, b_dev, wb_dev, vb_dev, rest);
+    eigh_run(p, 2, true, stream);
   });
 }
 

@@ -15,14 +15,13 @@ two spectra are convolved by FFT, and the kernel k / (k - i w) is summed over
 the convolved grid.
 
 GPU work, all in the library's own FP64 kernels: the radical blocks come
-from the library's split tables; their eigen-decompositions are batched over
-the field orientations (``rpm_he_eigh``: Householder tridiagonalisation,
-implicit tridiagonal QR, back-transformation, one CTA per matrix); the spin
-operators are rotated into the eigenbases by ``rpm_zgemm_hn`` (V^H (S (x) 1)
-V); the lines are binned by ``rpm_bin_transition_lines``; the two spectra
-are convolved by radix-2 FFTs (``rpm_fft_pow2``, zero-padded to a power of two
-no shorter than the linear convolution, which leaves the convolution itself
-unchanged).
+from the library's split tables; both radicals' eigen-decompositions run
+batched over the field orientations (``rpm_he_eigh_pair``: Householder
+tridiagonalisation, implicit tridiagonal QR, back-transformation); the spin
+operators in the eigenbases, the binned lines of all nine (p, q), their FFT
+convolution (zero-padded to a power of two no shorter than the linear
+convolution, which leaves the convolution itself unchanged) and the lifetime
+sums are ``rpm_factorized_yields``, all orientations in the same launches.
 """
 
 from __future__ import annotations
@@ -36,9 +35,8 @@ import numpy as np
 from . import _lib
 from .engine import _torch
 
-_SPIN_HALF = (np.array([[0.0, 0.5], [0.5, 0.0]], dtype=complex),
-              np.array([[0.0, -0.5j], [0.5j, 0.0]], dtype=complex),
-              np.array([[0.5, 0.0], [0.0, -0.5]], dtype=complex))
+# bytes of workspace per call; more orientations go in several calls
+_WORKSPACE_BYTES = 2_000_000_000
 
 
 def radical_blocks(hamiltonian) -> tuple[np.ndarray, np.ndarray]:
@@ -63,7 +61,7 @@ def hermitian_eigh(blocks):
         vec.fill_(1.0)
         return lam, vec
     # chunks: at most 65535 matrices (grid limit) and about 2 GB of workspace
-    chunk = int(max(1, min(65535, 2_000_000_000 // (48 * n * n + 64 * n))))
+    chunk = int(max(1, min(65535, _WORKSPACE_BYTES // (48 * n * n + 64 * n))))
     for b0 in range(0, batch, chunk):
         nb = min(chunk, batch - b0)
         size = ctypes.c_longlong()
@@ -74,31 +72,35 @@ def hermitian_eigh(blocks):
     return lam, vec
 
 
-class _Spectrum:
-    """Eigenvalues of one radical block and its electron spin operators in the
-    eigenbasis, <i| S_p (x) 1 |j>."""
+def _eigh_pair(blocks_a, blocks_b):
+    """Eigensystems of both radicals (device tensors) of equally many
+    orientations, in the same launches; inputs Hermitian-symmetrised."""
+    torch = _torch()
+    out = []
+    for blocks in (blocks_a, blocks_b):
+        out.append(torch.empty(blocks.shape[:2], dtype=torch.float64, device="cuda"))
+        out.append(torch.empty_like(blocks))
+    (lam_a, vec_a, lam_b, vec_b), (na, nb) = out, (blocks_a.shape[-1], blocks_b.shape[-1])
+    batch = blocks_a.shape[0]
+    chunk = int(max(1, min(32767, _WORKSPACE_BYTES // (48 * (na * na + nb * nb) + 64 * (na + nb)))))
+    for k in range(0, batch, chunk):
+        s = slice(k, min(k + chunk, batch))
+        count = s.stop - k
+        size, total = ctypes.c_longlong(), 0
+        for n in (na, nb):
+            _lib.call("rpm_he_eigh_workspace", n, count, ctypes.byref(size))
+            total += size.value
+        work = torch.empty(total, dtype=torch.uint8, device="cuda")
+        _lib.call("rpm_he_eigh_pair", na, nb, count, _lib.ptr(blocks_a[s]), _lib.ptr(blocks_b[s]), _lib.ptr(lam_a[s]),
+                  _lib.ptr(lam_b[s]), _lib.ptr(vec_a[s]), _lib.ptr(vec_b[s]), _lib.ptr(work), _lib.stream_handle())
+    return lam_a, vec_a, lam_b, vec_b
 
-    def __init__(self, torch, lam, vec):
-        d = vec.shape[0]
-        self.lam = lam
-        self.d = d
-        self.nuclear = d // 2
-        v3 = vec.reshape(2, self.nuclear, d)
-        self.ops = []
-        for s in _SPIN_HALF:
-            # (S (x) 1) V: rows of electron e are s[e, 0] V_0 + s[e, 1] V_1
-            w = torch.cat([complex(s[e, 0]) * v3[0] + complex(s[e, 1]) * v3[1] for e in (0, 1)]).contiguous()
-            op = torch.empty_like(w)
-            _lib.call("rpm_zgemm_hn", d, 1, _lib.ptr(vec), _lib.ptr(w), _lib.ptr(op), _lib.stream_handle())
-            self.ops.append(op)
-        self.max_gap = float((self.lam.max() - self.lam.min()).item())
 
-
-def _binned(torch, spec: _Spectrum, p: int, q: int, delta: float, half: int, bad):
-    grid = torch.zeros(2 * half + 1, dtype=torch.complex128, device="cuda")
-    _lib.call("rpm_bin_transition_lines", _lib.ptr(spec.lam), _lib.ptr(spec.ops[p]), _lib.ptr(spec.ops[q]), spec.d,
-              1.0 / spec.nuclear, float(delta), int(half), _lib.ptr(grid), _lib.ptr(bad), _lib.stream_handle())
-    return grid
+def _half_widths(lam: np.ndarray, delta: float) -> np.ndarray:
+    """Bins either side of zero that hold every line of each orientation."""
+    margin = 3
+    return np.array([int(math.ceil(float(gap) / delta)) + margin for gap in lam.max(axis=1) - lam.min(axis=1)],
+                    dtype=np.int64)
 
 
 def factorized_singlet_yields(hamiltonians: Sequence, lifetimes_us: Iterable[float], *,
@@ -117,43 +119,33 @@ def factorized_singlet_yields(hamiltonians: Sequence, lifetimes_us: Iterable[flo
     if bins_per_linewidth < 2.0:
         raise ValueError("bins_per_linewidth must be at least 2.")
     delta = (1.0 / max(lifetimes)) / float(bins_per_linewidth)
-    yields = np.empty((len(hamiltonians), len(lifetimes)))
-    initial = np.empty(len(hamiltonians))
-    bad = torch.zeros(1, dtype=torch.int32, device="cuda")
     blocks = [radical_blocks(h) for h in hamiltonians]
-    # one batched eigen-decomposition per radical over all orientations
-    eig_a = hermitian_eigh(torch.from_numpy(np.stack([b[0] for b in blocks])).to("cuda"))
-    eig_b = hermitian_eigh(torch.from_numpy(np.stack([b[1] for b in blocks])).to("cuda"))
-    stream = _lib.stream_handle()
-    for row in range(len(hamiltonians)):
-        spec_a = _Spectrum(torch, eig_a[0][row], eig_a[1][row])
-        spec_b = _Spectrum(torch, eig_b[0][row], eig_b[1][row])
-        margin = 3
-        half_a = int(math.ceil(spec_a.max_gap / delta)) + margin
-        half_b = int(math.ceil(spec_b.max_gap / delta)) + margin
-        out_len = (2 * half_a + 1) + (2 * half_b + 1) - 1
-        nfft = 1 << max(1, (out_len - 1).bit_length())
-        # rows 0..8: radical A's binned spectra of (p, q), rows 9..17: radical B's, zero-padded
-        rows = torch.zeros((18, nfft), dtype=torch.complex128, device="cuda")
-        for p in range(3):
-            for q in range(3):
-                ga = _binned(torch, spec_a, p, q, delta, half_a, bad)
-                gb = _binned(torch, spec_b, p, q, delta, half_b, bad)
-                rows[3 * p + q, :ga.numel()] = ga
-                rows[9 + 3 * p + q, :gb.numel()] = gb
-        if int(bad.item()):
-            raise ValueError("Frequency grid is too small for transition spectrum.")
-        scratch = torch.empty_like(rows)
-        _lib.call("rpm_fft_pow2", nfft, 18, _lib.ptr(rows), _lib.ptr(scratch), 0, stream)
-        combined = torch.zeros((1, nfft), dtype=torch.complex128, device="cuda")
-        for k in range(9):
-            _lib.call("rpm_spectrum_mac", nfft, _lib.ptr(combined), _lib.ptr(rows[k]), _lib.ptr(rows[9 + k]), stream)
-        _lib.call("rpm_fft_pow2", nfft, 1, _lib.ptr(combined), _lib.ptr(scratch), 1, stream)
-        conv = combined[0, :out_len] / nfft
-        omega = (torch.arange(out_len, dtype=torch.float64, device="cuda") - (half_a + half_b)) * delta
-        initial[row] = float((0.25 + conv.sum()).real.item())
-        for col, tau in enumerate(lifetimes):
-            k = 1.0 / tau
-            kern = k / (k - 1j * omega)
-            yields[row, col] = float((0.25 + (conv * kern).sum()).real.item())
-    return yields, initial
+    # one batched eigen-decomposition of both radicals over all orientations
+    lam_a, vec_a, lam_b, vec_b = _eigh_pair(*(torch.from_numpy(np.stack([b[k] for b in blocks])).to("cuda")
+                                              for k in (0, 1)))
+    da, db, count = lam_a.shape[1], lam_b.shape[1], len(blocks)
+    half_a, half_b = (_half_widths(lam.cpu().numpy(), delta) for lam in (lam_a, lam_b))
+    times = np.array(lifetimes)
+    out = torch.empty((count, 1 + len(lifetimes)), dtype=torch.float64, device="cuda")
+    bad = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def size(k, n):
+        need = ctypes.c_longlong()
+        _lib.call("rpm_factorized_workspace", da, db, n, half_a[k:].ctypes.data, half_b[k:].ctypes.data,
+                  len(lifetimes), ctypes.byref(need))
+        return need.value
+
+    k = 0
+    while k < count:
+        n = min(count - k, 32767)
+        while n > 1 and size(k, n) > _WORKSPACE_BYTES:
+            n = (n + 1) // 2
+        work = torch.empty(size(k, n), dtype=torch.uint8, device="cuda")
+        _lib.call("rpm_factorized_yields", da, db, n, _lib.ptr(lam_a[k:]), _lib.ptr(vec_a[k:]), _lib.ptr(lam_b[k:]),
+                  _lib.ptr(vec_b[k:]), delta, half_a[k:].ctypes.data, half_b[k:].ctypes.data, times.ctypes.data,
+                  len(lifetimes), _lib.ptr(out[k:]), _lib.ptr(bad), _lib.ptr(work), _lib.stream_handle())
+        k += n
+    if int(bad.item()):
+        raise ValueError("Frequency grid is too small for transition spectrum.")
+    values = out.cpu().numpy()
+    return np.ascontiguousarray(values[:, 1:]), np.ascontiguousarray(values[:, 0])
