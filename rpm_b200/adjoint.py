@@ -57,7 +57,7 @@ import numpy as np
 from . import _lib
 from .batched import STATUS_TEXT, BatchedPropagator
 from .engine import CompiledFullPairHamiltonian, _torch
-from .model import zeeman_operator
+from .model import _kron, zeeman_operator
 
 PARAMETERS = ("field_microT", "theta", "phi", "pulse_nT", "hyperfine_scale")
 TAYLOR_TOLERANCE = 1e-10
@@ -102,7 +102,7 @@ def electron_pair_zeeman(field_mT) -> np.ndarray:
     """4 x 4 operator Z(B) (x) 1 + 1 (x) Z(B) on (eA, eB), index 2 eA + eB."""
     z = zeeman_operator(np.asarray(field_mT, dtype=float))
     eye = np.eye(2)
-    return np.kron(z, eye) + np.kron(eye, z)
+    return _kron(z, eye) + _kron(eye, z)
 
 
 def _unit_vectors(theta: float, phi: float):
@@ -222,15 +222,22 @@ def _uniform_grid(times_us) -> tuple[np.ndarray, float]:
     return t, dt
 
 
-def spectral_radius(hamiltonian, *, iterations: int = 40, seed: int = 7) -> float:
+def _radius_start(n: int, seed: int):
+    """The normalised random vector that :func:`spectral_radius` starts from."""
+    rng = np.random.default_rng(seed)
+    v = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    return _torch().as_tensor(v / np.linalg.norm(v), dtype=_torch().complex128, device="cuda")
+
+
+def spectral_radius(hamiltonian, *, iterations: int = 40, seed: int = 7, start=None) -> float:
     """Largest |Ritz value| of an FP64 Lanczos basis grown from a random vector
-    (``rpm_lanczos_basis``): a close lower estimate of ||H||."""
+    (``rpm_lanczos_basis``): a close lower estimate of ||H||.  ``start``: the
+    start vector on the device, for several operators of one dimension (drawing
+    one of 221,184 components takes 8 ms, the basis 2.2 ms)."""
     torch = _torch()
     n = hamiltonian.dimension
     m = int(min(iterations, n))
-    rng = np.random.default_rng(seed)
-    v = rng.standard_normal(n) + 1j * rng.standard_normal(n)
-    state = torch.as_tensor(v / np.linalg.norm(v), dtype=torch.complex128, device="cuda")
+    state = _radius_start(n, seed) if start is None else start
     basis = torch.empty((m, n), dtype=torch.complex128, device="cuda")
     alpha = torch.zeros(m, dtype=torch.float64, device="cuda")
     beta = torch.zeros(max(m - 1, 1), dtype=torch.float64, device="cuda")
@@ -315,7 +322,8 @@ class AdjointYieldGradient:
         hams = (h_static, h_pulse)
         seg = self.model.interval_segments(t)
         ntraj = len(initial_states)
-        radius = 1.1 * max(spectral_radius(h_static), spectral_radius(h_pulse))
+        start = _radius_start(h_static.dimension, 7)
+        radius = 1.1 * max(spectral_radius(h, start=start) for h in hams)
         degree = taylor_degree(radius * dt, self.taylor_tolerance)
         n = int(np.prod(self.model.dimensions))
         # the batched propagator fixes the state layout (leading dimension)
