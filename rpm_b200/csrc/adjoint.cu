@@ -521,28 +521,26 @@ double read_tail(rpm_adjoint* a, size_t need, cudaStream_t st) {
 constexpr int kTaylorThreads = 384;
 constexpr size_t kTaylorSmem = 200 * 1024;
 
-__global__ void __launch_bounds__(kTaylorThreads) k_adj_taylor(const CubeView<double2>* __restrict__ view,
-                                                              double2* __restrict__ U, int groups, long long ld,
+__global__ void __launch_bounds__(kTaylorThreads) k_adj_taylor(const direct::Args<double2> a, double2* __restrict__ U, int groups, long long ld,
                                                               long long slot, const double* __restrict__ scales,
                                                               int degree) {
   using namespace direct;
   __shared__ Tables tb;
   extern __shared__ __align__(16) double2 tsm[];
-  const int hr = view->half_r, hl = view->half_l;
+  const int hr = a.hr, hl = groups / hr;
   double2* tab = tsm;
-  HRec* lrec = reinterpret_cast<HRec*>(tab + view->L.ntab + view->R.ntab);
+  HRec* lrec = reinterpret_cast<HRec*>(tab + a.ntl + a.ntr);
   HRec* rrec = lrec + hl;
   double2* cur = reinterpret_cast<double2*>(rrec + hr);
   double2* nxt = cur + 4 * groups;
-  load_tables(view, tb, tab);
   constexpr int W = sizeof(HRec) / sizeof(double2);
   for (int k = threadIdx.x; k < hl * W; k += blockDim.x)
-    reinterpret_cast<double2*>(lrec)[k] = static_cast<const double2*>(view->lrec)[k];
+    reinterpret_cast<double2*>(lrec)[k] = static_cast<const double2*>(a.lrec)[k];
   for (int k = threadIdx.x; k < hr * W; k += blockDim.x)
-    reinterpret_cast<double2*>(rrec)[k] = static_cast<const double2*>(view->rrec)[k];
+    reinterpret_cast<double2*>(rrec)[k] = static_cast<const double2*>(a.rrec)[k];
   double2* u = U + (long long)blockIdx.x * ld;
   for (int k = threadIdx.x; k < 4 * groups; k += blockDim.x) cur[k] = u[k];
-  __syncthreads();
+  load_tables(a, tb, tab);
   for (int t = 0; t < degree; ++t) {
     const double s = scales[t];
     double2* out = u + (long long)(t + 1) * slot;
@@ -588,7 +586,8 @@ bool taylor_one_launch(rpm_adjoint* a, rpm_system* h, int count, cudaStream_t st
   check_cuda(cudaFuncSetAttribute(k_adj_taylor, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTaylorSmem),
              "adjoint Taylor smem attr");
   const int threads = std::min(kTaylorThreads, (groups + 31) / 32 * 32);
-  k_adj_taylor<<<count, threads, taylor_smem(h), st>>>(h->cube64_dev, static_cast<double2*>(a->U), groups, a->ld,
+  k_adj_taylor<<<count, threads, taylor_smem(h), st>>>(direct::make_args(h->cube64, h->cube64_dev),
+                                                       static_cast<double2*>(a->U), groups, a->ld,
                                                        2LL * a->B * a->ld, a->scales, a->degree);
   check_launch("k_adj_taylor");
   return true;

@@ -190,6 +190,8 @@ struct CubeView {
   // the direct H psi (hpsi_direct.cuh, hpsi_direct32.cu); else null
   const void* lrec;
   const void* rrec;
+  const void* parts;  // partner lists of both radicals (direct::Partner)
+  int parts_n[2];
   // complex128: bit k set when nucleus k of the radical has any transition to
   // another level (its block of the table is not diagonal in the nucleus)
   unsigned moves_l, moves_r;

@@ -35,41 +35,76 @@ struct __align__(16) Partner {
   int stride, offx, pad2;
 };
 
-struct Tables {
+template <class T>
+struct TablesOf {
   int np[2];
+  int has_pair, pad;
   Partner part[2][kMaxPartners];
-  double2 pair[16];
-  int has_pair;
+  T pair[16];
+};
+using Tables = TablesOf<double2>;
+
+// What a launch passes beside the device view, so that a block's first loads do
+// not wait for one another.  Through the view (its sizes, then its pointers,
+// then the tables; the partner lists built by each block) the direct H psi took
+// 5.0 us at 864 x 64, 11.9 at 221,184 x 1, 183 at 221,184 x 32, now 4.1, 10.8
+// and 173; staging the tables once for several vectors instead (a loop over the
+// batch in each block) spills at 80 registers: 187 us.
+template <class T>
+struct Args {
+  const CubeView<T>* view;
+  const T *tab_l, *tab_r;
+  const Partner* parts;
+  const void *lrec, *rrec;
+  int ntl, ntr, hr, np[2];
 };
 
-// Fills `tb` and stages both coefficient tables (left first) into `tab`;
-// every thread of the block takes part, a barrier has to follow.
-__device__ __forceinline__ void load_tables(const CubeView<double2>* view, Tables& tb, double2* tab) {
-  const int nl = view->L.ntab;
-  for (int k = threadIdx.x; k < nl; k += blockDim.x) tab[k] = view->tabL[k];
-  for (int k = threadIdx.x; k < view->R.ntab; k += blockDim.x) tab[nl + k] = view->tabR[k];
-  for (int k = threadIdx.x; k < 2 * kCubeMaxDigits; k += blockDim.x) {
-    const int side = k / kCubeMaxDigits, q = k % kCubeMaxDigits;
-    const CubeSide& s = side ? view->R : view->L;
-    // nuclei without transitions (a quadrupole system's spin-1/2 ones) have no partners
-    const unsigned moves = side ? view->moves_r : view->moves_l;
-    if (q < s.K) {
-      int at = 0;
-      for (int p = 0; p < q; ++p) at += (moves >> p) & 1u ? s.dim[p] - 1 : 0;
-      const int d = (moves >> q) & 1u ? s.dim[q] : 1;
-      for (int t = 1; t < d; ++t)
-        tb.part[side][at + t - 1] =
-            Partner{(unsigned char)(4 * q), (unsigned char)t, (unsigned char)d, 0,
-                    s.gs[q] * (side ? 1 : view->half_r), s.offX[q] + (side ? nl : 0), 0};
-      if (q == s.K - 1) tb.np[side] = at + d - 1;
+template <class T>
+inline Args<T> make_args(const CubeView<T>& host, const CubeView<T>* dev) {
+  return Args<T>{dev,       host.tabL,   host.tabR,   static_cast<const Partner*>(host.parts), host.lrec, host.rrec,
+                 host.L.ntab, host.R.ntab, host.half_r, {host.parts_n[0], host.parts_n[1]}};
+}
+
+// Partner lists of both radicals ([2][kMaxPartners]); nuclei without
+// transitions (a quadrupole system's spin-1/2 ones) have none.
+inline std::vector<Partner> partner_lists(const CubeSide& l, const CubeSide& r, int half_r, unsigned moves_l,
+                                          unsigned moves_r, int (&np)[2]) {
+  std::vector<Partner> out(2 * kMaxPartners);
+  for (int side = 0; side < 2; ++side) {
+    const CubeSide& s = side ? r : l;
+    int at = 0;
+    for (int q = 0; q < s.K; ++q) {
+      if (!(((side ? moves_r : moves_l) >> q) & 1u)) continue;
+      for (int t = 1; t < s.dim[q]; ++t)
+        out[side * kMaxPartners + at++] =
+            Partner{(unsigned char)(4 * q), (unsigned char)t, (unsigned char)s.dim[q], 0,
+                    s.gs[q] * (side ? 1 : half_r), s.offX[q] + (side ? l.ntab : 0), 0};
     }
+    np[side] = at;
   }
-  if (threadIdx.x < 16) tb.pair[threadIdx.x] = view->pair[threadIdx.x];
-  if (threadIdx.x == 0) {
-    bool any = false;
-    for (int k = 0; k < 16; ++k) any = any || view->pair[k].x != 0.0 || view->pair[k].y != 0.0;
-    tb.has_pair = any ? 1 : 0;
+  return out;
+}
+
+// Fills `tb` and stages both coefficient tables (left first) into `tab`; every
+// thread of the block takes part.  Ends with a barrier.
+template <class T>
+__device__ __forceinline__ void load_tables(const Args<T>& a, TablesOf<T>& tb, T* tab) {
+  for (int k = threadIdx.x; k < a.ntl; k += blockDim.x) tab[k] = a.tab_l[k];
+  for (int k = threadIdx.x; k < a.ntr; k += blockDim.x) tab[a.ntl + k] = a.tab_r[k];
+#pragma unroll
+  for (int side = 0; side < 2; ++side)
+    for (int k = threadIdx.x; k < a.np[side]; k += blockDim.x)
+      reinterpret_cast<int4*>(tb.part[side])[k] = reinterpret_cast<const int4*>(a.parts + side * kMaxPartners)[k];
+  bool any = false;
+  if (threadIdx.x < 16) {
+    const T p = a.view->pair[threadIdx.x];
+    tb.pair[threadIdx.x] = p;
+    any = p.x != 0 || p.y != 0;
   }
+  if (threadIdx.x < 2) tb.np[threadIdx.x] = threadIdx.x ? a.np[1] : a.np[0];
+  const int has = __syncthreads_or(any);
+  if (threadIdx.x == 0) tb.has_pair = has;
+  __syncthreads();
 }
 
 // out[2 eA + eB] = (H x)[eA, eB, l, r]; x: the thread's own components,

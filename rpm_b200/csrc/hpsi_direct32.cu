@@ -7,14 +7,15 @@
 // that the batched propagation uses (their order of additions is part of its
 // results) move a partial result through memory and take two launches, the
 // second behind the first.  Two passes -> this kernel, microseconds:
-//   864 x 64           13.2 ->   5.4
-//   13,824 x 1          9.3 ->   6.7
-//   55,296 x 8         13.6 ->  10.1
-//   221,184 x 1, 4, 8  21.9, 22.2, 33.5 -> 9.1, 15.0, 26.3
-//   221,184 x 48        146 -> 129
+//   864 x 64           13.2 ->   4.9
+//   13,824 x 1          9.3 ->   6.3
+//   55,296 x 8         13.6 ->   9.1
+//   221,184 x 1, 4, 8  21.9, 22.2, 33.5 -> 8.3, 14.3, 24.6
+//   221,184 x 48        146 -> 122
 // Bound by the load/store unit (each component is read once per partner, from
-// L1 and L2).  Six blocks of 128 threads per SM: at five 136 us, at four 145,
-// at seven 133, at eight 138; 64 threads 139, 256 threads 131.
+// L1 and L2).  Six blocks of 128 threads per SM: 129 us before the tables came
+// by argument; then at five 136 us, at four 145, at seven 133, at eight 138; 64
+// threads 139, 256 threads 131.
 #include "hpsi_direct.cuh"
 
 #include <cstring>
@@ -38,52 +39,25 @@ using direct::Partner;
 
 constexpr int kThreads32 = 128;
 
-struct Tables32 {
-  int np[2];  // partners; the right radical's without its fastest nucleus
-  Partner part[2][kMaxPartners];
-  float2 pair[16];
-  float2 fast[16];  // block of the fastest right nucleus, (e, m) x (e', m')
-  int has_pair;
-};
+using direct::Args;
+using Tables32 = direct::TablesOf<float2>;  // the right partners without the fastest nucleus's
 
-__global__ void __launch_bounds__(kThreads32, 6) k_hpsi_direct32(const CubeView<float2>* __restrict__ view,
+__global__ void __launch_bounds__(kThreads32, 6) k_hpsi_direct32(const Args<float2> ar,
                                                                 const float2* __restrict__ in,
-                                                                float2* __restrict__ out, int pairs, long long ld) {
+                                                                float2* __restrict__ out, int pairs, long long ld,
+                                                                int off_fast) {
   __shared__ Tables32 tb;
   extern __shared__ float2 tab32[];
-  const int ntl = view->L.ntab, ntr = view->R.ntab, hr = view->half_r;
-  for (int k = threadIdx.x; k < ntl; k += kThreads32) tab32[k] = view->tabL[k];
-  for (int k = threadIdx.x; k < ntr; k += kThreads32) tab32[ntl + k] = view->tabR[k];
-  for (int k = threadIdx.x; k < 2 * kCubeMaxDigits; k += kThreads32) {
-    const int side = k / kCubeMaxDigits, q = k % kCubeMaxDigits;
-    const CubeSide& s = side ? view->R : view->L;
-    const int count = s.K - side;  // digits that go through partners
-    if (q < count) {
-      int at = 0;
-      for (int p = 0; p < q; ++p) at += s.dim[p] - 1;
-      const int d = s.dim[q];
-      for (int t = 1; t < d; ++t)
-        tb.part[side][at + t - 1] = Partner{(unsigned char)(4 * q), (unsigned char)t, (unsigned char)d, 0,
-                                            s.gs[q] * (side ? 1 : hr), s.offX[q] + (side ? ntl : 0), 0};
-      if (q == count - 1) tb.np[side] = at + d - 1;
-    }
-    if (q == 0 && count == 0) tb.np[side] = 0;
-  }
-  if (threadIdx.x < 16) {
-    tb.pair[threadIdx.x] = view->pair[threadIdx.x];
-    tb.fast[threadIdx.x] = view->tabR[view->R.offX[view->R.K - 1] + threadIdx.x];
-  }
-  if (threadIdx.x == 0) {
-    bool any = false;
-    for (int k = 0; k < 16; ++k) any = any || view->pair[k].x != 0.f || view->pair[k].y != 0.f;
-    tb.has_pair = any ? 1 : 0;
-  }
-  __syncthreads();
   const int idx = blockIdx.x * kThreads32 + threadIdx.x;
-  if (idx >= pairs) return;
-  const int hr2 = hr / 2;
+  const int hr2 = ar.hr / 2;
   const int l = idx / hr2, r = 2 * (idx - l * hr2);
+  load_tables(ar, tb, tab32);
+  if (idx >= pairs) return;
+  const float2* fast = tab32 + off_fast;  // block of the fastest right nucleus, (e, m) x (e', m')
   const long long q = 2LL * pairs;
+  const HRec32 lr = static_cast<const HRec32*>(ar.lrec)[l];
+  const HRec32* rp = static_cast<const HRec32*>(ar.rrec) + r;
+  const unsigned long long rdigits = rp[0].digits;
   const float2* v = in + (long long)blockIdx.y * ld + 2LL * idx;
   auto load = [&](int delta, float2 (&y)[4][2]) {
 #pragma unroll
@@ -101,9 +75,6 @@ __global__ void __launch_bounds__(kThreads32, 6) k_hpsi_direct32(const CubeView<
   for (int e = 0; e < 4; ++e)
 #pragma unroll
     for (int i = 0; i < 2; ++i) o[e][i] = w[e][i] = czero<float2>();
-  const HRec32 lr = static_cast<const HRec32*>(view->lrec)[l];
-  const HRec32* rp = static_cast<const HRec32*>(view->rrec) + r;
-  const unsigned long long rdigits = rp[0].digits;
 #pragma unroll
   for (int side = 0; side < 2; ++side) {
     float2(&acc)[4][2] = side ? w : o;
@@ -150,8 +121,8 @@ __global__ void __launch_bounds__(kThreads32, 6) k_hpsi_direct32(const CubeView<
           z[2 * a + b][i] = cfma(lr.f[a], x[2 * (1 - a) + b][i], t);
           // the electron flip and the fastest nucleus belong to the right radical
           t = cfma(rr.f[b], x[2 * a + 1 - b][i], w[2 * a + b][i]);
-          t = cfma(tb.fast[(2 * b + i) * 4 + 1 - i], x[2 * a][1 - i], t);
-          w[2 * a + b][i] = cfma(tb.fast[(2 * b + i) * 4 + 2 + 1 - i], x[2 * a + 1][1 - i], t);
+          t = cfma(fast[(2 * b + i) * 4 + 1 - i], x[2 * a][1 - i], t);
+          w[2 * a + b][i] = cfma(fast[(2 * b + i) * 4 + 2 + 1 - i], x[2 * a + 1][1 - i], t);
         }
   }
   if (tb.has_pair) {
@@ -185,8 +156,11 @@ bool direct32_usable(const rpm_system* sys, const float2* in, const float2* out,
 void launch_direct32(rpm_system* sys, const float2* in, float2* out, int batch, long long ld, cudaStream_t stream) {
   const int pairs = (int)(sys->n / 8);
   const size_t smem = sizeof(float2) * (size_t)(sys->cube_l.ntab + sys->cube_r.ntab);
-  k_hpsi_direct32<<<dim3((pairs + kThreads32 - 1) / kThreads32, batch), kThreads32, smem, stream>>>(
-      sys->cube32_dev, in, out, pairs, ld);
+  const int gx = (pairs + kThreads32 - 1) / kThreads32;
+  const CubeSide& cr = sys->cube_r;
+  k_hpsi_direct32<<<dim3(gx, batch), kThreads32, smem, stream>>>(
+      direct::make_args(sys->cube32, sys->cube32_dev), in, out, pairs, ld,
+      sys->cube_l.ntab + cr.offX[cr.K - 1]);
   check_launch("k_hpsi_direct32");
 }
 

@@ -45,6 +45,7 @@ constexpr size_t kDynamicLimit = 208 * 1024;  // dynamic shared memory beside ab
 
 struct PlainBasis {
   const CubeView<double2>* view;
+  direct::Args<double2> tables;
   const double2* state;
   double2* basis;
   long long n;
@@ -116,7 +117,7 @@ __global__ void __launch_bounds__(kPT, 1) k_plain_basis(const PlainBasis p) {
   HRec* rrec = lrec + p.lrecs;
   double2* w = reinterpret_cast<double2*>(rrec + hr);  // [e][gpb]
   double2* vc = w + 4 * p.gpb;                         // [k][e][gpb]
-  direct::load_tables(p.view, tb, tab);
+  direct::load_tables(p.tables, tb, tab);
   {
     const double2* ls = reinterpret_cast<const double2*>(static_cast<const HRec*>(p.view->lrec) + l0);
     const double2* rs = static_cast<const double2*>(p.view->rrec);
@@ -302,6 +303,7 @@ bool launch_plain_basis(rpm_system* sys, const double2* state, int m, double tol
     }
   }
   p.view = sys->cube64_dev;
+  p.tables = direct::make_args(sys->cube64, sys->cube64_dev);
   p.state = state;
   p.basis = basis;
   p.n = sys->n;

@@ -425,6 +425,7 @@ static void upload_system(rpm_system* sys) {
         c32.orec_bytes_l = (int)(rl.size() * sizeof(float));  // records (padded to 16 bytes) + 128 pair bytes
       }
       c64.lrec = c64.rrec = c32.lrec = c32.rrec = nullptr;
+      c64.parts = c32.parts = nullptr;
       c32.moves_l = c32.moves_r = 0;
       c64.moves_l = moving_digits(cl, tl64);
       c64.moves_r = moving_digits(cr, tr64);
@@ -432,10 +433,16 @@ static void upload_system(rpm_system* sys) {
         const auto lr = direct_records(cl, tl64), rr = direct_records(cr, tr64);
         c64.lrec = upload<direct::HRec>(sys, lr.data(), lr.size() * sizeof(direct::HRec));
         c64.rrec = upload<direct::HRec>(sys, rr.data(), rr.size() * sizeof(direct::HRec));
+        const auto parts = direct::partner_lists(cl, cr, cr.half, c64.moves_l, c64.moves_r, c64.parts_n);
+        c64.parts = upload<direct::Partner>(sys, parts.data(), parts.size() * sizeof(direct::Partner));
         if (cr.dim[cr.K - 1] == 2) {
           const auto l32 = direct32_records(cl, sys->cube_tab_l), r32 = direct32_records(cr, sys->cube_tab_r);
           c32.lrec = upload<unsigned char>(sys, l32.data(), l32.size());
           c32.rrec = upload<unsigned char>(sys, r32.data(), r32.size());
+          // the fastest right nucleus has no partners: its pair is in registers
+          const auto parts32 = direct::partner_lists(cl, cr, cr.half, c64.moves_l,
+                                                     c64.moves_r & ~(1u << (cr.K - 1)), c32.parts_n);
+          c32.parts = upload<direct::Partner>(sys, parts32.data(), parts32.size() * sizeof(direct::Partner));
         }
       }
       sys->cube64_dev = upload<CubeView<double2>>(sys, &c64, sizeof(c64));
