@@ -103,6 +103,35 @@ def test_full_size_action_matches_general_kernels():
     assert float(torch.linalg.vector_norm(a - b) / torch.linalg.vector_norm(b)) < REL
 
 
+@pytest.mark.parametrize("case", [0, 1, 4, 6])
+@pytest.mark.parametrize("batch", [592, 3001])
+def test_two_vectors_per_thread_match_dense(case, batch):
+    """Batches from which vectors go in pairs (two blocks per SM), even and with one left over."""
+    import torch
+
+    import rpm_b200 as rb
+    from rpm_b200 import _lib
+
+    left, right = SHAPES[case]
+    dims = (2, 2) + left + right
+    rng = np.random.default_rng(300 + case)
+    terms = _terms(rb, rng, left, right, pair=case % 4 == 0)
+    h = rb.CompiledFullPairHamiltonian(dims, terms, left_axes=(0,) + tuple(range(2, 2 + len(left))),
+                                       right_axes=(1,) + tuple(range(2 + len(left), len(dims))))
+    n = h.dimension
+    x = rng.normal(size=(n, batch)) + 1j * rng.normal(size=(n, batch))
+    ref = _dense_apply(dims, terms, x)
+    ld = n + 3
+    xs = torch.full((batch, ld), float("nan"), dtype=torch.complex128, device="cuda")
+    xs[:, :n] = torch.from_numpy(np.ascontiguousarray(x.T))
+    out = torch.full_like(xs, 7.0)
+    _lib.call("rpm_hpsi", h._system.handle, _lib.PREC_C128, _lib.ptr(xs), _lib.ptr(out), batch, ld,
+              _lib.stream_handle())
+    got = out.cpu().numpy()
+    assert np.linalg.norm(got[:, :n].T - ref) <= REL * np.linalg.norm(ref)
+    assert np.all(got[:, n:] == 7.0)
+
+
 # fastest right nucleus a spin-1/2 (the complex64 form's condition): a lone
 # right nucleus, index-pair counts below, at and around one 128-thread block,
 # spins above 1/2 before it
