@@ -140,10 +140,10 @@ SHAPES32 = [((2,), (2,)), ((3,), (2, 2)), ((5, 3), (7, 2)), ((16,), (8, 2)), ((2
 
 
 @pytest.mark.parametrize("case", range(len(SHAPES32)))
-@pytest.mark.parametrize("batch,rates", [(1, None), (3, (1.0, 2.5))])
+@pytest.mark.parametrize("batch,rates", [(1, None), (3, (1.0, 2.5)), (741, None)])
 @pytest.mark.parametrize("offset,pad", [(0, 6), (1, 6), (0, 5)])
 def test_complex64_action_matches_dense(case, batch, rates, offset, pad):
-    """offset 1 (8-byte aligned) and the odd stride take the general passes.
+    """offset 1 (8-byte aligned) and the odd stride take the general passes; 741 vectors go in pairs, one is left over.
 
     Bar 2e-6 of the norm: fewer than 200 products of rounding 6e-8, as a random sum 200^0.5 x 6e-8 = 0.9e-6.
     """
