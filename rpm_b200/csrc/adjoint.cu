@@ -14,7 +14,8 @@
 // One backward sweep walks a run of intervals.  Per interval it builds the
 // Taylor basis u_j = (dt H)^j x / j! (j <= degree) of the pair
 // x = [lambda_{k+1}; psi_{k+1}] (one batched H psi launch of 2B vectors per
-// term, the dt / (j + 1) factor folded into the load), then one kernel forms
+// term, the dt / (j + 1) factor folded in; small complex128 states take all terms
+// in one launch), then one kernel forms
 // lambda and psi at the Gauss-Legendre nodes of the interval and at its
 // start, accumulates the electron-pair transition density
 //   M_ab += dt w_q sum_i conj(lambda_q[a, i]) psi_q[b, i]   (a, b = 2 eA + eB)

@@ -9,8 +9,9 @@
 //     exp(-i T t) e1, the error control and the singlet Gram/populations are
 //     FP64.
 // Each Krylov step is a fixed kernel sequence over all trajectories:
-//   start -> m x [H psi (pass L, pass R + alpha), update + beta]
-//         -> control -> rebuild -> gram -> observe
+//   start -> Lanczos or Arnoldi iterations per shape group (one persistent
+//   launch, one block per small state, or m pass pairs) -> control, with the
+//   Gram forked beside it -> rebuild, Gram sums -> observe
 // captured once as a CUDA graph and replayed until every trajectory reached
 // the last observation time.  Per-trajectory controller state lives on the
 // device; the host only polls a done-counter.

@@ -1,15 +1,15 @@
 // FP64 Krylov machinery for the plain (single-vector, complex128) propagator.
 //
 //   * Hermitian Lanczos with two classical Gram-Schmidt passes
-//     (rpm_statevector_engine.py:651-688), as a fixed launch sequence per
-//     basis vector with device-side breakdown flag, so no host round trip
-//     happens inside a basis build.
+//     (rpm_statevector_engine.py:651-688): one cooperative launch per basis where
+//     plain_lanczos.cu covers the system, else the fixed launch sequence per
+//     basis vector of this file with a device-side breakdown flag, so no host
+//     round trip happens inside a basis build.
 //   * Deterministic reductions: every block writes its partial sums, the
 //     last block to finish (atomic ticket) adds them in block order.
-//   * Symmetric tridiagonal eigen-decomposition by implicit QR with Wilkinson
-//     shifts (Golub & Van Loan, Matrix Computations, sec. 8.3): one thread runs
-//     the scalar bulge chase and records the Givens rotations; all threads
-//     then apply them to their own rows of the eigenvector matrix.
+//   * exp(-i T t) e1 by Chebyshev series of the tridiagonal (step control and
+//     rpm_krylov_coefficients); spectra by implicit QR with Wilkinson shifts
+//     (Golub & Van Loan, Matrix Computations, sec. 8.3) for rpm_krylov_spectra.
 //   * exp(-i T t) e1 coefficients, embedded error norms and projected singlet
 //     populations (rpm_statevector_engine.py:569-609, 690-715, 521-538).
 //   * Singlet Gram, state recombination, norms and the Simpson yield
