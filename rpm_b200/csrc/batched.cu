@@ -336,7 +336,7 @@ __device__ __forceinline__ void pair_sync(int pair) { asm volatile("bar.sync %0,
 // Latency-bound FP64 chains: with four warps in all, every warp applying its
 // own rotations and evaluating hi and lo one after the other, a step took 233
 // us at M = 30 and 472 us at M = 40; with branches in each rotation of the
-// chase 197 and 340 us; now 171 us at M = 30.
+// chase 197 and 387 us; now 171 and 289 us.
 // Dynamic shared memory: two spectra records (hi, lo).
 constexpr int kCtlWarps = 16;
 constexpr int kCtlPairs = kCtlWarps / 2;

@@ -40,22 +40,6 @@ __device__ __forceinline__ double warp_reduce(double v) {
   return v;
 }
 
-// Sum over the block (every thread returns the total).
-__device__ double block_reduce_sum(double v, double* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  __syncthreads();
-  v = warp_reduce(v);
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  if (warp == 0) {
-    double t = lane < nw ? red[lane] : 0.0;
-    t = warp_reduce(t);
-    if (lane == 0) red[0] = t;
-  }
-  __syncthreads();
-  return red[0];
-}
-
 // One size's share of a call; two radicals' matrices run in the same launches.
 struct HePart {
   int n = 0;
@@ -75,7 +59,9 @@ struct HePair {
 };
 
 constexpr int kHeSmem = 200 * 1024;    // rows of eigenvectors
-constexpr int kHeMatSmem = 193 * 1024; // the matrix, beside 33 KB of vectors
+// the reduction's vectors and the whole matrix
+__host__ __device__ constexpr size_t tridiag_smem(int n) { return sizeof(double2) * ((size_t)n * n + 3 * (size_t)n); }
+__host__ __device__ constexpr bool tridiag_in_smem(int n) { return tridiag_smem(n) <= 224 * 1024; }
 
 // 0.5 (A + A^H) in place.
 __global__ void __launch_bounds__(256) k_he_symmetrise(HePair p) {
@@ -96,72 +82,69 @@ __global__ void __launch_bounds__(256) k_he_symmetrise(HePair p) {
 // Householder reduction of matrix b: a (n x n, row-major, overwritten), d, e
 // (n, n - 1 real), house (n x n: row k holds v_k, v_k[j] for j > k, v_k[k+1]
 // = 1), tau (n - 1 complex).  Bound by the barriers and latencies of its n - 1
-// serial steps.  A matrix that fits is worked on in shared memory (n <= 111),
-// and rows go to warps, without a division per element: 6 x 72 and 6 x 48 took
-// 313 + 172 us from global memory, one size after the other; now 290 us together
-// (512 threads 275, but 288 x 288 8.7 ms against 6.4; 256 threads 330).
+// serial steps.  A matrix that fits is worked on in shared memory (n <= 118),
+// rows go to warps, one warp makes the reflector alone, and every warp forms
+// w^H v for itself: four barriers a step.  6 x 72 and 6 x 48 took 313 + 172 us
+// from global memory with eleven barriers a step, one size after the other; 290 us
+// together with eleven barriers and the matrix in shared memory, 244 us now; 192,
+// 288, 384 dimensions (in global memory) 2.4, 6.7, 14.2 -> 2.1, 6.3, 13.3 ms.
 __global__ void __launch_bounds__(kHeThreads) k_he_tridiag(HePair p) {
-  __shared__ double2 v[kHeMaxN], w[kHeMaxN];
-  __shared__ double red[32];
   __shared__ double2 s_tau;
-  __shared__ double s_beta;
   extern __shared__ double2 he_smem[];
   int b;
   const HePart& h = p.of(blockIdx.x, &b);
   const int n = h.n;
   const size_t nn = (size_t)n * n;
+  double2 *v = he_smem, *w = v + n, *u = w + n;  // u = w + alpha v
   double2* a = h.a + b * nn;
   double* d = h.d + (size_t)b * n;
   double* e = h.e + (size_t)b * n;
   double2* house = h.house + b * nn;
   double2* tau = h.tau + (size_t)b * n;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if (nn * sizeof(double2) <= kHeMatSmem) {
-    for (int k = threadIdx.x; k < (int)nn; k += blockDim.x) he_smem[k] = a[k];
-    a = he_smem;
+  if (tridiag_in_smem(n)) {
+    double2* own = u + n;
+    for (int k = threadIdx.x; k < (int)nn; k += blockDim.x) own[k] = a[k];
+    a = own;
     __syncthreads();
   }
   for (int k = 0; k + 1 < n; ++k) {
     const int m = n - k - 1;  // trailing size
-    // x = A[k+1:, k] = conj(A[k, k+1:]) (A Hermitian, full storage)
-    double part = 0.0;
-    for (int j = 1 + threadIdx.x; j < m; j += blockDim.x) {
-      const double2 x = a[(size_t)k * n + k + 1 + j];
-      part += x.x * x.x + x.y * x.y;
-    }
-    const double xnorm2 = block_reduce_sum(part, red);
-    if (threadIdx.x == 0) {
-      const double2 alpha = cconj(a[(size_t)k * n + k + 1]);
-      if (xnorm2 == 0.0 && alpha.y == 0.0) {
-        s_tau = make_double2(0.0, 0.0);
-        s_beta = alpha.x;
-      } else {
-        const double beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xnorm2), alpha.x);
-        s_tau = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
-        s_beta = beta;
+    if (warp == 0) {
+      // x = A[k+1:, k] = conj(A[k, k+1:]) (A Hermitian, full storage)
+      const double2* row = a + (size_t)k * n + k + 1;
+      double part = 0.0;
+      for (int j = 1 + lane; j < m; j += 32) {
+        const double2 x = row[j];
+        part += x.x * x.x + x.y * x.y;
+      }
+      const double xnorm2 = warp_reduce(part);
+      const double2 alpha = cconj(row[0]);
+      double2 t = make_double2(0.0, 0.0), scale = t;
+      double beta = alpha.x;
+      if (!(xnorm2 == 0.0 && alpha.y == 0.0)) {
+        beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xnorm2), alpha.x);
+        t = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
         // 1 / (alpha - beta)
         const double2 den = make_double2(alpha.x - beta, alpha.y);
         const double dd = den.x * den.x + den.y * den.y;
-        w[0] = make_double2(den.x / dd, -den.y / dd);
+        scale = make_double2(den.x / dd, -den.y / dd);
+      }
+      for (int j = lane; j < m; j += 32) {
+        const double2 vj = j > 0 ? cmul(cconj(row[j]), scale) : make_double2(1.0, 0.0);
+        v[j] = vj;
+        house[(size_t)k * n + k + 1 + j] = vj;
+      }
+      if (lane == 0) {
+        s_tau = t;
+        tau[k] = t;
+        d[k] = a[(size_t)k * n + k].x;
+        e[k] = beta;
       }
     }
     __syncthreads();
     const double2 t = s_tau;
-    const bool reflect = t.x != 0.0 || t.y != 0.0;
-    const double2 scale = w[0];
-    for (int j = threadIdx.x; j < m; j += blockDim.x) {
-      double2 vj = make_double2(1.0, 0.0);
-      if (j > 0) vj = reflect ? cmul(cconj(a[(size_t)k * n + k + 1 + j]), scale) : make_double2(0.0, 0.0);
-      v[j] = vj;
-      house[(size_t)k * n + k + 1 + j] = vj;
-    }
-    if (threadIdx.x == 0) {
-      tau[k] = t;
-      d[k] = a[(size_t)k * n + k].x;
-      e[k] = s_beta;
-    }
-    __syncthreads();
-    if (reflect) {
+    if (t.x != 0.0 || t.y != 0.0) {
       // w = tau A22 v, one warp per row (lanes over the row's columns)
       for (int i = warp; i < m; i += nw) {
         const double2* row = a + (size_t)(k + 1 + i) * n + k + 1;
@@ -176,34 +159,35 @@ __global__ void __launch_bounds__(kHeThreads) k_he_tridiag(HePair p) {
         if (lane == 0) w[i] = cmul(t, make_double2(sx, sy));
       }
       __syncthreads();
-      // alpha = -1/2 tau (w^H v), by every warp for itself; w += alpha v
-      double wx = 0.0, wy = 0.0;
-      for (int j = lane; j < m; j += 32) {
-        const double2 q = cmul(cconj(w[j]), v[j]);
-        wx += q.x;
-        wy += q.y;
-      }
-      wx = warp_reduce(wx);
-      wy = warp_reduce(wy);
-      const double2 al = cmul(make_double2(-0.5 * t.x, -0.5 * t.y), make_double2(wx, wy));
-      __syncthreads();
-      for (int j = threadIdx.x; j < m; j += blockDim.x) {
-        const double2 q = cmul(al, v[j]);
-        w[j] = make_double2(w[j].x + q.x, w[j].y + q.y);
-      }
-      __syncthreads();
-      // A22 -= v w^H + w v^H (full storage)
-      for (int i = warp; i < m; i += nw) {
-        double2* row = a + (size_t)(k + 1 + i) * n + k + 1;
-        const double2 vi = v[i], wi = w[i];
+      // alpha = -1/2 tau (w^H v), by every warp that has columns; u = w + alpha v
+      if (warp * 32 < m) {
+        double wx = 0.0, wy = 0.0;
         for (int j = lane; j < m; j += 32) {
-          const double2 q = cmul(vi, cconj(w[j])), u = cmul(wi, cconj(v[j]));
-          const double2 x = row[j];
-          row[j] = make_double2(x.x - q.x - u.x, x.y - q.y - u.y);
+          const double2 q = cmul(cconj(w[j]), v[j]);
+          wx += q.x;
+          wy += q.y;
+        }
+        wx = warp_reduce(wx);
+        wy = warp_reduce(wy);
+        const double2 al = cmul(make_double2(-0.5 * t.x, -0.5 * t.y), make_double2(wx, wy));
+        for (int j = threadIdx.x; j < m; j += blockDim.x) {
+          const double2 q = cmul(al, v[j]);
+          u[j] = make_double2(w[j].x + q.x, w[j].y + q.y);
         }
       }
       __syncthreads();
+      // A22 -= v u^H + u v^H (full storage)
+      for (int i = warp; i < m; i += nw) {
+        double2* row = a + (size_t)(k + 1 + i) * n + k + 1;
+        const double2 vi = v[i], ui = u[i];
+        for (int j = lane; j < m; j += 32) {
+          const double2 q = cmul(vi, cconj(u[j])), r = cmul(ui, cconj(v[j]));
+          const double2 x = row[j];
+          row[j] = make_double2(x.x - q.x - r.x, x.y - q.y - r.y);
+        }
+      }
     }
+    __syncthreads();
   }
   if (threadIdx.x == 0) d[n - 1] = a[(size_t)(n - 1) * n + n - 1].x;
 }
@@ -609,8 +593,7 @@ void eigh_run(HePair& p, int parts, bool symmetrise, cudaStream_t stream) {
     row_blocks = std::max(row_blocks, (h.n + h.rows - 1) / h.rows);
     row_threads = std::max(row_threads, (h.rows + 31) / 32 * 32);
     eig_smem = std::max(eig_smem, sizeof(double) * (size_t)(2 * h.n + kEigPad + h.n * h.rows));
-    const size_t mat = sizeof(double2) * (size_t)h.n * h.n;
-    if (mat <= (size_t)kHeMatSmem) red_smem = std::max(red_smem, mat);
+    red_smem = std::max(red_smem, tridiag_in_smem(h.n) ? tridiag_smem(h.n) : sizeof(double2) * 3 * (size_t)h.n);
     check_cuda(cudaMemsetAsync(h.status, 0, sizeof(int) * p.batch, stream), "eigh status");
   }
   const int items = p.batch * parts;
