@@ -372,7 +372,8 @@ int rpm_he_eigh_pair(int na, int nb, int batch, void* a_dev, void* b_dev, double
  * k = 1 / lifetimes[t] (host array, nlife >= 1).  lam: ascending eigenvalues,
  * v: eigenvectors as columns (electron digit slowest, even da, db).
  * *bad_dev is raised when a line falls outside its grid.  work_dev:
- * rpm_factorized_workspace bytes.  Asynchronous on the stream. */
+ * rpm_factorized_workspace bytes.  Asynchronous on the stream; copies host
+ * arrays, so not for stream capture. */
 int rpm_factorized_workspace(int da, int db, int batch, const long long* half_a, const long long* half_b, int nlife,
                              long long* bytes);
 int rpm_factorized_yields(int da, int db, int batch, const double* lam_a_dev, const void* va_dev,

@@ -239,6 +239,13 @@ struct rpm_system {
   rpm::CubeView<double2>* cube64_dev = nullptr;  // device copy of cube64
   rpm::CubeView<float2>* cube32_dev = nullptr;
   std::vector<void*> allocations;
+  // tables on their way to the device: pieces of one allocation, copied together
+  struct UploadBlock {
+    char* dev;
+    size_t cap;
+    std::vector<char> host;
+  };
+  std::vector<UploadBlock> uploads;
 
   // scratch buffers, one per slot, grown on demand (cudaMalloc'd) ---------
   void* scratch[8] = {};
