@@ -254,7 +254,9 @@ struct rpm_system {
 
 namespace rpm {
 // Scratch slots of a system.  Each slot is a grow-only device buffer, zeroed
-// when (re)allocated and freed by rpm_system_destroy.
+// when (re)allocated and freed by rpm_system_destroy.  Growing a slot frees its
+// former buffer: a slot's pointer is not held across a call that may ask the
+// same slot for more.
 enum Slot : int {
   SLOT_YA = 0,        // pass-A partial of the radical-split H psi
   SLOT_REDUCE = 1,    // block partials + completion counters of reductions

@@ -1020,10 +1020,11 @@ static void plain_propagate(rpm_system* sys, const rpm_plain_knobs& k, double2* 
   }
   LanczosScalars* sc = scalars(sys);
   const int nb = row_blocks(n);
-  double2* partials = reduce_partials(sys, (size_t)nb * (RPM_MAX_KRYLOV + 1));
   PlainOut o{};
   auto run = [&](const PlainIn& in) {
     lanczos_basis_launch(sys, state, in.target, k.breakdown_tolerance, b.basis, b.alpha, b.beta, st);
+    // after the basis, which may grow the slot (and free its former buffer)
+    double2* partials = reduce_partials(sys, (size_t)nb * (RPM_MAX_KRYLOV + 1));
     if (in.npts > 0) singlet_gram_launch(sys, b.basis, in.built, b.gram, st);
     k_plain_control<<<1, kPlainWarps * 32, kPlainSmem, st>>>(b.alpha, b.beta, sc, in, b.gram, b.times, b.values,
                                                             b.perr, b.coef, b.out);
