@@ -733,6 +733,7 @@ extern "C" int rpm_adjoint_create(int ntraj, long long n, long long ld, int degr
       alloc(&a->node_out, (size_t)nodes * ntraj * vec, "the derivative outputs");
       alloc((void**)&a->hpsi64, (size_t)ntraj * ld * sizeof(double2), "the FP64 H psi");
       alloc((void**)&a->scales, (size_t)kAdjMaxDegree * sizeof(double), "the Taylor scales");
+      settle_legacy("cudaMemset(adjoint workspace)");
     } catch (...) {
       cudaFree(a->U);
       cudaFree(a->node_p);

@@ -2010,6 +2010,7 @@ int rpm_batch_create(rpm_system* const* systems, int nsys, const rpm_batch_confi
     check_cuda(cudaMalloc(&B->views_dev, sizeof(CubeView<float2>) * nsys), "cudaMalloc(views)");
     check_cuda(cudaMemcpy(B->views_dev, views.data(), sizeof(CubeView<float2>) * nsys, cudaMemcpyHostToDevice),
                "copy views");
+    settle_legacy("copy views");
     *out = B.release();
   });
 }

@@ -266,6 +266,11 @@ enum Slot : int {
   SLOT_PLAIN = 5,     // basis and step buffers of the device-driven plain propagation
 };
 void* system_scratch(rpm_system* sys, int slot, size_t bytes);
+// Waits for what was queued on the legacy default stream.  A cudaMemset, and the
+// tail of a cudaMemcpy from pageable memory, run there asynchronously to the
+// host, and a non-blocking stream (every torch.cuda.Stream) does not wait for
+// them: memory prepared that way is settled before a caller's stream may use it.
+void settle_legacy(const char* what);
 // Stream-ordered scratch of one call, from a memory pool of the library's own
 // (one per device) that keeps up to kPoolKeep bytes mapped between calls; the
 // default pool unmaps its memory at every synchronisation, which made a small

@@ -33,6 +33,8 @@ void check_cuda(cudaError_t status, const char* what) {
 
 void check_launch(const char* what) { check_cuda(cudaGetLastError(), what); }
 
+void settle_legacy(const char* what) { check_cuda(cudaStreamSynchronize(cudaStreamLegacy), what); }
+
 void* system_scratch(rpm_system* sys, int slot, size_t bytes) {
   if (slot < 0 || slot >= 8) fail(RPM_E_INVALID, "bad scratch slot");
   if (bytes <= sys->scratch_bytes[slot]) return sys->scratch[slot];
@@ -45,6 +47,7 @@ void* system_scratch(rpm_system* sys, int slot, size_t bytes) {
   size_t grown = std::max(bytes, (size_t)1 << 16);
   check_cuda(cudaMalloc(&sys->scratch[slot], grown), "cudaMalloc(scratch)");
   check_cuda(cudaMemset(sys->scratch[slot], 0, grown), "cudaMemset(scratch)");
+  settle_legacy("cudaMemset(scratch)");
   sys->scratch_bytes[slot] = grown;
   return sys->scratch[slot];
 }
@@ -259,6 +262,7 @@ static void flush_uploads(rpm_system* sys) {
     check_cuda(cudaMemcpy(b.dev, b.host.data(), b.host.size(), cudaMemcpyHostToDevice), "cudaMemcpy(system tables)");
   sys->uploads.clear();
   sys->uploads.shrink_to_fit();
+  settle_legacy("cudaMemcpy(system tables)");
 }
 
 // Outer-index records of the shape-specialised passes (see CubeView): for
@@ -723,6 +727,7 @@ int rpm_system_set_recombination(rpm_system* sys, double singlet_rate, double tr
         rpm::check_cuda(cudaMemcpy(sys->cube32_dev, &sys->cube32, sizeof(sys->cube32), cudaMemcpyHostToDevice),
                    "update cube view");
       }
+      rpm::settle_legacy("update pair operator");
     }
   });
 }

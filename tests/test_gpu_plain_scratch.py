@@ -48,3 +48,53 @@ def test_first_propagation_of_a_fresh_system(left, right):
     host = _propagate(s, h, psi, times, device_steps=False)
     np.testing.assert_allclose(first.observable_values, host.observable_values, atol=1e-12)
     np.testing.assert_allclose(first.final_state, host.final_state, atol=1e-11)
+
+
+def _behind_a_busy_default_stream(run):
+    """``run()`` on a stream of its own while the default stream still works for about 3 ms."""
+    import torch
+
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    torch.cuda._sleep(5_000_000)
+    with torch.cuda.stream(stream):
+        out = run()
+    torch.cuda.synchronize()
+    return out
+
+
+@pytest.mark.parametrize("left,right", [((2, 3), (1, 4)), ((2, 5), (1, 6))])
+def test_propagation_on_a_stream_of_its_own(left, right):
+    """A fresh system propagated on a non-blocking stream, with the default stream
+    busy when its scratch is made, and again with more scratch, gives the bits
+    that the default stream gives."""
+    times = np.arange(41) * 0.00125
+    want = _propagate(*_case(left, right), times)
+    s, h, psi = _case(left, right)
+    few = _behind_a_busy_default_stream(lambda: _propagate(s, h, psi, times[:9]))
+    np.testing.assert_array_equal(few.observable_values, _propagate(s, h, psi, times[:9]).observable_values)
+    got = _behind_a_busy_default_stream(lambda: _propagate(s, h, psi, times))
+    np.testing.assert_array_equal(got.observable_values, want.observable_values)
+    np.testing.assert_array_equal(got.final_state, want.final_state)
+
+
+def test_gradient_on_a_stream_of_its_own():
+    """The adjoint's workspace, made on a non-blocking stream while the default
+    stream is busy, gives the default stream's gradients (1e-12: its sums are
+    FP64 atomics)."""
+    import torch
+
+    from rpm_b200 import synthetic
+    from rpm_b200.adjoint import AdjointYieldGradient, ParametricRadicalPair
+
+    def gradient():
+        s = synthetic.make_system(5, (2, 3), (1, 4))
+        model = ParametricRadicalPair(s, pulse_start_us=0.005, pulse_duration_us=0.02)
+        psi = torch.from_numpy(np.stack([_case((2, 3), (1, 4), seed)[2] for seed in (3, 4)])).to("cuda")
+        r = AdjointYieldGradient(model, precision="c128")(np.array([50.0, 0.7, 0.3, 200.0, 1.0]), psi,
+                                                          np.arange(33) * 0.00125, 1.0)
+        return r.yields, r.gradients, r.populations
+
+    want = gradient()
+    for a, b in zip(_behind_a_busy_default_stream(gradient), want):
+        np.testing.assert_allclose(a, b, rtol=1e-12, atol=1e-12 * np.max(np.abs(b)))
