@@ -829,6 +829,7 @@ __global__ void __launch_bounds__(kPlainWarps * 32) k_plain_control(const double
   __shared__ double s_diag[kPlainLD], s_off[kPlainLD];
   __shared__ int s_hi[kPlainMaxCand], s_lo[kPlainMaxCand];  // candidate dimensions (lo 0: exact)
   __shared__ int s_ncand, s_status, s_sel, s_size, s_exact;
+  __shared__ bool s_finite;
   __shared__ double s_err[kPlainMaxCand], s_norm;
   __shared__ ChebScale s_scale;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -870,15 +871,17 @@ __global__ void __launch_bounds__(kPlainWarps * 32) k_plain_control(const double
     s_ncand = nc;
   }
   __syncthreads();
-  if (s_status == 0) {
-    const int size = s_size;
+  // the same in every warp: s_status is written only where all wait before they read it
+  int status = s_status;
+  if (status == 0) {
     if (warp == 0) {
-      const bool fine = warp_scale(alpha, beta, size, s_diag, s_off, &s_scale);
-      if (lane == 0 && !fine) s_status = 3;
+      const bool fine = warp_scale(alpha, beta, s_size, s_diag, s_off, &s_scale);
+      if (lane == 0) s_finite = fine;
     }
     __syncthreads();
+    if (!s_finite) status = 3;
   }
-  if (s_status == 0) {
+  if (status == 0) {
     for (int c = warp; c < s_ncand; c += kPlainWarps) {
       double err = 0.0;
       if (s_lo[c] > 0)
@@ -897,8 +900,8 @@ __global__ void __launch_bounds__(kPlainWarps * 32) k_plain_control(const double
       s_status = sel >= 0 ? 0 : (in.mode == 0 && in.max_dim > in.min_dim ? 2 : 1);
     }
     __syncthreads();
+    status = s_status;
   }
-  const int status = s_status;
   if (status == 0) {
     const int mh = s_hi[s_sel], ml = s_lo[s_sel];
     const double nn = s_norm * s_norm;

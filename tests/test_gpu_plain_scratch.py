@@ -98,3 +98,22 @@ def test_gradient_on_a_stream_of_its_own():
     want = gradient()
     for a, b in zip(_behind_a_busy_default_stream(gradient), want):
         np.testing.assert_allclose(a, b, rtol=1e-12, atol=1e-12 * np.max(np.abs(b)))
+
+
+def test_a_basis_that_is_not_finite_is_reported():
+    """Couplings of 1e160 overflow the norms of the basis: the step control's block
+    ends with an error on every call, and the system stays usable."""
+    import rpm_b200 as rb
+    from rpm_b200 import _lib
+
+    rng = np.random.default_rng(1)
+    a = rng.normal(size=(4, 4)) + 1j * rng.normal(size=(4, 4))
+    h = rb.CompiledFullPairHamiltonian((2, 2, 2, 2), [rb.LocalTerm((0, 2), 1e160 * (a + a.conj().T)),
+                                                      rb.LocalTerm((1, 3), a + a.conj().T)],
+                                       left_axes=(0, 2), right_axes=(1, 3))
+    psi = rng.normal(size=16) + 1j * rng.normal(size=16)
+    prop = rb.AdaptiveLanczosPropagator(h, minimum_dimension=6, maximum_dimension=12)
+    for _ in range(20):
+        with pytest.raises(_lib.RpmError) as e:
+            prop.propagate(psi / np.linalg.norm(psi), [0.0, 0.01], rb.SingletPopulationObservable((2, 2, 2, 2)))
+        assert e.value.code == _lib.RPM_E_NUMERIC
