@@ -191,8 +191,11 @@ int rpm_krylov_eval(const double* spectra_dev, int nreq, const rpm_krylov_req* r
 
 /* As rpm_krylov_eval straight from the tridiagonal (alpha, beta) of a basis of
  * `size` vectors, without spectra: hi and lo of a request are dimensions (lo <=
- * 0: none).  The exponentials are Chebyshev series of the tridiagonal, so that
- * small embedded errors carry no eigen-solver rounding (ENG:569-609, 690-715). */
+ * 0: none), times finite.  The exponentials are Chebyshev series of the
+ * tridiagonal, so that small embedded errors carry no eigen-solver rounding
+ * (ENG:569-609, 690-715); times beyond 2,048 / (half the Gershgorin interval)
+ * take spectra, at a cost that does not depend on the time.  RPM_E_NUMERIC when
+ * the tridiagonal is not finite. */
 int rpm_krylov_coefficients(const double* alpha_dev, const double* beta_dev, int size, int nreq,
                             const rpm_krylov_req* reqs_host, double safety, double state_norm, const void* gram_dev,
                             int gram_ld, void* coef_dev, int coef_ld, double* err_host, double* value_host,

@@ -9,7 +9,8 @@
 //     last block to finish (atomic ticket) adds them in block order.
 //   * exp(-i T t) e1 by Chebyshev series of the tridiagonal (step control and
 //     rpm_krylov_coefficients); spectra by implicit QR with Wilkinson shifts
-//     (Golub & Van Loan, Matrix Computations, sec. 8.3) for rpm_krylov_spectra.
+//     (Golub & Van Loan, Matrix Computations, sec. 8.3) for rpm_tridiag_spectra
+//     and for times beyond the series' reach.
 //   * exp(-i T t) e1 coefficients, embedded error norms and projected singlet
 //     populations (rpm_statevector_engine.py:569-609, 690-715, 521-538).
 //   * Singlet Gram, state recombination, norms and the Simpson yield
@@ -17,6 +18,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "common.cuh"
@@ -261,12 +263,14 @@ __global__ void k_tridiag_spectra(const double* __restrict__ alpha, const double
   }
 }
 
-__global__ void k_krylov_eval(const double* __restrict__ spectra, const rpm_krylov_req* reqs, double safety,
-                              double state_norm, const double2* __restrict__ gram, int gram_ld, double2* coef,
-                              int coef_ld, double* err_out, double* value_out) {
+// Request k's results go to row rows[k] of coef, err_out and value_out (null: row k).
+__global__ void k_krylov_eval(const double* __restrict__ spectra, const rpm_krylov_req* reqs, const int* rows,
+                              double safety, double state_norm, const double2* __restrict__ gram, int gram_ld,
+                              double2* coef, int coef_ld, double* err_out, double* value_out) {
   __shared__ double2 ph[RPM_MAX_KRYLOV], chi[RPM_MAX_KRYLOV], clo[RPM_MAX_KRYLOV];
   __shared__ double red[kThreads / 32];
   const rpm_krylov_req rq = reqs[blockIdx.x];
+  const int row = rows ? rows[blockIdx.x] : blockIdx.x;
   const double* rhi = spectra + (size_t)rq.hi * RPM_SPECTRUM_DOUBLES;
   const int mh = (int)rhi[0];
   spectral_coefficients(rhi, rq.time, ph, chi);
@@ -276,7 +280,7 @@ __global__ void k_krylov_eval(const double* __restrict__ spectra, const rpm_kryl
     ml = (int)rlo[0];
     spectral_coefficients(rlo, rq.time, ph, clo);
   }
-  for (int i = threadIdx.x; i < mh; i += blockDim.x) coef[(size_t)blockIdx.x * coef_ld + i] = chi[i];
+  for (int i = threadIdx.x; i < mh; i += blockDim.x) coef[(size_t)row * coef_ld + i] = chi[i];
   // ||c_hi - [c_lo; 0]||
   double acc = 0.0;
   if (rq.lo >= 0) {
@@ -295,7 +299,7 @@ __global__ void k_krylov_eval(const double* __restrict__ spectra, const rpm_kryl
   if (threadIdx.x == 0) {
     double s = 0.0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
-    err_out[blockIdx.x] = rq.lo >= 0 ? safety * state_norm * sqrt(s) : 0.0;
+    err_out[row] = rq.lo >= 0 ? safety * state_norm * sqrt(s) : 0.0;
   }
   __syncthreads();
   if (gram) {
@@ -312,7 +316,7 @@ __global__ void k_krylov_eval(const double* __restrict__ spectra, const rpm_kryl
     if (threadIdx.x == 0) {
       double s = 0.0;
       for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
-      value_out[blockIdx.x] = state_norm * state_norm * s;
+      value_out[row] = state_norm * state_norm * s;
     }
   }
 }
@@ -604,6 +608,12 @@ constexpr int kPlainWarps = 16;
 constexpr int kPlainMaxCand = 15;                             // candidate dimensions per step
 constexpr double kChebMaxArg = 256.0;  // longer times go in equal parts
 constexpr int kChebTerms = 384;         // >= 256 + 13 * 256^(1/3) + 14 + the recurrence's head start
+// A request beyond this radius x time takes the spectra instead (implicit QR,
+// whose cost does not depend on the time): steps of such a length pass the
+// embedded error only where the basis is exact.  Eight requests at 24, 32, 64,
+// 128 dimensions: series at radius x time 2,000 692, 684, 664, 1,010 us, spectra
+// 446, 738, 2,590, 11,170 us.
+constexpr double kChebReach = 8 * kChebMaxArg;
 
 struct PlainIn {
   int mode;  // 0: the minimum dimension alone; 1: ladder from the minimum; 2: ladder from minimum + increment
@@ -614,7 +624,7 @@ struct PlainIn {
 
 struct PlainOut {
   int status;  // 0 accepted, 1 rejected, 2 the maximum basis is needed, 3 eigen-solver failure, 4 zero vector,
-               // 5 a grid barrier of the basis build gave up
+               // 5 a grid barrier of the basis build gave up, 6 the step is beyond the series' reach
   int size, selected, lo, exact, pad;
   double err, norm, new_norm;
 };
@@ -725,7 +735,8 @@ struct ChebScale {
 };
 
 // Gershgorin interval of the whole tridiagonal (its leading blocks lie
-// inside), and diag / off scaled with it, by one warp; false: not finite.
+// inside), and diag / off scaled with it, by one warp; false: the entries or
+// the interval are not finite.
 static __device__ bool warp_scale(const double* alpha, const double* beta, int size, double* diag, double* off,
                                   ChebScale* sc) {
   const int lane = threadIdx.x & 31;
@@ -749,11 +760,11 @@ static __device__ bool warp_scale(const double* alpha, const double* beta, int s
   }
   if (lane == 0) *sc = ChebScale{centre, radius};
   __syncwarp();
-  return !__any_sync(0xffffffffu, bad);
+  return !__any_sync(0xffffffffu, bad) && isfinite(centre) && isfinite(radius);
 }
 
-// ch = exp(-i T_mh t) e1 (32 NE entries) by one warp; returns
-// |ch - [exp(-i T_ml t) e1; 0]|^2 (0 for ml = 0).
+// ch = exp(-i T_mh t) e1 (32 NE entries) by one warp, radius x t within
+// kChebReach; returns |ch - [exp(-i T_ml t) e1; 0]|^2 (0 for ml = 0).
 template <int NE>
 static __device__ double warp_exp_e1(const double* diag, const double* off, ChebScale sc, int mh, int ml, double t,
                                      double* bes, double2* ch) {
@@ -796,18 +807,22 @@ static __device__ double warp_quadratic(const double2* gram, int ld, const doubl
 }
 
 // rpm_krylov_coefficients: one warp per request (dimensions up to 32 NE).
+// flags: 0 done, 1 beyond the series' reach, 2 not finite (nothing written).
 template <int NE>
 __global__ void __launch_bounds__(32) k_krylov_coefficients(const double* __restrict__ alpha,
                                                             const double* __restrict__ beta, int size,
                                                             const rpm_krylov_req* reqs, double safety,
                                                             double state_norm, const double2* __restrict__ gram,
                                                             int gram_ld, double2* coef, int coef_ld, double* err_out,
-                                                            double* value_out) {
+                                                            double* value_out, int* flags) {
   __shared__ double diag[32 * NE], off[32 * NE], bes[kChebTerms];
   __shared__ double2 ch[32 * NE];
   __shared__ ChebScale sc;
   const rpm_krylov_req rq = reqs[blockIdx.x];
-  warp_scale(alpha, beta, size, diag, off, &sc);
+  const bool finite = warp_scale(alpha, beta, size, diag, off, &sc);
+  const int flag = !finite ? 2 : sc.radius * rq.time > kChebReach ? 1 : 0;
+  if (threadIdx.x == 0) flags[blockIdx.x] = flag;
+  if (flag) return;
   const double e2 = warp_exp_e1<NE>(diag, off, sc, rq.hi, max(rq.lo, 0), rq.time, bes, ch);
   for (int i = threadIdx.x; i < rq.hi; i += 32) coef[(size_t)blockIdx.x * coef_ld + i] = ch[i];
   const double v = gram ? warp_quadratic(gram, gram_ld, ch, rq.hi) : 0.0;
@@ -815,6 +830,43 @@ __global__ void __launch_bounds__(32) k_krylov_coefficients(const double* __rest
     err_out[blockIdx.x] = rq.lo > 0 ? safety * state_norm * sqrt(e2) : 0.0;
     if (gram) value_out[blockIdx.x] = state_norm * state_norm * v;
   }
+}
+
+// Candidate dimensions of a step (lo 0: exact) over a basis of `size` vectors.
+static __host__ __device__ int plain_candidates(const PlainIn& in, int size, bool exact, int* hi, int* lo) {
+  int nc = 0;
+  // (d, d - offset) as the reference's candidate evaluation (ENG:690-715)
+  auto add = [&](int d) {
+    d = d < size ? d : size;
+    const int low = d - in.offset > 1 ? d - in.offset : 1;
+    hi[nc] = d;
+    lo[nc] = low == d ? 0 : low;
+    ++nc;
+  };
+  if (exact) {
+    hi[0] = size;
+    lo[0] = 0;
+    nc = 1;
+  } else if (in.mode == 0) {
+    add(in.min_dim);
+  } else {
+    int last = 0;
+    for (int d = in.mode == 1 ? in.min_dim : in.min_dim + in.inc; d <= in.max_dim; d += in.inc) {
+      add(d);
+      last = d;
+    }
+    if (last != in.max_dim) add(in.max_dim);
+  }
+  return nc;
+}
+
+// The first candidate within the budget (-1: none), and the step's status.
+static __host__ __device__ int plain_select(const PlainIn& in, int nc, const double* err, int* status) {
+  int sel = -1;
+  for (int c = 0; c < nc && sel < 0; ++c)
+    if (err[c] <= in.budget) sel = c;
+  *status = sel >= 0 ? 0 : (in.mode == 0 && in.max_dim > in.min_dim ? 2 : 1);
+  return sel;
 }
 
 constexpr size_t kPlainSmem = kPlainWarps * (sizeof(double2) * kPlainLD + sizeof(double) * kChebTerms);
@@ -840,35 +892,10 @@ __global__ void __launch_bounds__(kPlainWarps * 32) k_plain_control(const double
     s_norm = sc->norm;
     const int size = stop > 0 ? stop : in.built;
     const int exact = size < in.target;
-    int nc = 0;
-    // (d, d - offset) as the reference's candidate evaluation (ENG:690-715)
-    auto add = [&](int d) {
-      d = min(d, size);
-      const int lo = max(1, d - in.offset);
-      s_hi[nc] = d;
-      s_lo[nc] = lo == d ? 0 : lo;
-      ++nc;
-    };
-    if (stop < 0) {
-      nc = 0;
-    } else if (exact) {
-      s_hi[0] = size;
-      s_lo[0] = 0;
-      nc = 1;
-    } else if (in.mode == 0) {
-      add(in.min_dim);
-    } else {
-      int last = 0;
-      for (int d = in.mode == 1 ? in.min_dim : in.min_dim + in.inc; d <= in.max_dim; d += in.inc) {
-        add(d);
-        last = d;
-      }
-      if (last != in.max_dim) add(in.max_dim);
-    }
+    s_ncand = stop < 0 ? 0 : plain_candidates(in, size, exact, s_hi, s_lo);
     s_status = sc->timeout ? 5 : stop < 0 ? 4 : 0;
     s_size = stop < 0 ? 0 : size;
     s_exact = exact;
-    s_ncand = nc;
   }
   __syncthreads();
   // the same in every warp: s_status is written only where all wait before they read it
@@ -880,6 +907,7 @@ __global__ void __launch_bounds__(kPlainWarps * 32) k_plain_control(const double
     }
     __syncthreads();
     if (!s_finite) status = 3;
+    else if (s_scale.radius * in.trial > kChebReach) status = 6;
   }
   if (status == 0) {
     for (int c = warp; c < s_ncand; c += kPlainWarps) {
@@ -889,16 +917,7 @@ __global__ void __launch_bounds__(kPlainWarps * 32) k_plain_control(const double
       if (lane == 0) s_err[c] = err;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      int sel = -1;
-      for (int c = 0; c < s_ncand; ++c)
-        if (s_err[c] <= in.budget) {
-          sel = c;
-          break;
-        }
-      s_sel = sel;
-      s_status = sel >= 0 ? 0 : (in.mode == 0 && in.max_dim > in.min_dim ? 2 : 1);
-    }
+    if (threadIdx.x == 0) s_sel = plain_select(in, s_ncand, s_err, &s_status);
     __syncthreads();
     status = s_status;
   }
@@ -979,6 +998,71 @@ __global__ void __launch_bounds__(kThreads) k_plain_combine(const double2* __res
   }
 }
 
+// Pool scratch of one call, freed in stream order.
+struct PoolScratch {
+  void* p;
+  cudaStream_t st;
+  PoolScratch(size_t bytes, cudaStream_t stream) : p(pool_alloc(bytes, stream)), st(stream) {}
+  ~PoolScratch() { cudaFreeAsync(p, st); }
+  PoolScratch(const PoolScratch&) = delete;
+  PoolScratch& operator=(const PoolScratch&) = delete;
+};
+
+static void spectra_launch(const double* alpha, const double* beta, int ndims, const int* dims_dev, double* spectra,
+                           cudaStream_t st) {
+  constexpr size_t smem = sizeof(double) * (RPM_MAX_KRYLOV * RPM_MAX_KRYLOV + 2 * RPM_MAX_KRYLOV) +
+                          sizeof(double2) * RPM_MAX_KRYLOV;
+  check_cuda(cudaFuncSetAttribute(k_tridiag_spectra, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+             "cudaFuncSetAttribute(spectra)");
+  k_tridiag_spectra<<<ndims, 128, smem, st>>>(alpha, beta, dims_dev, spectra);
+  check_launch("k_tridiag_spectra");
+}
+
+// Requests whose hi and lo are dimensions (lo <= 0: none) by spectra of the
+// tridiagonal: coefficients to row rows[k] of `coef`, errors and values to
+// err[rows[k]] and val[rows[k]] (host; val only with a Gram).  Synchronises.
+static void spectral_requests(const double* alpha, const double* beta, const std::vector<rpm_krylov_req>& reqs,
+                              const std::vector<int>& rows, double safety, double state_norm, const double2* gram,
+                              int gram_ld, double2* coef, int coef_ld, double* err, double* val, cudaStream_t st) {
+  std::vector<int> dims;
+  auto record = [&](int d) {
+    size_t at = std::find(dims.begin(), dims.end(), d) - dims.begin();
+    if (at == dims.size()) dims.push_back(d);
+    return (int)at;
+  };
+  std::vector<rpm_krylov_req> rec(reqs);
+  for (auto& r : rec) {
+    r.hi = record(r.hi);
+    r.lo = r.lo > 0 ? record(r.lo) : -1;
+  }
+  const int nd = (int)dims.size(), n = (int)rec.size(), nrows = 1 + *std::max_element(rows.begin(), rows.end());
+  const size_t record_bytes = sizeof(double) * RPM_SPECTRUM_DOUBLES;
+  PoolScratch spec(record_bytes * nd, st), buf((sizeof(rpm_krylov_req) + sizeof(int)) * n + sizeof(int) * nd, st),
+      res(sizeof(double) * 2 * nrows, st);
+  auto* d_req = static_cast<rpm_krylov_req*>(buf.p);
+  int* d_rows = reinterpret_cast<int*>(d_req + n);
+  int* d_dims = d_rows + n;
+  auto* d_err = static_cast<double*>(res.p);
+  check_cuda(cudaMemcpyAsync(d_req, rec.data(), sizeof(rpm_krylov_req) * n, cudaMemcpyHostToDevice, st), "copy reqs");
+  check_cuda(cudaMemcpyAsync(d_rows, rows.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st), "copy rows");
+  check_cuda(cudaMemcpyAsync(d_dims, dims.data(), sizeof(int) * nd, cudaMemcpyHostToDevice, st), "copy dims");
+  spectra_launch(alpha, beta, nd, d_dims, static_cast<double*>(spec.p), st);
+  k_krylov_eval<<<n, kThreads, 0, st>>>(static_cast<const double*>(spec.p), d_req, d_rows, safety, state_norm, gram,
+                                        gram_ld, coef, coef_ld, d_err, d_err + nrows);
+  check_launch("k_krylov_eval");
+  std::vector<double> out(2 * (size_t)nrows), status(nd);
+  check_cuda(cudaMemcpyAsync(out.data(), res.p, sizeof(double) * out.size(), cudaMemcpyDeviceToHost, st), "copy errors");
+  check_cuda(cudaMemcpy2DAsync(status.data(), sizeof(double), static_cast<const double*>(spec.p) + 1, record_bytes,
+                               sizeof(double), nd, cudaMemcpyDeviceToHost, st), "copy spectra status");
+  check_cuda(cudaStreamSynchronize(st), "spectra sync");
+  for (double s : status)
+    if (s != 0.0) fail(RPM_E_NUMERIC, "tridiagonal eigen-solver did not converge");
+  for (int r : rows) {
+    err[r] = out[r];
+    if (gram) val[r] = out[nrows + r];
+  }
+}
+
 // Device buffers of a plain propagation, kept with the system (SLOT_PLAIN).
 struct PlainBuffers {
   double2 *basis = nullptr, *gram = nullptr, *coef = nullptr;
@@ -1024,6 +1108,53 @@ static void plain_propagate(rpm_system* sys, const rpm_plain_knobs& k, double2* 
   LanczosScalars* sc = scalars(sys);
   const int nb = row_blocks(n);
   PlainOut o{};
+  // A step beyond the series' reach: the control's decisions and results from spectra.
+  auto run_spectral = [&](const PlainIn& in) {
+    int hi[kPlainMaxCand], lo[kPlainMaxCand];
+    double err[kPlainMaxCand];
+    const int nc = plain_candidates(in, o.size, o.exact != 0, hi, lo);
+    std::vector<rpm_krylov_req> reqs(nc);
+    std::vector<int> rows(nc);
+    for (int c = 0; c < nc; ++c) {
+      reqs[c] = rpm_krylov_req{hi[c], lo[c], in.trial};
+      rows[c] = c;
+    }
+    constexpr int kChunk = 1024;  // observation points at a time
+    PoolScratch coefs(sizeof(double2) * kPlainLD * std::max(kPlainMaxCand, std::min(in.npts, kChunk)), st);
+    auto* rowbuf = static_cast<double2*>(coefs.p);
+    spectral_requests(b.alpha, b.beta, reqs, rows, in.safety, o.norm, nullptr, 0, rowbuf, kPlainLD, err, nullptr, st);
+    const int sel = plain_select(in, nc, err, &o.status);
+    if (o.status != 0) return;
+    o.selected = hi[sel];
+    o.lo = lo[sel];
+    o.err = err[sel];
+    check_cuda(cudaMemcpyAsync(b.coef, rowbuf + (size_t)sel * kPlainLD, sizeof(double2) * kPlainLD,
+                               cudaMemcpyDeviceToDevice, st), "copy coefficients");
+    std::vector<double> perr(in.npts), val(in.npts);
+    for (int p0 = 0; p0 < in.npts; p0 += kChunk) {
+      const int count = std::min(kChunk, in.npts - p0);
+      reqs.resize(count);
+      rows.resize(count);
+      for (int p = 0; p < count; ++p) {
+        reqs[p] = rpm_krylov_req{o.selected, o.lo, times[in.first + p0 + p] - in.t_now};
+        rows[p] = p;
+      }
+      spectral_requests(b.alpha, b.beta, reqs, rows, in.safety, o.norm, b.gram, in.built, rowbuf, kPlainLD,
+                        perr.data() + p0, val.data() + p0, st);
+    }
+    if (in.npts > 0) {
+      check_cuda(cudaMemcpyAsync(b.values + in.first, val.data(), sizeof(double) * in.npts, cudaMemcpyHostToDevice, st),
+                 "copy values");
+      check_cuda(cudaMemcpyAsync(b.perr + in.first, perr.data(), sizeof(double) * in.npts, cudaMemcpyHostToDevice, st),
+                 "copy errors");
+    }
+    check_cuda(cudaMemcpyAsync(b.out, &o, sizeof(PlainOut), cudaMemcpyHostToDevice, st), "copy step record");
+    k_plain_combine<<<nb, kThreads, 0, st>>>(b.basis, n, b.coef, state, reduce_partials(sys, (size_t)nb * (RPM_MAX_KRYLOV + 1)),
+                                             &sc->counter[6], b.out);
+    check_launch("plain step");
+    check_cuda(cudaMemcpyAsync(&o, b.out, sizeof(PlainOut), cudaMemcpyDeviceToHost, st), "copy step record");
+    check_cuda(cudaStreamSynchronize(st), "plain step sync");
+  };
   auto run = [&](const PlainIn& in) {
     lanczos_basis_launch(sys, state, in.target, k.breakdown_tolerance, b.basis, b.alpha, b.beta, st);
     // after the basis, which may grow the slot (and free its former buffer)
@@ -1035,6 +1166,7 @@ static void plain_propagate(rpm_system* sys, const rpm_plain_knobs& k, double2* 
     check_launch("plain step");
     check_cuda(cudaMemcpyAsync(&o, b.out, sizeof(PlainOut), cudaMemcpyDeviceToHost, st), "copy step record");
     check_cuda(cudaStreamSynchronize(st), "plain step sync");
+    if (o.status == 6) run_spectral(in);
   };
   const double t_end = times[ntimes - 1];
   double now = 0.0, acc = 0.0, step = t_end > 0.0 ? std::min(k.initial_step_us, t_end) : 0.0;
@@ -1146,12 +1278,7 @@ int rpm_tridiag_spectra(const double* alpha_dev, const double* beta_dev, int ndi
     auto st = static_cast<cudaStream_t>(stream);
     auto* d_dims = static_cast<int*>(pool_alloc(sizeof(int) * ndims, st));
     check_cuda(cudaMemcpyAsync(d_dims, dims_host, sizeof(int) * ndims, cudaMemcpyHostToDevice, st), "copy dims");
-    const size_t smem = sizeof(double) * (RPM_MAX_KRYLOV * RPM_MAX_KRYLOV + 2 * RPM_MAX_KRYLOV) +
-                        sizeof(double2) * RPM_MAX_KRYLOV;
-    check_cuda(cudaFuncSetAttribute(k_tridiag_spectra, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-               "cudaFuncSetAttribute(spectra)");
-    k_tridiag_spectra<<<ndims, 128, smem, st>>>(alpha_dev, beta_dev, d_dims, spectra_dev);
-    check_launch("k_tridiag_spectra");
+    spectra_launch(alpha_dev, beta_dev, ndims, d_dims, spectra_dev, st);
     pool_free(d_dims, st);
   });
 }
@@ -1169,7 +1296,7 @@ int rpm_krylov_eval(const double* spectra_dev, int nreq, const rpm_krylov_req* r
     auto* d_err = reinterpret_cast<double*>(static_cast<char*>(dbuf) + req_bytes);
     double* d_val = d_err + nreq;
     check_cuda(cudaMemcpyAsync(d_req, reqs_host, req_bytes, cudaMemcpyHostToDevice, st), "copy reqs");
-    k_krylov_eval<<<nreq, kThreads, 0, st>>>(spectra_dev, d_req, safety, state_norm,
+    k_krylov_eval<<<nreq, kThreads, 0, st>>>(spectra_dev, d_req, nullptr, safety, state_norm,
                                               static_cast<const double2*>(gram_dev), gram_ld,
                                               static_cast<double2*>(coef_dev), coef_ld, d_err, d_val);
     check_launch("k_krylov_eval");
@@ -1191,25 +1318,41 @@ int rpm_krylov_coefficients(const double* alpha_dev, const double* beta_dev, int
     if (size < 1 || size > RPM_MAX_KRYLOV) fail(RPM_E_UNSUPPORTED, "Krylov dimension must be in [1, 128]");
     for (int k = 0; k < nreq; ++k)
       if (reqs_host[k].hi < 1 || reqs_host[k].hi > size || reqs_host[k].lo > reqs_host[k].hi ||
-          !(reqs_host[k].time >= 0.0) || reqs_host[k].hi > coef_ld || (gram_dev && reqs_host[k].hi > gram_ld))
+          !(reqs_host[k].time >= 0.0) || !std::isfinite(reqs_host[k].time) || reqs_host[k].hi > coef_ld || (gram_dev && reqs_host[k].hi > gram_ld))
         fail(RPM_E_INVALID, "bad coefficient request");
     auto st = static_cast<cudaStream_t>(stream);
     const size_t req_bytes = sizeof(rpm_krylov_req) * nreq;
-    void* dbuf = pool_alloc(req_bytes + sizeof(double) * 2 * nreq, st);
-    auto* d_req = static_cast<rpm_krylov_req*>(dbuf);
-    auto* d_err = reinterpret_cast<double*>(static_cast<char*>(dbuf) + req_bytes);
+    PoolScratch buf(req_bytes + (2 * sizeof(double) + sizeof(int)) * nreq, st);
+    auto* d_req = static_cast<rpm_krylov_req*>(buf.p);
+    auto* d_err = reinterpret_cast<double*>(static_cast<char*>(buf.p) + req_bytes);
     double* d_val = d_err + nreq;
+    int* d_flags = reinterpret_cast<int*>(d_val + nreq);
     check_cuda(cudaMemcpyAsync(d_req, reqs_host, req_bytes, cudaMemcpyHostToDevice, st), "copy reqs");
     auto* kern = size <= 64 ? k_krylov_coefficients<2> : k_krylov_coefficients<4>;
     kern<<<nreq, 32, 0, st>>>(alpha_dev, beta_dev, size, d_req, safety, state_norm,
                               static_cast<const double2*>(gram_dev), gram_ld, static_cast<double2*>(coef_dev), coef_ld,
-                              d_err, d_val);
+                              d_err, d_val, d_flags);
     check_launch("k_krylov_coefficients");
-    check_cuda(cudaMemcpyAsync(err_host, d_err, sizeof(double) * nreq, cudaMemcpyDeviceToHost, st), "copy err");
-    if (gram_dev)
-      check_cuda(cudaMemcpyAsync(value_host, d_val, sizeof(double) * nreq, cudaMemcpyDeviceToHost, st), "copy values");
-    pool_free(dbuf, st);
+    // errors, values and flags in one copy
+    std::vector<char> out((2 * sizeof(double) + sizeof(int)) * nreq);
+    check_cuda(cudaMemcpyAsync(out.data(), d_err, out.size(), cudaMemcpyDeviceToHost, st), "copy coefficient records");
     check_cuda(cudaStreamSynchronize(st), "coefficients sync");
+    memcpy(err_host, out.data(), sizeof(double) * nreq);
+    if (gram_dev) memcpy(value_host, out.data() + sizeof(double) * nreq, sizeof(double) * nreq);
+    std::vector<int> flags(nreq);
+    memcpy(flags.data(), out.data() + 2 * sizeof(double) * nreq, sizeof(int) * nreq);
+    std::vector<rpm_krylov_req> wide;
+    std::vector<int> rows;
+    for (int k = 0; k < nreq; ++k) {
+      if (flags[k] == 2) fail(RPM_E_NUMERIC, "the tridiagonal is not finite");
+      if (flags[k] == 1) {
+        wide.push_back(reqs_host[k]);
+        rows.push_back(k);
+      }
+    }
+    if (!wide.empty())
+      spectral_requests(alpha_dev, beta_dev, wide, rows, safety, state_norm, static_cast<const double2*>(gram_dev),
+                        gram_ld, static_cast<double2*>(coef_dev), coef_ld, err_host, value_host, st);
   });
 }
 
