@@ -634,12 +634,14 @@ static __device__ __forceinline__ int cheb_terms(double x) { return (int)(x + 13
 
 // bes[k] = J_k(x), k <= K, by one warp: backwards from a start eight orders
 // above K, normalised by J_0^2 + 2 sum J_k^2 = 1 (every J_k above the
-// argument is positive, which fixes the sign).
+// argument is positive, which fixes the sign).  Below 1e-100, where a step of
+// the recurrence can leave the range of the numbers, J_0 = 1 and J_1 = x / 2.
 static __device__ void warp_bessel(double x, int K, double* bes) {
   if ((threadIdx.x & 31) == 0) {
-    if (x == 0.0) {
-      for (int k = 1; k <= K; ++k) bes[k] = 0.0;
+    if (x < 1e-100) {
+      for (int k = 2; k <= K; ++k) bes[k] = 0.0;
       bes[0] = 1.0;
+      bes[1] = 0.5 * x;
     } else {
       const double two = 2.0 / x;
       double hi = 0.0, now = 1e-60, sum = 0.0;
@@ -753,7 +755,9 @@ static __device__ bool warp_scale(const double* alpha, const double* beta, int s
     lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
     hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
   }
-  const double centre = 0.5 * (lo + hi), radius = 0.5 * (hi - lo), inv = radius > 0.0 ? 1.0 / radius : 0.0;
+  const double centre = 0.5 * (lo + hi), half = 0.5 * (hi - lo);
+  const double radius = half < DBL_MIN ? 0.0 : half;  // (1 / radius stays in range)
+  const double inv = radius > 0.0 ? 1.0 / radius : 0.0;
   for (int i = lane; i < size; i += 32) {
     diag[i] = (alpha[i] - centre) * inv;
     off[i] = i + 1 < size ? beta[i] * inv : 0.0;

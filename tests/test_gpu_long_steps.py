@@ -154,3 +154,17 @@ def test_long_first_steps_are_rejected():
     assert (out[0].stats.accepted_steps, out[0].stats.rejected_steps, out[0].stats.matvecs) == \
         (out[1].stats.accepted_steps, out[1].stats.rejected_steps, out[1].stats.matvecs)
     np.testing.assert_allclose(out[0].observable_values, out[1].observable_values, atol=1e-12)
+
+
+@pytest.mark.parametrize("scale,time", [(1.0, 1e-90), (1.0, 1e-110), (1.0, 1e-150), (1.0, 1e-300), (1e-200, 1.0),
+                                        (1e-310, 1.0), (5e-324, 1e10)])
+def test_coefficients_of_vanishing_times(scale, time):
+    """Arguments down to the smallest numbers: e1 with the first-order entry -i beta_0 t (1e-13 of it; subnormal
+    couplings count as zero).  The error's sum of squares underflows below 1e-162, so it is only bounded above."""
+    alpha, beta = scale * np.array([0.5, -0.5, 0.25]), scale * np.array([1.0, 0.75, 0.0])
+    got, err, _ = _coefficients(alpha, beta, [(3, 1, time), (2, -1, time)])
+    first = -1j * beta[0] * time if scale > 1e-300 else 0.0
+    for k in range(2):
+        assert abs(got[k, 0] - 1.0) <= 1e-15
+        assert abs(got[k, 1] - first) <= 1e-13 * abs(first)
+    assert 0.0 <= err[0] <= (1.0 + 1e-13) * abs(first) and err[1] == 0.0
