@@ -263,7 +263,6 @@ enum Slot : int {
   SLOT_WORK = 2,      // Lanczos work vector
   SLOT_SMALL = 3,     // small device scalars (alpha, beta, h coefficients, flags)
   SLOT_GRAM = 4,      // Gram partials
-  SLOT_PLAIN = 5,     // basis and step buffers of the device-driven plain propagation
 };
 void* system_scratch(rpm_system* sys, int slot, size_t bytes);
 // Waits for what was queued on the legacy default stream.  A cudaMemset, and the
@@ -275,7 +274,9 @@ void settle_legacy(const char* what);
 // (one per device) that keeps up to kPoolKeep bytes mapped between calls; the
 // default pool unmaps its memory at every synchronisation, which made a small
 // allocation cost half a millisecond.  Trimmed when the last system goes.
-constexpr size_t kPoolKeep = (size_t)64 << 20;  // (the driver maps 32 MB at a time)
+// Room for a plain propagation of 221,184 components at the largest basis (64
+// vectors, 226 MB) beside small scratch (the driver maps 32 MB at a time).
+constexpr size_t kPoolKeep = (size_t)288 << 20;
 void* pool_alloc(size_t bytes, cudaStream_t stream);
 void pool_free(void* p, cudaStream_t stream);
 // H psi launchers (hpsi.cu).  `scale_dev`, when non-null, multiplies the input

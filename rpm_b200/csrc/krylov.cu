@@ -1067,7 +1067,7 @@ static void spectral_requests(const double* alpha, const double* beta, const std
   }
 }
 
-// Device buffers of a plain propagation, kept with the system (SLOT_PLAIN).
+// Device buffers of one plain propagation.
 struct PlainBuffers {
   double2 *basis = nullptr, *gram = nullptr, *coef = nullptr;
   double *alpha = nullptr, *beta = nullptr, *times = nullptr, *values = nullptr, *perr = nullptr;
@@ -1090,9 +1090,12 @@ static void plain_propagate(rpm_system* sys, const rpm_plain_knobs& k, double2* 
                o_coef = take(sizeof(double2) * kPlainLD), o_alpha = take(sizeof(double) * kPlainLD),
                o_beta = take(sizeof(double) * kPlainLD), o_times = take(sizeof(double) * ntimes), o_values = take(sizeof(double) * ntimes),
                o_perr = take(sizeof(double) * ntimes), o_out = take(sizeof(PlainOut));
-  // (a stream-ordered allocation per call was mapped anew each time: up to
-  // 80 ms for the full system's 145 MB)
-  char* base = static_cast<char*>(system_scratch(sys, SLOT_PLAIN, off));
+  // From the library's pool, which keeps the full system's buffers mapped from
+  // call to call: kept with each system they were 145 MB for every one that was
+  // ever propagated, at the same time (0.05 us of 221,184 components: 12.6 ms,
+  // 12.7 with buffers of the system's own).
+  PoolScratch buffers(off, st);
+  char* base = static_cast<char*>(buffers.p);
   b.basis = reinterpret_cast<double2*>(base + o_basis);
   b.gram = reinterpret_cast<double2*>(base + o_gram);
   b.coef = reinterpret_cast<double2*>(base + o_coef);
