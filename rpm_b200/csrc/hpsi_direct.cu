@@ -45,9 +45,12 @@ __global__ void __launch_bounds__(kDirectThreads, 6) k_hpsi_direct(const direct:
 
 // Two vectors per thread: partner arithmetic and coefficients, half of the load
 // / store pipe's work on the right radical (its lanes' digits differ), serve
-// both.  Five blocks per SM (96 registers): 221,184 x 2, 8, 32 from 15.0, 47.7,
-// 173 us to 13.5, 37.8, 132; at three blocks 161 us, at four 141, at six 156.
-__global__ void __launch_bounds__(kDirectThreads, 5) k_hpsi_direct2(const direct::Args<double2> a,
+// both.  The order of additions is the one-vector kernel's, a sum per radical:
+// a vector's result does not depend on its neighbours.  Four blocks per SM (128
+// registers): 221,184 x 2, 8, 32 12.9, 38.0, 142 us, against 14.1, 46.5, 171 by
+// single vectors.  One sum for both radicals fits five blocks (131 us for 32)
+// but rounds 7 to 13 % more.
+__global__ void __launch_bounds__(kDirectThreads, 4) k_hpsi_direct2(const direct::Args<double2> a,
                                                                const double2* __restrict__ in,
                                                                double2* __restrict__ out, int groups, int batch,
                                                                long long ld, const double* __restrict__ scale) {
@@ -66,13 +69,14 @@ __global__ void __launch_bounds__(kDirectThreads, 5) k_hpsi_direct2(const direct
   const HRec* rrp = static_cast<const HRec*>(a.rrec) + r;
   const unsigned long long rdig = rrp->digits;
   const double2* v = in + (long long)b0 * ld + g;
-  double2 o[2][4];
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) o[i][e] = make_double2(0.0, 0.0);
+  // a sum per radical, added to the local part in apply_group's order
+  double2 acc[2][2][4];
 #pragma unroll
   for (int side = 0; side < 2; ++side) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[side][i][e] = make_double2(0.0, 0.0);
     const unsigned long long digits = side ? rdig : lr.digits;
     const int np = tb.np[side];
     for (int p = 0; p < np; ++p) {
@@ -88,13 +92,14 @@ __global__ void __launch_bounds__(kDirectThreads, 5) k_hpsi_direct2(const direct
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         double2 y[4];
+        double2(&o)[4] = acc[side][i];
 #pragma unroll
         for (int e = 0; e < 4; ++e) y[e] = v[i * second + e * q + delta];
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
           const int i0 = side ? 2 * s : s, i1 = side ? 2 * s + 1 : 2 + s;
-          o[i][i0] = cfma(c01, y[i1], cfma(c00, y[i0], o[i][i0]));
-          o[i][i1] = cfma(c11, y[i1], cfma(c10, y[i0], o[i][i1]));
+          o[i0] = cfma(c01, y[i1], cfma(c00, y[i0], o[i0]));
+          o[i1] = cfma(c11, y[i1], cfma(c10, y[i0], o[i1]));
         }
       }
     }
@@ -124,7 +129,10 @@ __global__ void __launch_bounds__(kDirectThreads, 5) k_hpsi_direct2(const direct
     if (i >= count) break;
     double2* w = out + (long long)(b0 + i) * ld + g;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) w[e * q] = make_double2(s * (z[e].x + o[i][e].x), s * (z[e].y + o[i][e].y));
+    for (int e = 0; e < 4; ++e) {
+      const double2 t = cadd(cadd(z[e], acc[0][i][e]), acc[1][i][e]);
+      w[e * q] = make_double2(s * t.x, s * t.y);
+    }
   }
 }
 
@@ -138,10 +146,11 @@ void launch_direct(rpm_system* sys, const double2* in, double2* out, int batch, 
   const size_t smem = sizeof(double2) * (size_t)(sys->cube_l.ntab + sys->cube_r.ntab);
   const int gx = (groups + kDirectThreads - 1) / kDirectThreads;
   // Pairs where they still make two blocks per SM.  Pairs against single
-  // vectors, us: 13,824 x 9 8.1 / 7.9, x 16 9.3 / 9.4, x 22 (the line) 11.0 /
-  // 11.5, x 32 11.6 / 13.0; 55,296 x 4 10.3 / 10.1, x 6 12.0 / 12.4, x 7 12.4 /
-  // 13.7; 221,184 x 2 13.5 / 15.0, x 5 29.1 / 32.3, x 17 78 / 95; three vectors
-  // waste a quarter of the work: 23.1 / 21.8.
+  // vectors, us: 3,456 x 64 7.7 / 8.0, x 128 11.1 / 13.0; 13,824 x 9 7.8 / 7.6,
+  // x 16 9.1 / 8.8, x 22 (the line) 10.3 / 10.8, x 32 11.0 / 12.3; 55,296 x 4
+  // 9.7 / 9.6, x 6 11.4 / 11.7, x 7 11.7 / 12.9; 221,184 x 2 12.9 / 14.1, x 4
+  // 22.7 / 25.1, x 5 31.3 / 31.2, x 17 83 / 94; three vectors waste a quarter
+  // of the work: 21.3 / 20.8.
   if (batch != 3 && (long long)gx * (batch / 2) >= kPairBlocks) {
     k_hpsi_direct2<<<dim3(gx, (batch + 1) / 2), kDirectThreads, smem, stream>>>(
         direct::make_args(sys->cube64, sys->cube64_dev), in, out, groups, batch, ld, scale_dev);
