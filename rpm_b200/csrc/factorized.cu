@@ -59,9 +59,10 @@ struct HePair {
 };
 
 constexpr int kHeSmem = 200 * 1024;    // rows of eigenvectors
+constexpr int kHeReduceSmem = 224 * 1024;
 // the reduction's vectors and the whole matrix
 __host__ __device__ constexpr size_t tridiag_smem(int n) { return sizeof(double2) * ((size_t)n * n + 3 * (size_t)n); }
-__host__ __device__ constexpr bool tridiag_in_smem(int n) { return tridiag_smem(n) <= 224 * 1024; }
+__host__ __device__ constexpr bool tridiag_in_smem(int n) { return tridiag_smem(n) <= kHeReduceSmem; }
 
 // 0.5 (A + A^H) in place.
 __global__ void __launch_bounds__(256) k_he_symmetrise(HePair p) {
@@ -549,6 +550,8 @@ __global__ void k_fft_mac(double2* acc, const double2* x, const double2* y, long
 
 int grid_for(long long work) { return (int)std::max(1LL, std::min((work + 255) / 256, 65535LL * 4)); }
 
+// A kernel's limit is the most that any size needs, whatever the call's own
+// sizes: calls of other threads may stand between this and their launches.
 template <class K>
 void set_smem(K kern, size_t bytes) {
   check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "eigh shared memory");
@@ -578,7 +581,7 @@ char* eigh_part(HePart& h, int n, int batch, void* a, double* w, void* v, char* 
   h.status = reinterpret_cast<int*>(take((long long)batch * 8));
   h.house = reinterpret_cast<double2*>(take((long long)batch * nn * 16));
   h.z = reinterpret_cast<double*>(take((long long)batch * nn * 8));
-  // as many rows per CTA as fit beside d and e (n = 1024: 23)
+  // as many rows per CTA as fit beside d and e (n = 1024: 22)
   h.rows = std::min({n, 31 * 32, (kHeSmem / 8 - 2 * n - kEigPad) / n});
   return p;
 }
@@ -599,10 +602,11 @@ void eigh_run(HePair& p, int parts, bool symmetrise, cudaStream_t stream) {
   const int items = p.batch * parts;
   if (symmetrise)
     k_he_symmetrise<<<dim3((unsigned)(((long long)nmax * nmax + 255) / 256), items), 256, 0, stream>>>(p);
-  const size_t back_smem = sizeof(double2) * (size_t)kBackWarps * kBackCols * nmax;
-  set_smem(k_he_tridiag, red_smem);
-  set_smem(k_he_tridiag_eig, eig_smem);
-  set_smem(k_he_back, back_smem);
+  auto back_bytes = [](int n) { return sizeof(double2) * (size_t)kBackWarps * kBackCols * n; };
+  const size_t back_smem = back_bytes(nmax);
+  set_smem(k_he_tridiag, kHeReduceSmem);
+  set_smem(k_he_tridiag_eig, kHeSmem);
+  set_smem(k_he_back, back_bytes(kHeMaxN));
   k_he_tridiag<<<items, kHeThreads, red_smem, stream>>>(p);
   k_he_tridiag_eig<<<dim3(row_blocks, items), 32 + row_threads, eig_smem, stream>>>(p);
   k_he_sort<<<items, 256, 0, stream>>>(p);
