@@ -1106,12 +1106,9 @@ static void plain_propagate(rpm_system* sys, const rpm_plain_knobs& k, double2* 
   b.perr = reinterpret_cast<double*>(base + o_perr);
   b.out = reinterpret_cast<PlainOut*>(base + o_out);
   check_cuda(cudaMemcpyAsync(b.times, times, sizeof(double) * ntimes, cudaMemcpyHostToDevice, st), "copy times");
-  static bool attr = false;
-  if (!attr) {
-    check_cuda(cudaFuncSetAttribute(k_plain_control, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlainSmem),
-               "cudaFuncSetAttribute(k_plain_control)");
-    attr = true;
-  }
+  // (on every call: the limit belongs to the current device)
+  check_cuda(cudaFuncSetAttribute(k_plain_control, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlainSmem),
+             "cudaFuncSetAttribute(k_plain_control)");
   LanczosScalars* sc = scalars(sys);
   const int nb = row_blocks(n);
   PlainOut o{};
