@@ -408,7 +408,8 @@ __global__ void __launch_bounds__(1024) k_he_tridiag_eig(HePair p) {
 }
 
 // Ascending order of the eigenvalues: perm[r] = index of the r-th smallest
-// (ties by index), sorted values into w (which holds them in QR order).
+// (ties by index, NaN behind the numbers, so that perm is a permutation whatever
+// the matrix held), sorted values into w (which holds them in QR order).
 __global__ void __launch_bounds__(256) k_he_sort(HePair p) {
   __shared__ double d[kHeMaxN];
   int b;
@@ -423,7 +424,8 @@ __global__ void __launch_bounds__(256) k_he_sort(HePair p) {
     int r = 0;
     for (int j = 0; j < n; ++j) {
       const double y = d[j];
-      r += (y < x || (y == x && j < i)) ? 1 : 0;
+      const bool same = y == x || (isnan(x) && isnan(y));
+      r += (same ? j < i : y < x || isnan(x)) ? 1 : 0;
     }
     perm[r] = i;
     w[r] = x;

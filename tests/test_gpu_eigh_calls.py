@@ -1,4 +1,4 @@
-"""Hermitian eigen-solver calls of several host threads (GPU)."""
+"""Hermitian eigen-solver: calls of several host threads, matrices that are not finite (GPU)."""
 
 import threading
 
@@ -41,3 +41,25 @@ def test_sizes_solved_by_several_threads_at_once():
     for t in threads:
         t.join()
     assert failures == []
+
+
+# in shared memory and one block of eigenvector rows; in global memory and several
+@pytest.mark.parametrize("n", [6, 72, 160])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_matrices_that_are_not_finite_are_reported(n, bad):
+    """An error, and the solver goes on working."""
+    import torch
+
+    from rpm_b200 import _lib
+    from rpm_b200.factorized import hermitian_eigh
+
+    rng = np.random.default_rng(n)
+    a = rng.normal(size=(3, n, n)) + 1j * rng.normal(size=(3, n, n))
+    a = torch.from_numpy(a + a.conj().transpose(0, 2, 1)).to("cuda")
+    broken = a.clone()
+    broken[1, 2, 1] = broken[1, 1, 2] = bad
+    with pytest.raises(_lib.RpmError) as e:
+        hermitian_eigh(broken)
+    assert e.value.code == _lib.RPM_E_NUMERIC
+    lam, _ = hermitian_eigh(a)
+    np.testing.assert_allclose(lam.cpu().numpy(), np.linalg.eigvalsh(a.cpu().numpy()), atol=1e-12 * n)
