@@ -109,12 +109,12 @@ __global__ void __launch_bounds__(256) k_bin_lines9(Radical ra, Radical rb, doub
   const double* lam = r.lam + (size_t)b * d;
   const double pos = (lam[i] - lam[j]) / delta + (double)half;
   const double fl = floor(pos);
-  const long long lower = (long long)fl;
-  const double frac = pos - fl;
-  if (!(lower >= 0 && lower + 1 < 2 * half + 1)) {
+  if (!(fl >= 0.0 && fl < (double)(2 * half))) {  // before the conversion: infinite and NaN positions too
     atomicExch(bad, 1);
     return;
   }
+  const long long lower = (long long)fl;
+  const double frac = pos - fl;
   const size_t dd = (size_t)d * d;
   const double2* ops = r.ops + 3 * (size_t)b * dd;
   const double scale = 1.0 / (double)(d / 2);

@@ -268,12 +268,12 @@ __global__ void k_bin_lines(const double* __restrict__ lam, const double2* __res
   const double cx = (a.x * b.x - a.y * b.y) * scale, cy = (a.x * b.y + a.y * b.x) * scale;
   const double pos = (lam[i] - lam[j]) / delta + (double)half_width;
   const double fl = floor(pos);
-  const long long lower = (long long)fl;
-  const double frac = pos - fl;
-  if (lower < 0 || lower + 1 >= size) {
+  if (!(fl >= 0.0 && fl < (double)(size - 1))) {  // before the conversion: infinite and NaN positions too
     atomicExch(bad, 1);
     return;
   }
+  const long long lower = (long long)fl;
+  const double frac = pos - fl;
   atomicAdd(&grid[lower].x, cx * (1.0 - frac));
   atomicAdd(&grid[lower].y, cy * (1.0 - frac));
   atomicAdd(&grid[lower + 1].x, cx * frac);
