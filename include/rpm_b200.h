@@ -89,7 +89,9 @@ int rpm_hpsi(rpm_system* sys, int precision, const void* psi_dev, void* out_dev,
  * wide; 0 = built-in heuristic): inner spin-1/2 digits per radical cube
  * (ni_l, ni_r in {1, 2}), pass-L column tile tr in {1, 2, 4, 8} and pass-R
  * row tile tl in {1, ..., 16}.  A choice that cannot run for a system falls
- * back to the heuristic.  Used by the autotuner; no reference counterpart. */
+ * back to the heuristic.  H psi inside the one-launch Lanczos basis and the
+ * one-launch Taylor terms is no launch of its own.  Used by the autotuner; no
+ * reference counterpart. */
 int rpm_set_cube_tuning(int ni_l, int ni_r, int tr, int tl);
 
 /* Haberkorn recombination with singlet / triplet rates (1/us) on a radical-

@@ -574,6 +574,12 @@ __global__ void __launch_bounds__(kTaylorThreads) k_adj_taylor(const direct::Arg
 
 // Whether a system's Taylor terms run in one launch: the direct H psi covers it
 // and two copies of a vector fit in shared memory (up to about 6,000 components).
+// The line is that capacity, not the crossing: a gradient of 80 intervals with
+// 1, 4, 16 vectors takes, one launch against a direct launch per term, 864
+// components 14.0, 14.9, 16.1 / 18.5, 19.4, 20.3 ms; 1,728 19.2, 21.3, 23.0 /
+// 20.4, 22.3, 25.6; 3,456 28.0, 27.9, 32.0 / 23.6, 24.3, 26.9; 5,184 36.5, 38.1,
+// 42.0 / 23.8, 25.8, 29.6 (one SM per vector works in several rounds there; two
+// cube passes per term took 38.8, 49.0, 83.5).
 size_t taylor_smem(const rpm_system* h) {
   return sizeof(double2) * (size_t)(h->cube_l.ntab + h->cube_r.ntab + 2 * h->n) +
          sizeof(direct::HRec) * (size_t)(h->half_l + h->half_r);

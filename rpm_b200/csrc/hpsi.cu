@@ -704,11 +704,11 @@ CubePlan cube_plan(rpm_system* const* systems, int nsys) {
 }
 
 // The direct H psi takes every complex128 call of a standard-layout system: one
-// launch without scratch, at any batch (the full system: 13 us for one vector
-// and 334 us for 64 against 35 and 428 us of two shape-specialised tiled
+// launch without scratch, at any batch (the full system: 10.8 us for one vector
+// and 142 us for 32 against 34 and 218 us of two shape-specialised tiled
 // passes, whose few large tiles left most SMs idle for small batches; 864
-// dimensions, 32 vectors: 10 against 23 us of two general cube passes).  An
-// explicit cube-kernel variant (rpm_set_cube_tuning) keeps the cube kernels.
+// dimensions: 4.1 us for 64 vectors against 23 us for 32 by two general cube
+// passes).  An explicit cube-kernel variant (rpm_set_cube_tuning) keeps the cube kernels.
 template <class T>
 static bool try_direct(rpm_system* sys, const T* in, T* out, int batch, long long ld, const double* scale_dev,
                        cudaStream_t stream) {

@@ -6,7 +6,7 @@ namespace {
 
 // Bound by the load / store pipe (61 % of its wavefronts at 28 % occupancy, FP64
 // pipe 32 %, DRAM 6 %: ncu, 8 vectors of 221,184).  Six blocks of 128 threads
-// per SM (80 registers): 173 us for 32 vectors; before the tables came by
+// per SM (80 registers): 171 us for 32 vectors; before the tables came by
 // argument 181, against 187 us at 92 registers and 202 us at 64, which spills.
 constexpr int kDirectThreads = 128;
 constexpr int kPairBlocks = 296;
